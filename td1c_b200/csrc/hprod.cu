@@ -118,6 +118,9 @@ struct Ctx {
   // ---- device tables
   double *xrad = nullptr, *mask = nullptr, *radk = nullptr, *radk0 = nullptr, *radp = nullptr, *cost = nullptr;
   double *legf1 = nullptr, *legb1 = nullptr, *legf2 = nullptr, *legb2 = nullptr, *alph = nullptr;
+  // parity halves of the same tables (null when the bound theta grid is not symmetric)
+  double *pf1 = nullptr, *pb1 = nullptr, *pf2 = nullptr, *pb2 = nullptr;
+  bool leg_par = false;
   double *tdiag = nullptr, *d2ll = nullptr, *d2rinv = nullptr, *rpl0 = nullptr, *rpl1 = nullptr, *invr = nullptr, *fac2 = nullptr, *fac1 = nullptr;
   double *ps_tabf = nullptr, *ps_tabb = nullptr;  // Poisson row tables (forward, backward)
   PoissonArgs ps_main{}, ps_fcfc{};  // Poisson arguments with encoded tensor maps (RHS pairs, fcfc pairs)
@@ -742,6 +745,53 @@ PoissonArgs poisson_args(const Ctx& c, int npair, int pair0) {
   return pa;
 }
 
+// Parity halves of the Legendre tables for the folded transforms (legendre_par.cu), when
+// every table has P_l^m(-x) = (-1)^(l+m) P_l^m(x) under the mirror t -> nlat - 1 - t to
+// 1e-14 of its largest value (a Gauss-Legendre grid's tables have it to the last bit, or to
+// the rounding of the nodes); else, or where a value is not finite, the dense transforms run.
+// to_theta tables are [m][theta][l], the others [m][l][theta].
+void build_parity_tables(Ctx& c) {
+  struct Tab { const std::vector<double>* h; int mmax, nl; bool to_theta; double** dst; };
+  const Tab tabs[4] = {{&c.h_legf1, c.mmax1, c.L1, true, &c.pf1}, {&c.h_legb1, c.mmax1, c.L1, false, &c.pb1},
+                       {&c.h_legf2, c.mmax2, c.L2, true, &c.pf2}, {&c.h_legb2, c.mmax2, c.L2, false, &c.pb2}};
+  const int nt = c.nlat, ht = (nt + 1) / 2;
+  c.leg_par = nt >= 2;
+  for (const Tab& T : tabs) {
+    double big = 0.0, off = 0.0;
+    auto at = [&](int m, int l, int t) {
+      return (*T.h)[T.to_theta ? ((size_t)m * nt + t) * T.nl + l : ((size_t)m * T.nl + l) * nt + t];
+    };
+    bool finite = true;
+    for (int m = 0; m <= 2 * T.mmax; ++m)
+      for (int l = 0; l < T.nl; ++l) {
+        const double sg = ((l + std::abs(m - T.mmax)) & 1) ? -1.0 : 1.0;
+        for (int t = 0; t < nt; ++t) {
+          const double x = at(m, l, t);
+          finite = finite && std::isfinite(x);
+          big = std::max(big, std::fabs(x));
+          off = std::max(off, std::fabs(x - sg * at(m, l, nt - 1 - t)));
+        }
+      }
+    if (!finite || !(off <= 1e-14 * big)) c.leg_par = false;
+  }
+  if (!c.leg_par) return;
+  for (const Tab& T : tabs) {
+    const int hl = (T.nl + 1) / 2, rows = T.to_theta ? ht : hl, ld = legendre_ldp(T.to_theta ? hl : ht);
+    std::vector<double> p((size_t)(2 * T.mmax + 1) * 2 * rows * ld, 0.0);
+    for (int m = 0; m <= 2 * T.mmax; ++m)
+      for (int l = 0; l < T.nl; ++l) {
+        const int q = (l + std::abs(m - T.mmax)) & 1;  // parity of l + m
+        for (int t = 0; t < ht; ++t) {
+          if (q && 2 * t == nt - 1) continue;  // odd functions vanish at cos(theta) = 0
+          const int r = T.to_theta ? t : l / 2, k = T.to_theta ? l / 2 : t;
+          const size_t src = T.to_theta ? ((size_t)m * nt + t) * T.nl + l : ((size_t)m * T.nl + l) * nt + t;
+          p[(((size_t)m * 2 + q) * rows + r) * ld + k] = (*T.h)[src];
+        }
+      }
+    *T.dst = dupload(p);
+  }
+}
+
 int build_tables(Ctx& c) {
   const int bw = 2 * c.nd + 1;
   c.xrad = dupload(c.h_xrad);
@@ -765,6 +815,7 @@ int build_tables(Ctx& c) {
   c.legb1 = pad_tables(c.h_legb1, 2 * c.mmax1 + 1, c.L1, c.nlat);
   c.legf2 = pad_tables(c.h_legf2, 2 * c.mmax2 + 1, c.nlat, c.L2);
   c.legb2 = pad_tables(c.h_legb2, 2 * c.mmax2 + 1, c.L2, c.nlat);
+  build_parity_tables(c);
   (void)bw;
   // alph_lm (bas_gen_alph.F90:2-26)
   std::vector<double> alph((size_t)c.L1 * (2 * c.mmax1 + 1), 0.0);
@@ -896,37 +947,45 @@ int build_batches(Ctx& c) {
   auto lb1 = [&](int m) { return c.legb1 + (size_t)(m + c.mmax1) * c.L1 * ldn; };
   auto lf2 = [&](int m) { return c.legf2 + (size_t)(m + c.mmax2) * c.nlat * ld2; };
   auto lb2 = [&](int m) { return c.legb2 + (size_t)(m + c.mmax2) * c.L2 * ldn; };
+  const size_t ht = (c.nlat + 1) / 2, h1 = (c.L1 + 1) / 2, h2 = (c.L2 + 1) / 2;
+  auto pf1 = [&](int m) { return c.pf1 ? c.pf1 + (size_t)(m + c.mmax1) * 2 * ht * legendre_ldp((int)h1) : nullptr; };
+  auto pb1 = [&](int m) { return c.pb1 ? c.pb1 + (size_t)(m + c.mmax1) * 2 * h1 * legendre_ldp((int)ht) : nullptr; };
+  auto pf2 = [&](int m) { return c.pf2 ? c.pf2 + (size_t)(m + c.mmax2) * 2 * ht * legendre_ldp((int)h2) : nullptr; };
+  auto pb2 = [&](int m) { return c.pb2 ? c.pb2 + (size_t)(m + c.mmax2) * 2 * h2 * legendre_ldp((int)ht) : nullptr; };
   std::vector<LegGemmBatch> v;
   // sph2ang1 of dynamic orbitals: orbg[f] = legf1[m] (nlat x L1) * orb[f] (L1 x 2Nr)
   for (int f = c.nfcore; f < c.nfun; ++f)
-    v.push_back({lf1(c.mval[f]), (const double*)(c.orb + f * c.nbas), nullptr, (double*)(c.orbg + f * c.ngrid), N, N, ld1, 0});
+    v.push_back({lf1(c.mval[f]), (const double*)(c.orb + f * c.nbas), nullptr, (double*)(c.orbg + f * c.ngrid), N, N, ld1, std::abs(c.mval[f]) & 1, pf1(c.mval[f])});
   c.n_orbg = (int)v.size(); batch_upload(c.b_orbg, v); v.clear();
   // sph2ang1 of the stored frozen core (set-up): orbg0[f] = legf1 * orb0[f]
   for (int f = 0; f < c.nfcore; ++f)
-    v.push_back({lf1(c.mval[f]), (const double*)(c.orb0 + f * c.nbas), nullptr, (double*)(c.orbg0 + f * c.ngrid), N, N, ld1, 0});
+    v.push_back({lf1(c.mval[f]), (const double*)(c.orb0 + f * c.nbas), nullptr, (double*)(c.orbg0 + f * c.ngrid), N, N, ld1, std::abs(c.mval[f]) & 1, pf1(c.mval[f])});
   batch_upload(c.b_orbg0, v); v.clear();
   // ang2sph1 of the gauge-transformed frozen core: orb[f] = legb1 (L1 x nlat) * orbg[f]
   for (int f = 0; f < c.nfcore; ++f)
-    v.push_back({lb1(c.mval[f]), (const double*)(c.orbg + f * c.ngrid), nullptr, (double*)(c.orb + f * c.nbas), N, N, ldn, 0});
+    v.push_back({lb1(c.mval[f]), (const double*)(c.orbg + f * c.ngrid), nullptr, (double*)(c.orb + f * c.nbas), N, N, ldn, std::abs(c.mval[f]) & 1, pb1(c.mval[f])});
   c.n_orbfc = (int)v.size(); batch_upload(c.b_orbfc, v); v.clear();
   // pair density -> rho2 (M = L2, K = nlat)
   for (int p = 0; p < c.npair; ++p) {
     int a = c.pa[p], b = c.pb[p];
     v.push_back({lb2(c.mval[b] - c.mval[a]), (const double*)(c.orbg + a * c.ngrid), (const double*)(c.orbg + b * c.ngrid),
-                 (double*)(c.rho2 + (size_t)p * c.nbas2), N, N, ldn, 0});
+                 (double*)(c.rho2 + (size_t)p * c.nbas2), N, N, ldn, std::abs(c.mval[b] - c.mval[a]) & 1,
+                 pb2(c.mval[b] - c.mval[a])});
   }
   batch_upload(c.b_rho, v); c.h_b_rho = v; v.clear();
   for (int p = c.npair; p < c.npair_all; ++p) {
     int a = c.pa[p], b = c.pb[p];
     v.push_back({lb2(c.mval[b] - c.mval[a]), (const double*)(c.orbg + a * c.ngrid), (const double*)(c.orbg + b * c.ngrid),
-                 (double*)(c.rho2 + (size_t)p * c.nbas2), N, N, ldn, 0});
+                 (double*)(c.rho2 + (size_t)p * c.nbas2), N, N, ldn, std::abs(c.mval[b] - c.mval[a]) & 1,
+                 pb2(c.mval[b] - c.mval[a])});
   }
   batch_upload(c.b_rho_fcfc, v); v.clear();
   // W = legf2 (nlat x L2) * v2sph
   for (int p = 0; p < c.npair_all; ++p) {
     int a = c.pa[p], b = c.pb[p];
     v.push_back({lf2(c.mval[b] - c.mval[a]), (const double*)(c.v2sph + (size_t)p * c.nbas2), nullptr,
-                 (double*)(c.W + (size_t)p * c.ngrid), N, N, ld2, 0});
+                 (double*)(c.W + (size_t)p * c.ngrid), N, N, ld2, std::abs(c.mval[b] - c.mval[a]) & 1,
+                 pf2(c.mval[b] - c.mval[a])});
   }
   {
     std::vector<LegGemmBatch> v1(v.begin(), v.begin() + c.npair), v2(v.begin() + c.npair, v.end());
@@ -936,12 +995,12 @@ int build_batches(Ctx& c) {
   v.clear();
   // ang2sph1 of g and v2 for dynamic orbitals (M = L1, K = nlat)
   for (int f = c.nfcore; f < c.nfun; ++f)
-    v.push_back({lb1(c.mval[f]), (const double*)(c.gorbg + f * c.ngrid), nullptr, (double*)(c.gorb + f * c.nbas), N, N, ldn, 0});
+    v.push_back({lb1(c.mval[f]), (const double*)(c.gorbg + f * c.ngrid), nullptr, (double*)(c.gorb + f * c.nbas), N, N, ldn, std::abs(c.mval[f]) & 1, pb1(c.mval[f])});
   for (int f = c.nfcore; f < c.nfun; ++f)
-    v.push_back({lb1(c.mval[f]), (const double*)(c.v2orbg + f * c.ngrid), nullptr, (double*)(c.v2orb + f * c.nbas), N, N, ldn, 0});
+    v.push_back({lb1(c.mval[f]), (const double*)(c.v2orbg + f * c.ngrid), nullptr, (double*)(c.v2orb + f * c.nbas), N, N, ldn, std::abs(c.mval[f]) & 1, pb1(c.mval[f])});
   c.n_gorb = (int)v.size(); batch_upload(c.b_gorb, v); v.clear();
   for (int f = 0; f < c.nfcore; ++f)
-    v.push_back({lb1(c.mval[f]), (const double*)(c.gorbg + f * c.ngrid), nullptr, (double*)(c.gorb + f * c.nbas), N, N, ldn, 0});
+    v.push_back({lb1(c.mval[f]), (const double*)(c.gorbg + f * c.ngrid), nullptr, (double*)(c.gorb + f * c.nbas), N, N, ldn, std::abs(c.mval[f]) & 1, pb1(c.mval[f])});
   batch_upload(c.b_gorbfc, v);
   return 0;
 }
@@ -1359,8 +1418,11 @@ int build_ci(Ctx& c) {
 // ===========================================================================
 // the RHS
 // ===========================================================================
-int gemm(Ctx& c, const LegGemmBatch* b, int nb, int M, int K, bool pair) {
+// one theta <-> l transform: to_l theta -> l (K = nlat), else l -> theta (M = nlat); folded by
+// parity on a symmetric theta grid
+int gemm(Ctx& c, const LegGemmBatch* b, int nb, int M, int K, bool to_l, bool pair = false) {
   c.launches++;
+  if (c.leg_par) return launch_legendre_par(b, nb, M, K, 2 * c.Nr, to_l, pair, c.tune_mt, c.st);
   return launch_legendre_gemm_mt(b, nb, M, K, 2 * c.Nr, pair, c.tune_mt, c.st);
 }
 // the int2e K split: the tuned value where one is set (at most the allocated split)
@@ -1389,7 +1451,7 @@ int mfprod_run(Ctx& c, cudaStream_t st) {
 // the mean field's transforms (pair densities theta -> l, pair potentials l -> theta):
 // FP64 DMMA, or split TF32 on tcgen05 in the mixed-precision form
 int gemm_mf(Ctx& c, const LegGemmBatch* b, int nb, int M, int K, bool pair) {
-  if (!c.mixed) return gemm(c, b, nb, M, K, pair);
+  if (!c.mixed) return gemm(c, b, nb, M, K, pair, pair);  // pair densities go to l, potentials to theta
   c.launches++;
   if (c.mixed != 2 && b == c.b_rho && c.tc_ok_rho) return launch_legendre_tc(c.tc_rho, c.d_status, c.st);
   if (c.mixed != 2 && b == c.b_W && c.tc_ok_W) return launch_legendre_tc(c.tc_W, c.d_status, c.st);
@@ -1465,7 +1527,7 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
       size_t nfc = c.ngrid * c.nfcore;
       fc_phase_kernel<<<(unsigned)((nfc + 255) / 256), 256, 0, st>>>(c.Nr, c.nlat, c.nfcore, c.xrad, c.cost, d_lf, c.orbg0, c.orbg);
       c.launches++;
-      rc |= chk("fc gemm", gemm(c, c.b_orbfc, c.n_orbfc, c.L1, c.nlat, false));
+      rc |= chk("fc gemm", gemm(c, c.b_orbfc, c.n_orbfc, c.L1, c.nlat, true));
     }
   }
   mark();  // end orbin
@@ -1495,7 +1557,7 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
     rc |= chk("mfprod", mfprod_run(c, st));
     c.launches += 2;
     mark();  // end mfprod
-    rc |= chk("gorb gemm", gemm(c, c.b_gorb, c.n_gorb, c.L1, c.nlat, false));
+    rc |= chk("gorb gemm", gemm(c, c.b_gorb, c.n_gorb, c.L1, c.nlat, true));
   } else if (c.neltot >= 2 && c.npair > 0) {
     rc |= chk("rho gemm", gemm_mf(c, c.b_rho, c.npair, c.L2, c.nlat, true));
     mark();  // end rho_gemm
@@ -1523,7 +1585,7 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
     rc |= chk("mfprod", mfprod_run(c, st));
     c.launches += 2;
     mark();  // end mfprod
-    rc |= chk("gorb gemm", gemm(c, c.b_gorb, c.n_gorb, c.L1, c.nlat, false));
+    rc |= chk("gorb gemm", gemm(c, c.b_gorb, c.n_gorb, c.L1, c.nlat, true));
   } else {
     join();
     mark(); mark(); mark(); mark();
@@ -2703,7 +2765,7 @@ void hprod_set_wfn0_(const double* wfn, const double* cic, const char* v2xfc_typ
     return;
   }
   // sph2ang1 of the stored frozen core (lfield = 0: no gauge phase)
-  launch_legendre_gemm(c.b_orbg0, c.nfcore, c.nlat, c.L1, 2 * c.Nr, false, st);
+  gemm(c, c.b_orbg0, c.nfcore, c.nlat, c.L1, false);
   // frozen-core Hartree potential (hprod_mkrhofc, hprod_mkv2jfc)
   int* d_lval = dupload(c.lval);
   v2jfc_kernel<<<1, 1, 0, st>>>(c.Nr, c.nd, c.L1, c.nfcore, c.d_mval, d_lval, c.orb0, c.d2ll, c.d2rinv, c.rpl0, c.rpl1, c.invr,
@@ -2712,10 +2774,10 @@ void hprod_set_wfn0_(const double* wfn, const double* cic, const char* v2xfc_typ
   // orbg(fc) = orbg0; fcfc pair densities, Poisson, l->theta
   cudaMemcpyAsync(c.orbg, c.orbg0, c.nfcore * c.ngrid * sizeof(cplx), cudaMemcpyDeviceToDevice, st);
   if (c.igauge == 0) cudaMemcpyAsync(c.orb, c.orb0, c.nfcore * c.nbas * sizeof(cplx), cudaMemcpyDeviceToDevice, st);
-  else launch_legendre_gemm(c.b_orbfc, c.nfcore, c.L1, c.nlat, 2 * c.Nr, false, st);  // orb(fc) = ang2sph1(orbg(fc))
-  launch_legendre_gemm(c.b_rho_fcfc, c.nfcfc, c.L2, c.nlat, 2 * c.Nr, true, st);
+  else gemm(c, c.b_orbfc, c.nfcore, c.L1, c.nlat, true);  // orb(fc) = ang2sph1(orbg(fc))
+  gemm(c, c.b_rho_fcfc, c.nfcfc, c.L2, c.nlat, true, true);
   launch_poisson(c.ps_fcfc, st);
-  launch_legendre_gemm(c.b_W_fcfc, c.nfcfc, c.nlat, c.L2, 2 * c.Nr, false, st);
+  gemm(c, c.b_W_fcfc, c.nfcfc, c.nlat, c.L2, false);
   // frozen-core energy: enefc = 2 Re <phi|h0|phi> + Re <phi| v2jfc - sum_j W(j,i) phi_j >
   // with h0 from the bare kinetic table (before v2jfc is added)
   OneBodyArgs ob{};
@@ -2728,7 +2790,7 @@ void hprod_set_wfn0_(const double* wfn, const double* cic, const char* v2xfc_typ
   const size_t nfcg = c.nfcore * c.ngrid;
   fc_g_kernel<<<(unsigned)((nfcg + 255) / 256), 256, 0, st>>>(c.Nr, c.nlat, c.nfcore, c.nfun, c.orbg, c.W, c.pair_of,
                                                               c.pair_cj, c.v2jfc, c.gorbg);
-  launch_legendre_gemm(c.b_gorbfc, c.nfcore, c.L1, c.nlat, 2 * c.Nr, false, st);
+  gemm(c, c.b_gorbfc, c.nfcore, c.L1, c.nlat, true);
   dot_re_kernel<<<1, 256, 0, st>>>(c.orb, c.gorb, c.nfcore * c.nbas, c.d_scalar + 1);
   double es[2] = {0, 0};
   cudaMemcpyAsync(es, c.d_scalar, 2 * sizeof(double), cudaMemcpyDeviceToHost, st);
@@ -2930,7 +2992,7 @@ int td1c_gpu_dipole3(const void* d_wfn, const void* d_cic, const double* lfield,
       const size_t nfcg = c.nfcore * c.ngrid;
       fc_gfock_kernel<<<(unsigned)((nfcg + 255) / 256), 256, 0, st>>>(c.Nr, c.nlat, c.nfcore, c.ncore, c.nact, c.nfun, c.d_mval,
                                                                       c.orbg, c.W, c.pair_of, c.pair_cj, c.den1, c.gorbg);
-      rc |= chk("fc gorb gemm", gemm(c, c.b_gorbfc, c.nfcore, c.L1, c.nlat, false));
+      rc |= chk("fc gorb gemm", gemm(c, c.b_gorbfc, c.nfcore, c.L1, c.nlat, true));
     }
     w = c.orb;
   } else if (c.nact > 0) {

@@ -22,12 +22,18 @@ struct LegGemmBatch {
   const double* B0;  // slab (K rows x ldb reals) or conj operand for pair mode
   const double* B1;  // second operand for pair mode
   double* C;         // output, M rows x ldc reals
-  int ldb, ldc, lda, pad;
+  int ldb, ldc, lda;
+  int mpar = 0;               // |m| mod 2 of the table
+  const double* P = nullptr;  // the table's parity halves (legendre_par.cu): [2][half rows][legendre_ldp(half depth)]
 };
 // row pitch of the padded Legendre tables: depth rounded up to the GEMM's 32-deep chunks
 __host__ __device__ inline int legendre_lda(int k) { return (k + 31) / 32 * 32; }
-int launch_legendre_gemm(const LegGemmBatch* d_batches, int nbatch, int M, int K, int N, bool pair,
-                         cudaStream_t st);
+// row pitch of a parity half: depth rounded up to legendre_par.cu's 16-deep chunks
+__host__ __device__ inline int legendre_ldp(int k) { return (k + 15) / 16 * 16; }
+// the same transforms on tables whose theta grid is symmetric, with the parity of the Legendre
+// functions folded in (half the operations); to_l: theta -> l (K = nlat), else l -> theta (M = nlat)
+int launch_legendre_par(const LegGemmBatch* d_batches, int nbatch, int M, int K, int N, bool to_l, bool pair, int mt,
+                        cudaStream_t st);
 int launch_legendre_gemm_mt(const LegGemmBatch* d_batches, int nbatch, int M, int K, int N, bool pair, int mt,
                             cudaStream_t st);
 // the same transform in split TF32 on tcgen05 (FP32 accumulation, FP64 in and out);

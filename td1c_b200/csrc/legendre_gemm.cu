@@ -152,11 +152,6 @@ static void lg_launch(const LegGemmBatch* d_batches, int nbatch, int M, int K, i
   legendre_gemm_kernel<MT, PAIR><<<grid, 256, lg_smem_bytes(MT), st>>>(d_batches, M, K, N);
 }
 
-int launch_legendre_gemm(const LegGemmBatch* d_batches, int nbatch, int M, int K, int N, bool pair,
-                         cudaStream_t st) {
-  return launch_legendre_gemm_mt(d_batches, nbatch, M, K, N, pair, 0, st);
-}
-
 // mt: the CTA's m-tiles (3: 48 rows, 6: 96 rows); 0 chooses by M
 int launch_legendre_gemm_mt(const LegGemmBatch* d_batches, int nbatch, int M, int K, int N, bool pair, int mt,
                             cudaStream_t st) {
