@@ -195,7 +195,8 @@ struct Ctx {
   H1Slot h1slot[kH1Slots];
   int n_h1 = 0;
   cplx* h1_z[2] = {nullptr, nullptr};  // interior solutions (alternating passes)
-  cplx *h1_cb = nullptr, *h1_xb = nullptr;  // bridge shares, bridge values
+  cplx *h1_cb[2] = {nullptr, nullptr}, *h1_xb = nullptr;  // bridge shares (alternating passes), bridge values
+  double *h1_pf = nullptr, *h1_tf = nullptr, *h1_rinv = nullptr;  // band blocks of the folded passes, 1 / r
   double* h1_partial = nullptr;
   unsigned* h1_ticket = nullptr;
   int* h1_flags = nullptr;  // [0] done, [1] cycles of the last application, [2] cycle counter of a graph loop
@@ -1768,6 +1769,30 @@ void pulse_lfield(const Pulse& p, double t, double* lf) {
 // one-body propagators (h1prop.cu): factor cache and the application of
 // h1itr_prop / dpade_prod to the orbitals of a device state
 // ---------------------------------------------------------------------------
+// the tables of the folded passes (h1cycle.cu) beside a new factor; sizes or bands they do not
+// take leave w < 0 (the band's width is read back, so not inside a graph capture)
+int h1c_build(Ctx& c, H1Fac& f) {
+  f.w = -1;
+  cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(c.st, &cst);
+  if (cst != cudaStreamCaptureStatusNone || !h1c_fits(c.nd, c.nfun, 0, c.igauge)) return 0;
+  const size_t ne = (size_t)c.L1 * f.nfe;
+  if (!f.af) {
+    f.af = dalloc<cplx>(ne * h1c_af_size(c.nd));
+    f.glr = dalloc<cplx>(ne * 2 * f.ni);
+    f.sinv = dalloc<cplx>((size_t)c.L1 * std::max(1, f.nb) * std::max(1, f.nb));
+  }
+  if (!f.af || !f.glr || !f.sinv) return 0;
+  int w = 0;
+  int* d_w = c.h1_flags + 3;
+  cudaMemsetAsync(d_w, 0, sizeof(int), c.st);
+  const int rc = launch_h1c_setup(f, d_w, c.st);
+  cudaMemcpyAsync(&w, d_w, sizeof(int), cudaMemcpyDeviceToHost, c.st);
+  if (rc || cudaStreamSynchronize(c.st) != cudaSuccess) return ST_CUDA;
+  f.w = h1c_fits(c.nd, c.nfun, w, c.igauge) ? w : -1;
+  return 0;
+}
+
 int h1_factor(Ctx& c, cplx fac, H1Fac* out) {
   for (int i = 0; i < c.n_h1; ++i)
     if (c.h1slot[i].cre == fac.x && c.h1slot[i].cim == fac.y) { *out = c.h1slot[i].f; return 0; }
@@ -1795,6 +1820,7 @@ int h1_factor(Ctx& c, cplx fac, H1Fac* out) {
   src.Nr = c.Nr; src.L1 = c.L1; src.nd = c.nd; src.nfe = c.nfe; src.c = fac;
   src.radk = c.radk; src.radk0 = c.radk0; src.tdiag = c.tdiag; src.status = c.d_status;
   int rc = launch_h1fac(src, sl->f, c.st);
+  if (!rc) rc = h1c_build(c, sl->f);
   *out = sl->f;
   return rc ? ST_CUDA : 0;
 }
@@ -1805,11 +1831,18 @@ int h1_bufs(Ctx& c) {
   if (c.nfun - c.nfcore > 64 || h1elem_smem(c.nd, c.nfun) > 220 * 1024) return ST_CONFIG;
   c.h1_z[0] = dalloc<cplx>(nrow * c.nfe * (c.nd - 1));
   c.h1_z[1] = dalloc<cplx>(nrow * c.nfe * (c.nd - 1));
-  c.h1_cb = dalloc<cplx>(nrow * c.nfe * 2);
+  c.h1_cb[0] = dalloc<cplx>(nrow * c.nfe * 2);
+  c.h1_cb[1] = dalloc<cplx>(nrow * c.nfe * 2);
   c.h1_xb = dalloc<cplx>(nrow * std::max(1, c.nfe - 1));
   c.h1_partial = dalloc<double>(h1elem_partials(c.nfe, c.L1));
   c.h1_ticket = dalloc<unsigned>(1);  // zero (dalloc clears)
-  c.h1_flags = dalloc<int>(3);
+  c.h1_flags = dalloc<int>(4);
+  c.h1_pf = dalloc<double>((size_t)c.nfe * h1c_band_size(c.nd));
+  c.h1_tf = dalloc<double>((size_t)c.nfe * h1c_band_size(c.nd));
+  std::vector<double> rinv(c.h_xrad.size(), 0.0);
+  for (size_t k = 1; k < rinv.size(); ++k) rinv[k] = 1.0 / c.h_xrad[k];
+  c.h1_rinv = dupload(rinv);
+  if (launch_h1c_bands(c.nfe, c.nd, c.Nr, c.radp, c.radk0, c.h1_pf, c.h1_tf, c.st)) return ST_CUDA;
   return 0;
 }
 
@@ -1839,6 +1872,76 @@ int h1_apply(Ctx& c, bool pade, const double* d_lf, cplx* wfn, double dtime, cpl
   return h1_run(c, pade, fac, zf0, true, d_lf, wfn, maxcyc, thresh);
 }
 
+// h1_run on the folded passes: a first pass, then the correction cycles (one launch each) or the only solve
+constexpr int kH1Unroll = 4;
+int h1c_run(Ctx& c, bool pade, const H1Fac& F, cplx zf0, bool allow_cycles, const double* d_lf, cplx* wfn, int maxcyc,
+            double thresh) {
+  cudaStream_t st = c.st;
+  int rc = 0;
+  H1CycArgs E{};
+  E.fac = F; E.Nr = c.Nr; E.L1 = c.L1; E.nfun = c.nfun; E.nfcore = c.nfcore; E.mmax1 = c.mmax1; E.igauge = c.igauge;
+  E.radk = c.radk; E.tdiag = c.tdiag; E.xrad = c.xrad; E.rinv = c.h1_rinv; E.alph = c.alph; E.lfield = d_lf; E.pf = c.h1_pf; E.tf = c.h1_tf;
+  for (int k = 0; k < 2; ++k) { E.z[k] = c.h1_z[k]; E.cb[k] = c.h1_cb[k]; }
+  E.torb = wfn; E.in = wfn; E.thresh = thresh; E.norm_div = (double)c.nfun; E.partial = c.h1_partial; E.ticket = c.h1_ticket;
+  E.flags = c.h1_flags; E.maxcyc = maxcyc;
+  for (int f = 0; f < c.nfun && f < 16; ++f) E.mv[f] = c.mval[f];
+  // h1itr also solves the frozen-core columns once: their first correction
+  // enters the residual norm of the first cycle (h1itr_prop.F90:105-129)
+  E.f_first = pade ? c.nfcore : 0;
+  // first right-hand side: wfn (dpade) or wfn + zfac1 (T + zfield V) wfn (h1itr)
+  E.a = mkc(1, 0);
+  E.b = pade ? mkc(0, 0) : zf0;
+  E.cz0 = (!pade && c.isplit == 1) ? zf0 : mkc(0, 0);
+  rc |= launch_h1c(E, 0, st);
+  c.launches++;
+  const bool cycles = c.isplit == 1 && maxcyc > 0 && allow_cycles;
+  E.a = mkc(0, 0); E.b = mkc(0, 0); E.cz0 = zf0; E.in = nullptr;
+  if (cycles) {
+    // maxcyc cycles and the pass that only adds the last correction; a pass after the residual norm fell below
+    // thresh returns at once.  Inside a capture kH1Unroll passes stand in a row and a conditional loop takes
+    // the rest.  The loop costs 10 us even when it does not run and 6 us more per turn (measured with empty
+    // bodies), a pass that returns at once 0.7 us (He) to 2 us (Ne).  Eight split steps of He (3 cycles each
+    // half step), Ne (6) and an ensemble's, us, by kH1Unroll: 1: 2710, 6640, 11000; 3: 2573, 6690, 10500;
+    // 4: 2570, 6675, 10390; 6: 2614, 6655, 10170; 8: 2652, 6645, 10150; 24 (no loop): 2680, 6810, 10400.
+    const int total = maxcyc + 1;
+    cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
+    cudaGraph_t g = nullptr;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t ndep = 0;
+    if (cudaStreamGetCaptureInfo(st, &cst, nullptr, &g, &deps, &ndep) != cudaSuccess) return ST_CUDA;
+    const bool loop = cst == cudaStreamCaptureStatusActive && total > kH1Unroll;
+    if (loop && cudaGraphConditionalHandleCreate(&E.loop, g, 0, cudaGraphCondAssignDefault) != cudaSuccess) return ST_CUDA;
+    const int row = loop ? kH1Unroll : total;
+    for (int k = 0; k < row; ++k) {
+      E.use_loop = loop && k == row - 1;
+      rc |= launch_h1c(E, 1, st);
+    }
+    c.launches += row;
+    if (loop) {
+      cudaGraphNodeParams np{};
+      np.type = cudaGraphNodeTypeConditional;
+      np.conditional.handle = E.loop;
+      np.conditional.type = cudaGraphCondTypeWhile;
+      np.conditional.size = 1;
+      cudaGraphNode_t node;
+      if (cudaStreamGetCaptureInfo(st, &cst, nullptr, &g, &deps, &ndep) != cudaSuccess) return ST_CUDA;
+      if (cudaGraphAddNode(&node, g, deps, ndep, &np) != cudaSuccess) return ST_CUDA;
+      cudaGraph_t body = np.conditional.phGraph_out[0];
+      if (cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies) != cudaSuccess) return ST_CUDA;
+      if (cudaStreamBeginCaptureToGraph(c.st4, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
+        return ST_CUDA;
+      rc |= launch_h1c(E, 1, c.st4);
+      cudaGraph_t body_out = nullptr;
+      if (cudaStreamEndCapture(c.st4, &body_out) != cudaSuccess) return ST_CUDA;
+      c.launches++;
+    }
+  } else {
+    rc |= launch_h1c(E, 2, st);
+    c.launches++;
+  }
+  return rc ? ST_CUDA : 0;
+}
+
 // h1itr (pade false) or the shifted inverse (1 + fac (T + V))^-1 (pade true)
 // of the non-frozen orbitals, the laser by correction cycles of factor
 // zf0 lfield[2] when isplit is 1 and allow_cycles
@@ -1850,10 +1953,11 @@ int h1_run(Ctx& c, bool pade, cplx fac, cplx zf0, bool allow_cycles, const doubl
   H1Fac F;
   rc = h1_factor(c, fac, &F);
   if (rc) return rc;
+  if (F.w >= 0 && h1c_fits(c.nd, c.nfun, F.w, c.igauge)) return h1c_run(c, pade, F, zf0, allow_cycles, d_lf, wfn, maxcyc, thresh);
   H1ElemArgs E{};
   E.fac = F; E.Nr = c.Nr; E.L1 = c.L1; E.nfun = c.nfun; E.nfcore = c.nfcore; E.mmax1 = c.mmax1; E.igauge = c.igauge;
   E.mval = c.d_mval; E.radk = c.radk; E.radk0 = c.radk0; E.radp = c.radp; E.tdiag = c.tdiag; E.xrad = c.xrad;
-  E.alph = c.alph; E.lfield = d_lf; E.cb = c.h1_cb; E.xb = c.h1_xb; E.torb = wfn;
+  E.alph = c.alph; E.lfield = d_lf; E.cb = c.h1_cb[0]; E.xb = c.h1_xb; E.torb = wfn;
   E.thresh = thresh; E.norm_div = (double)c.nfun; E.partial = c.h1_partial; E.ticket = c.h1_ticket;
   E.done = c.h1_flags; E.ncyc = c.h1_flags + 1;
   E.iter = c.h1_flags + 2; E.zb0 = c.h1_z[0]; E.zb1 = c.h1_z[1]; E.iter_mode = 0;

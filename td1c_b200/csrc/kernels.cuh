@@ -320,6 +320,11 @@ struct H1Fac {
   cplx* tdu = nullptr;   //   first and
   cplx* tdu2 = nullptr;  //   second superdiagonal of U
   int* tpiv = nullptr;   // [L1][nb] row interchanges
+  // the folded passes (h1cycle.cu); w < 0: not built, the two-launch passes run
+  cplx* af = nullptr;    // [L1][nfe][h1c_af_size] interior inverse and bridge-share rows, fragment order
+  cplx* glr = nullptr;   // [L1][nfe][2][ni]: GL, GR
+  cplx* sinv = nullptr;  // [L1][nb][nb] inverse of the bridge matrix
+  int w = -1;            // half-width of the band of sinv that is used
 };
 struct H1FacSrc {
   int Nr, L1, nd, nfe;
@@ -376,6 +381,41 @@ int launch_h1elem(const H1ElemArgs& a, cudaStream_t st);
 // norm is not below thresh (*done == 0) and *iter < maxcyc
 int launch_h1loop_ctl(int* iter, const int* done, int maxcyc, cudaGraphConditionalHandle h, cudaStream_t st);
 int launch_h1bridge(const H1ElemArgs& a, cudaStream_t st);
+// The folded passes of h1cycle.cu: one launch per pass, z in [l][element][orbital][point] and the bridge
+// shares in [l][element][side][orbital], two buffers of each by the cycle's parity
+constexpr int H1C_WMAX = 8;  // widest band of the bridge inverse the folded passes take
+struct H1CycArgs {
+  H1Fac fac;
+  int Nr, L1, nfun, nfcore, mmax1, igauge;
+  int f_first;           // first orbital of the first right-hand side
+  int maxcyc, use_loop;
+  const double* radk;
+  const double* tdiag;
+  const double* xrad;    // [nrad + 1] radial points and
+  const double* rinv;    //   their reciprocals
+  const double* alph;
+  const double* lfield;  // device lfield (may be null: no laser term)
+  const double* pf;      // [nfe][h1c_band_size] derivative and kinetic blocks, fragment order
+  const double* tf;
+  cplx a, b, cz0;
+  const cplx* in;
+  cplx* z[2];
+  cplx* cb[2];
+  cplx* torb;
+  double thresh, norm_div;
+  double* partial;
+  unsigned* ticket;
+  int* flags;            // [0] residual norm below thresh, [1] corrections solved, [2] cycles run
+  int mv[16];
+  cudaGraphConditionalHandle loop;  // use_loop: the graph's loop around the cycle
+};
+size_t h1c_af_size(int nd);
+size_t h1c_band_size(int nd);
+int launch_h1c_bands(int nfe, int nd, int Nr, const double* radp, const double* radk0, double* pf, double* tf, cudaStream_t st);
+int launch_h1c_setup(const H1Fac& f, int* w, cudaStream_t st);
+bool h1c_fits(int nd, int nfun, int w, int igauge);
+int launch_h1c(const H1CycArgs& a, int mode, cudaStream_t st);  // mode 0 first pass, 1 cycle, 2 the only solve
+
 size_t h1elem_smem(int nd, int nfun);
 size_t h1elem_partials(int nfe, int L1);
 

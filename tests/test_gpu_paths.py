@@ -61,3 +61,45 @@ def test_folded_and_dense_transforms(cuda_ok, lmax, nlat):
         ang["legf2"] = t
     dense = _rhs_parity(wl, move)
     assert rel_err(folded, dense) < TOL
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("igauge", [0, 1])
+@pytest.mark.parametrize("nfe,ndvr,dtime", [(1, 10, 0.01), (2, 7, 0.01), (9, 7, 0.005), (9, 8, 3.0), (14, 6, 0.2), (14, 6, 2.0), (6, 20, 0.004)])
+def test_one_body_step_band(cuda_ok, igauge, nfe, ndvr, dtime):
+    """Grids without a bridge, with one, and steps whose bridge inverse is a narrow band, a wide one, or not
+    a band at all (the long steps)."""
+    wl = dict(W.MIXED_SMALL, nfe=nfe, ndvr=ndvr, rmax=1.75 * nfe, rmask=1.4 * nfe, igauge=igauge, split_type=1)
+    import torch
+    o, h, orb, cic = _pair(wl)
+    try:
+        lf = _field(wl) * (0.01 if dtime > 0.1 else 1.0)  # the correction cycles converge for a short step or a weak field
+        wo, no = o.h1itr_prop(lf, dtime, orb, 20, 1e-10)
+        d = torch.from_numpy(orb.reshape(-1).copy()).cuda()
+        ng = h.h1itr_dev(d.data_ptr(), lf, dtime, 20, 1e-10)
+        assert rel_err(d.cpu().numpy(), wo) < TOL and ng == no
+        wo, no = o.dpade_prod(lf, dtime, orb, 2.0, 20, 1e-10)
+        d = torch.from_numpy(orb.reshape(-1).copy()).cuda()
+        ng = h.dpade_dev(d.data_ptr(), lf, dtime, 2.0, 20, 1e-10)
+        assert rel_err(d.cpu().numpy(), wo) < TOL and ng == no
+    finally:
+        h.final()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("maxcyc,thresh", [(0, 1e-10), (1, 0.0), (2, 0.0), (3, 0.0), (4, 0.0), (20, 0.0), (20, 1e-10)])
+def test_correction_cycle_limits(cuda_ok, maxcyc, thresh):
+    """Cycle limits below, at and above the passes that stand in a row in a captured step (threshold 0: all
+    of them run), eager and captured steps alike."""
+    import torch
+    wl = dict(W.MIXED_SMALL, igauge=1, split_type=1)
+    o, h, orb, cic = _pair(wl)
+    try:
+        wo, co, _ = o.split2(orb, cic, 30.0, 0.004, 3, maxcyc, thresh)
+        for graph in (True, False):
+            x, c = torch.from_numpy(orb.reshape(-1).copy()).cuda(), torch.from_numpy(cic.copy()).cuda()
+            h.split2_dev(x.data_ptr(), c.data_ptr(), 30.0, 0.004, 3, maxcyc=maxcyc, thresh=thresh, use_graph=graph)
+            h.sync()
+            assert rel_err(x.cpu().numpy(), wo) < TOL and rel_err(c.cpu().numpy(), co) < TOL
+    finally:
+        h.final()
