@@ -1240,70 +1240,90 @@ int build_reductions(Ctx& c) {
     c.a2_nblk = (int)blks.size(); c.a2_nrow = (int)rws.size(); c.a2_ncol = (int)cls.size(); c.a2_ncoef = coff;
     c.a2_blk = dupload(blks); c.a2_rows = dupload(rws); c.a2_cols = dupload(cls); c.a2_map = dupload(map);
     c.a2_coef = dalloc<cplx>(std::max(1, coff));
-    // the tensor-core form: per Delta one block (rows not chunked) over the
-    // same rows list; coefficients C[row][kl] at coff + row pa + kl with pa
-    // = 4 mod 8 (double2) and zero padding; padded columns read the zero W row
+    // the tensor-core form: per |Delta m| one real block.  With W(k, l) = Wr + i Wi the stored pair and
+    // W(l, k) its conjugate, the terms c W(k, l) + c' W(l, k) of a row are (c + c') Wr + i (c - c') Wi, so
+    // a row is two real rows (re, im) over the depth (Wr, Wi) of each stored pair: half the products of the
+    // complex form over ordered pairs where a row takes both orders (m_k = m_l), and rows of -Delta share
+    // the columns of +Delta.  Coefficients C[2 row + part][2 pair + part] at coff + row pa + column, pa = 4
+    // or 12 mod 16 (doubles), zero padding; padded pairs read the zero W row
     std::vector<MfdBlock> dblk;
-    std::vector<int2> dcol;
-    std::vector<Act2Coef> dmap;
+    std::vector<int> dcol;
+    std::vector<MfdCoef> dmap;
+    std::vector<int2> drows;
     int dcoff = 0;
-    for (size_t b0 = 0; b0 < blks.size();) {
-      size_t b1 = b0;  // the row chunks of one Delta share col0
-      int nr = 0;
-      while (b1 < blks.size() && blks[b1].col0 == blks[b0].col0) nr += blks[b1++].nrow;
-      const Act2Block& B = blks[b0];
+    for (int d = 0; d <= dmax && n > 0; ++d) {
+      std::vector<int> pp;
+      for (int q = 0; q < c.npair; ++q)
+        if (c.pa[q] >= nc && c.pb[q] >= nc && std::abs(c.mval[c.pb[q]] - c.mval[c.pa[q]]) == d) pp.push_back(q);
       MfdBlock db{};
-      db.kpad = (B.ncol + 3) / 4 * 4;
-      db.pa = db.kpad % 8 == 0 ? db.kpad + 4 : db.kpad;
-      db.mt = (nr + 7) / 8; db.col0 = (int)dcol.size(); db.drow0 = B.row0; db.nr = nr; db.coff = dcoff;
-      for (int y = 0; y < db.kpad; ++y) dcol.push_back(y < B.ncol ? cls[B.col0 + y] : make_int2(c.npair, 0));
-      for (size_t bb = b0; bb < b1; ++bb)
-        for (int y = 0; y < blks[bb].ncol; ++y)
-          for (int x = 0; x < blks[bb].nrow; ++x) {
-            // the chunk's map entry (y, x) sits at coff + y nrow + x, like its slot
-            Act2Coef m{};
-            m.d2idx = map[blks[bb].coff + y * blks[bb].nrow + x].d2idx;
-            m.dst = dcoff + (blks[bb].row0 + x - B.row0) * db.pa + y;
-            dmap.push_back(m);
-          }
+      db.drow0 = (int)drows.size();
+      for (int sg = 1; sg >= (d ? -1 : 1); sg -= 2)
+        for (int ia = 0; ia < n; ++ia)
+          for (int ja = 0; ja <= ia; ++ja)
+            if (c.mval[nc + ia] - c.mval[nc + ja] == sg * d) drows.push_back(make_int2(ia, ja));
+      db.nr = (int)drows.size() - db.drow0;
+      if (!db.nr || pp.empty()) { drows.resize(db.drow0); continue; }
+      const int npp = ((int)pp.size() + 1) / 2 * 2;
+      db.kpad = 2 * npp;
+      db.pa = db.kpad;
+      while (db.pa % 16 != 4 && db.pa % 16 != 12) db.pa += 4;
+      db.mt = (2 * db.nr + 7) / 8; db.col0 = (int)dcol.size(); db.coff = dcoff;
+      for (int y = 0; y < npp; ++y) dcol.push_back(y < (int)pp.size() ? pp[y] : c.npair);
+      for (int r = 0; r < db.nr; ++r) {
+        const int ia = drows[db.drow0 + r].x, ja = drows[db.drow0 + r].y, dm = c.mval[nc + ia] - c.mval[nc + ja];
+        for (size_t y = 0; y < pp.size(); ++y) {
+          const int x0 = c.pa[pp[y]] - nc, x1 = c.pb[pp[y]] - nc, dp = c.mval[nc + x1] - c.mval[nc + x0];
+          MfdCoef m{-1, -1, dcoff + 2 * r * db.pa + 2 * (int)y, db.pa};
+          if (dp == dm) m.w = ja + n * (ia + n * (x1 + n * x0));                    // (k, l) = (x0, x1)
+          if (x0 != x1 && -dp == dm) m.wc = ja + n * (ia + n * (x0 + n * x1));  // (k, l) = (x1, x0)
+          dmap.push_back(m);
+        }
+      }
       dcoff += db.mt * 8 * db.pa;
       dblk.push_back(db);
-      b0 = b1;
     }
     // per target x the D2V rows in row order: (row, other orbital), conj flag in bit 16
     std::vector<int2> elist;
     std::vector<int> eoff(n + 1, 0);
     for (int x = 0; x < n; ++x) {
       eoff[x] = (int)elist.size();
-      for (size_t r = 0; r < rws.size(); ++r) {
-        if (rws[r].x == x) elist.push_back(make_int2((int)r, rws[r].y));
-        else if (rws[r].y == x && rws[r].x > rws[r].y) elist.push_back(make_int2((int)r, rws[r].x | (1 << 16)));
+      for (size_t r = 0; r < drows.size(); ++r) {
+        if (drows[r].x == x) elist.push_back(make_int2((int)r, drows[r].y));
+        else if (drows[r].y == x && drows[r].x > drows[r].y) elist.push_back(make_int2((int)r, drows[r].x | (1 << 16)));
       }
     }
     eoff[n] = (int)elist.size();
-    // (block, m-tile) items over the 4 warps of a CTA, longest first to the
-    // least loaded warp; at most 8 per warp
-    std::vector<std::pair<int, int2>> items;
-    for (size_t b = 0; b < dblk.size(); ++b)
-      for (int mt = 0; mt < dblk[b].mt; ++mt) items.push_back({dblk[b].kpad / 4, make_int2((int)b, mt)});
-    std::stable_sort(items.begin(), items.end(), [](const std::pair<int, int2>& x, const std::pair<int, int2>& y) { return x.first > y.first; });
-    int wload[4] = {0, 0, 0, 0}, wcount[4] = {0, 0, 0, 0};
-    bool items_fit = items.size() <= 32;
-    for (int w = 0; w < 4; ++w)
-      for (int k = 0; k < 8; ++k) c.mf.witem[w][k] = make_int2(-1, -1);
-    for (size_t k = 0; k < items.size() && items_fit; ++k) {
-      int best = -1;
-      for (int w = 0; w < 4; ++w)
-        if (wcount[w] < 8 && (best < 0 || wload[w] < wload[best])) best = w;
-      c.mf.witem[best][wcount[best]++] = items[k].second;
-      wload[best] += items[k].first;
+    // items (block, up to MFD_MI m-tiles, n-tile) over the warps of a CTA, longest first to the least loaded
+    std::vector<std::pair<int, int4>> items;
+    for (size_t b = 0; b < dblk.size(); ++b) {
+      const int ng = (dblk[b].mt + MFD_MI - 1) / MFD_MI;
+      for (int gq = 0; gq < ng; ++gq) {
+        const int m0 = dblk[b].mt * gq / ng, m1 = dblk[b].mt * (gq + 1) / ng;
+        for (int t = 0; t < MFD_TQ / 8; ++t) items.push_back({(m1 - m0) * dblk[b].kpad / 4, make_int4((int)b, m0, m1 - m0, t)});
+      }
     }
-    c.mf.dmma = n > 0 && !dblk.empty() && items_fit;
+    std::stable_sort(items.begin(), items.end(), [](const std::pair<int, int4>& x, const std::pair<int, int4>& y) { return x.first > y.first; });
+    std::vector<std::vector<int4>> wl(MFD_NT / 32);
+    std::vector<int> wload(MFD_NT / 32, 0), ioff;
+    for (auto& it : items) {
+      int best = 0;
+      for (int w = 1; w < MFD_NT / 32; ++w)
+        if (wload[w] < wload[best]) best = w;
+      wl[best].push_back(it.second);
+      wload[best] += it.first;
+    }
+    std::vector<int4> witem;
+    for (auto& v : wl) {
+      ioff.push_back((int)witem.size());
+      witem.insert(witem.end(), v.begin(), v.end());
+    }
+    ioff.push_back((int)witem.size());
+    c.mf.dmma = n > 0 && !dblk.empty();
     c.mf.nblk_d = (int)dblk.size(); c.mf.ndcol = (int)dcol.size(); c.mf.ncoef_d = dcoff; c.mf.nelist = (int)elist.size();
+    c.mf.nrow_d = (int)drows.size(); c.mf.nmap_d = (int)dmap.size(); c.mf.nitem = (int)witem.size();
     c.mf.dblk = dupload(dblk); c.mf.dcol = dupload(dcol); c.mf.dmap = dupload(dmap); c.mf.elist = dupload(elist);
-    c.mf.eoff = dupload(eoff);
-    c.mf.dcoef = dalloc<cplx>(std::max(1, dcoff));
-    cudaMemset(c.mf.dcoef, 0, sizeof(cplx) * std::max(1, dcoff));
+    c.mf.eoff = dupload(eoff); c.mf.witem = dupload(witem); c.mf.ioff = dupload(ioff);
+    c.mf.dcoef = dalloc<double>(std::max(1, dcoff));
   }
   // mean-field action arguments (fixed buffers; the tensor maps bind W and orbg)
   MfprodArgs& mf = c.mf;

@@ -184,12 +184,17 @@ struct Act2Block {     // one dense (ij) x (kl) block of the 2-RDM contraction
   int coff, pad0, pad1, pad2;  // coefficient offset, coef[coff + kl * nrow + ij]
 };
 struct Act2Coef { int d2idx, dst; };  // den2 element -> coefficient slot
-// one Delta-m block of the act2 contraction on the FP64 tensor cores:
-// coefficients C[row][kl] padded to mt m-tiles of 8 rows x kpad (multiple of
-// 4) columns, row pitch pa (double2, 4 mod 8) from coff; columns
-// dcol[col0 .. col0+kpad) (padding: the zero W row npair); D2V rows
-// drow0 .. drow0+nr
+// one |Delta m| block of the act2 contraction on the FP64 tensor cores, in real
+// form: coefficients C[2 row + part][2 pair + part] in mt m-tiles of 8 real rows
+// x kpad real columns, row pitch pa (doubles) from coff; stored pairs
+// dcol[col0 .. col0 + kpad / 2) (padding: the zero W row npair); D2V rows
+// drow0 .. drow0 + nr
 struct MfdBlock { int coff, pa, mt, kpad, col0, drow0, nr, pad; };
+// den2 elements that multiply a stored pair's W and its conjugate in a row (-1: none) -> the 2 x 2 block at dst
+struct MfdCoef { int w, wc, dst, pa; };
+constexpr int MFD_TQ = 16;   // points per tile (2 n-tiles)
+constexpr int MFD_NT = 256;  // threads
+constexpr int MFD_MI = 3;    // m-tiles of one warp item
 struct MfprodArgs {
   size_t ngrid;
   int nfun, npair;
@@ -214,15 +219,16 @@ struct MfprodArgs {
   cplx* coef;
   // tensor-core form of act2 (used when dmma != 0): its own padded
   // coefficient layout and map, per-target epilogue lists
-  int dmma, nblk_d, ndcol, ncoef_d, nelist;
+  int dmma, nblk_d, ndcol, ncoef_d, nelist, nrow_d, nmap_d, nitem;
   int max_cta;          // cap of the persistent DMMA grid (0: as many CTAs as are resident)
   const MfdBlock* dblk;
-  const int2* dcol;       // (pair, conj) of every padded column
-  const Act2Coef* dmap;   // den2 element -> padded coefficient slot
-  cplx* dcoef;            // [ncoef_d]
+  const int* dcol;        // stored pair of every padded pair column
+  const MfdCoef* dmap;    // [nmap_d]
+  double* dcoef;          // [ncoef_d]
   const int2* elist;      // per active target x: (D2V row, other orbital | conj << 16), in row order
   const int* eoff;        // [nact + 1] offsets into elist
-  int2 witem[4][8];       // per warp: (block, m-tile) items, -1 ends the list
+  const int4* witem;      // (block, first m-tile, m-tiles, n-tile) of every warp, in warp order
+  const int* ioff;        // [warps + 1] offsets into witem
 };
 int launch_mfprod(const MfprodArgs& a, cudaStream_t st);
 

@@ -166,28 +166,22 @@ __global__ void __launch_bounds__(MF_TQ) mfprod_kernel(MfprodArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// act2 on the FP64 tensor cores.  Persistent CTAs of 4 warps (2 per SM)
-// load the padded coefficients and the plan tables once, then loop over
-// tiles of MFD_TQ grid points:
-//   1. cp.async stages the tile's slice of every stored pair's W (rows of
-//      MFD_TQ points, pitch MFD_WP) and the orbitals in shared memory; row
-//      npair of the W slice is zero.
+// act2 on the FP64 tensor cores.  Persistent CTAs of 8 warps load the real
+// coefficients (MfdBlock) and the plan tables once, then loop over tiles of
+// MFD_TQ grid points:
+//   1. cp.async stages the tile's slice of every stored pair's W (pitch MFD_WP)
+//      and the orbitals in shared memory; row npair of the W slice is zero.
 //   2. core terms (fcx1, dcj, dcx into gorbg; actj, actx into v2orbg of the
 //      dynamic cores) over (point, orbital) items.
-//   3. D2V[ij][pt] = sum_kl C[ij][kl] W(kl)[pt] per block as
-//      mma.sync.m8n8k4.f64 tiles (rows ij, columns points, depth kl) with
-//      four real products per complex step, stored to shared memory.
-//   4. twfn_x[pt] from the target's D2V rows (in row order, as the
-//      reference's loop), then v2orbg_k = sum_x rden(x, k) twfn_x.
+//   3. D2V[2 ij + part][pt] = sum C[2 ij + part][2 p + part'] W[p][pt].part' per
+//      block as mma.sync.m8n8k4.f64 tiles (real rows, columns points, depth the
+//      real and imaginary parts of the stored pairs); each warp runs its items
+//      of up to MFD_MI m-tiles, which share the W fragments.
+//   4. twfn_x[pt] from the target's D2V rows (in row order), then
+//      v2orbg_k = sum_x rden(x, k) twfn_x.
 // ---------------------------------------------------------------------------
-constexpr int MFD_TQ = 16;              // points per CTA (2 n-tiles): 3 CTAs per SM
-constexpr int MFD_WP = MFD_TQ + 2;      // double2 pitch of a W row: rows 8 banks apart
-// double2 pitch of a D2V row: odd, so the 8 rows x 4 column pairs of one
-// fragment store fall on 8 different 16-byte bank groups (4 wavefronts, the
-// minimum for 512 bytes; a pitch of MFD_TQ put all 8 rows on one group)
-constexpr int MFD_DP = MFD_TQ + 1;
-constexpr int MFD_NT = 128;             // threads
-constexpr int MFD_MAXB = 16, MFD_MAXCOL = 256, MFD_MAXROW = 128, MFD_MAXE = 512;
+constexpr int MFD_WP = MFD_TQ + 4;  // double2 pitch of a W row: the 4 depths x 4 columns of a half-warp's loads fall in distinct banks
+constexpr int MFD_DP = MFD_TQ + 1;  // double2 pitch of a D2V row (odd: the 2 rows x 2 parts x 4 points of a half-warp's stores too)
 
 __device__ __forceinline__ void mfd_dmma(double& c0, double& c1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
@@ -200,29 +194,65 @@ __device__ __forceinline__ void mfd_cp16(void* dst, const void* src, unsigned by
                : "memory");
 }
 
-static size_t mfd_smem_bytes(const MfprodArgs& a) {
-  return sizeof(cplx) * ((size_t)(a.npair + 1) * MFD_WP + (size_t)a.ncoef_d + 2 * (size_t)a.nfun * MFD_TQ +
-                         (size_t)a.nrow * MFD_DP + (size_t)a.nact * MFD_TQ);
-}
-static bool mfd_fits(const MfprodArgs& a) {
-  return a.dmma && a.nfun <= MF_MAXF && a.nblk_d <= MFD_MAXB && a.ndcol <= MFD_MAXCOL && a.nrow <= MFD_MAXROW &&
-         a.nelist <= MFD_MAXE && mfd_smem_bytes(a) <= 200 * 1024;
+// dcoef from den2 (elements below thrwfn left out)
+__global__ void mfd_fill_kernel(int n, const MfdCoef* __restrict__ map, const cplx* __restrict__ den2, double* __restrict__ coef) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const MfdCoef m = map[e];
+  auto get = [&](int i) {
+    const cplx d = i >= 0 ? den2[i] : mkc(0.0, 0.0);
+    return sqrt(cabs2(d)) > 1.0e-15 ? d : mkc(0.0, 0.0);  // thrwfn (mod_const.F90:32)
+  };
+  const cplx a = get(m.w), b = get(m.wc);
+  *reinterpret_cast<double2*>(coef + m.dst) = make_double2(a.x + b.x, b.y - a.y);
+  *reinterpret_cast<double2*>(coef + m.dst + m.pa) = make_double2(a.y + b.y, a.x - b.x);
 }
 
-__global__ void __launch_bounds__(MFD_NT) mfprod_dmma_kernel(MfprodArgs a) {
-  extern __shared__ __align__(16) cplx mfd_smem[];
+// The contraction in real form: a row's two parts over the depth (Wr, Wi) of each stored pair, where the
+// complex form over ordered pairs did every product twice.  What bounds it: a tile's phases (DMMA, then the
+// FFMA twfn and v2orbg sums) follow one another inside a CTA, so its warps wait at the barriers between
+// them; three CTAs of 256 threads per SM fill part of that.  Ne, CAS(8e,9o), 136080 points: 112 -> 81 us.
+struct MfdSmem {
+  int nfun, nact, npair, nrow, ncoef, nelist, ndcol, nblk, nitem;
+  __host__ __device__ size_t w() const { return 0; }                                       // complex units
+  __host__ __device__ size_t phi() const { return w() + (size_t)(npair + 1) * MFD_WP; }
+  __host__ __device__ size_t d() const { return phi() + 2 * (size_t)nfun * MFD_TQ; }
+  __host__ __device__ size_t tw() const { return d() + (size_t)nrow * MFD_DP; }
+  __host__ __device__ size_t rden() const { return tw() + (size_t)nact * MFD_TQ; }
+  __host__ __device__ size_t den1() const { return rden() + (size_t)nact * nact; }
+  __host__ __device__ size_t item() const { return den1() + (size_t)nact * nact; }
+  __host__ __device__ size_t c() const { return item() + nitem; }
+  __host__ __device__ size_t blk() const { return c() + (size_t)(ncoef + 1) / 2; }
+  __host__ __device__ size_t el() const { return 2 * (blk() + 2 * (size_t)nblk); }         // 8-byte units
+  __host__ __device__ size_t ints() const { return 2 * (el() + nelist); }                  // 4-byte units: dcol, eoff, pair, mval, ioff
+  __host__ __device__ size_t bytes() const {
+    return 4 * (ints() + ndcol + nact + 1 + (size_t)nfun * nfun + nfun + MFD_NT / 32 + 1);
+  }
+};
+static MfdSmem mfd_smem(const MfprodArgs& a) {
+  return MfdSmem{a.nfun, a.nact, a.npair, a.nrow_d, a.ncoef_d, a.nelist, a.ndcol, a.nblk_d, a.nitem};
+}
+static bool mfd_fits(const MfprodArgs& a) { return a.dmma && a.nfun <= MF_MAXF && mfd_smem(a).bytes() <= 220 * 1024; }
+
+__global__ void __launch_bounds__(MFD_NT, 3) mfprod_dmma_kernel(MfprodArgs a) {
+  extern __shared__ __align__(16) cplx mfd_sm[];
   const int nact = a.nact, ncore = a.ncore, nfcore = a.nfcore, nfun = a.nfun, npair = a.npair;
-  cplx* sW = mfd_smem;                                   // [npair + 1][WP]
-  cplx* sC = sW + (size_t)(npair + 1) * MFD_WP;          // [ncoef_d]
-  cplx* sPhi2 = sC + a.ncoef_d;                          // 2 x [nfun][TQ]: this tile's and the next
-  cplx* sD = sPhi2 + 2 * (size_t)nfun * MFD_TQ;          // [nrow][DP]
-  cplx* sTw = sD + (size_t)a.nrow * MFD_DP;              // [nact][TQ]
-  __shared__ MfdBlock sblk[MFD_MAXB];
-  __shared__ int2 scol[MFD_MAXCOL];
-  __shared__ int2 sel[MFD_MAXE];
-  __shared__ int seoff[MF_MAXF + 1];
-  __shared__ cplx srden[MF_MAXF * MF_MAXF], sden1[MF_MAXF * MF_MAXF];
-  __shared__ int spo[MF_MAXF * MF_MAXF], spc[MF_MAXF * MF_MAXF], smv[MF_MAXF];
+  const MfdSmem lay{nfun, nact, npair, a.nrow_d, a.ncoef_d, a.nelist, a.ndcol, a.nblk_d, a.nitem};
+  cplx* sW = mfd_sm + lay.w();        // [npair + 1][WP]
+  cplx* sPhi2 = mfd_sm + lay.phi();   // 2 x [nfun][TQ]: this tile's and the next
+  cplx* sD = mfd_sm + lay.d();        // [nrow][DP]
+  cplx* sTw = mfd_sm + lay.tw();      // [nact][TQ]
+  cplx* srden = mfd_sm + lay.rden();
+  cplx* sden1 = mfd_sm + lay.den1();
+  int4* sitem = reinterpret_cast<int4*>(mfd_sm + lay.item());
+  double* sC = reinterpret_cast<double*>(mfd_sm + lay.c());
+  MfdBlock* sblk = reinterpret_cast<MfdBlock*>(mfd_sm + lay.blk());
+  int2* sel = reinterpret_cast<int2*>(mfd_sm) + lay.el();
+  int* scol = reinterpret_cast<int*>(mfd_sm) + lay.ints();
+  int* seoff = scol + a.ndcol;
+  int* spo = seoff + nact + 1;        // [nfun][nfun] stored pair | conj << 16
+  int* smv = spo + nfun * nfun;
+  int* sioff = smv + nfun;
   const int tid = threadIdx.x;
   const size_t ng = a.ngrid;
   const bool do_act2 = a.nelact >= 2 && nact > 0 && a.nblk_d > 0;
@@ -230,15 +260,17 @@ __global__ void __launch_bounds__(MFD_NT) mfprod_dmma_kernel(MfprodArgs a) {
 
   // ---- once per CTA: coefficients and tables
   if (do_act2)
-    for (int e = tid; e < a.ncoef_d; e += MFD_NT) mfd_cp16(sC + e, a.dcoef + e, 16u);
+    for (int e = tid; e < a.ncoef_d / 2; e += MFD_NT) mfd_cp16(sC + 2 * e, a.dcoef + 2 * e, 16u);
   asm volatile("cp.async.commit_group;" ::: "memory");
   for (int e = tid; e < MFD_WP; e += MFD_NT) sW[(size_t)npair * MFD_WP + e] = mkc(0, 0);
   for (int e = tid; e < a.nblk_d; e += MFD_NT) sblk[e] = a.dblk[e];
+  for (int e = tid; e < a.nitem; e += MFD_NT) sitem[e] = a.witem[e];
   for (int e = tid; e < a.ndcol; e += MFD_NT) scol[e] = a.dcol[e];
   for (int e = tid; e < a.nelist; e += MFD_NT) sel[e] = a.elist[e];
   for (int e = tid; e <= nact; e += MFD_NT) seoff[e] = a.eoff[e];
+  for (int e = tid; e <= MFD_NT / 32; e += MFD_NT) sioff[e] = a.ioff[e];
   for (int e = tid; e < nact * nact; e += MFD_NT) { srden[e] = a.rden[e]; sden1[e] = a.den1[e]; }
-  for (int e = tid; e < nfun * nfun; e += MFD_NT) { spo[e] = a.pair_of[e]; spc[e] = a.pair_cj[e]; }
+  for (int e = tid; e < nfun * nfun; e += MFD_NT) spo[e] = (a.pair_of[e] & 0xffff) | (a.pair_cj[e] << 16);
   for (int e = tid; e < nfun; e += MFD_NT) smv[e] = a.mval[e];
 
   // a tile's W rows and orbitals; row npair of the W slice is zero.  The
@@ -273,9 +305,9 @@ __global__ void __launch_bounds__(MFD_NT) mfprod_dmma_kernel(MfprodArgs a) {
 
   auto PHI = [&](int f, int t) { return sPhi[(size_t)f * MFD_TQ + t]; };
   auto WXY = [&](int x, int y, int t) {  // W(x, y) at point t from the stored pair
-    const int e = x * nfun + y;
-    const cplx w = sW[(size_t)spo[e] * MFD_WP + t];
-    return spc[e] ? cconj(w) : w;
+    const int e = spo[x * nfun + y];
+    const cplx w = sW[(size_t)(e & 0xffff) * MFD_WP + t];
+    return (e >> 16) ? cconj(w) : w;
   };
   const int ndcore = ncore - nfcore;
   // ---- 2. core terms (same sums and order as mfprod_kernel)
@@ -323,43 +355,43 @@ __global__ void __launch_bounds__(MFD_NT) mfprod_dmma_kernel(MfprodArgs a) {
     stage(tile + gridDim.x, buf ^ 1);
     continue;
   }
-  // ---- 3. D2V tiles on the tensor cores: each warp runs its (block,
-  //      m-tile) items over all MFD_TQ / 8 n-tiles at once, the four real
-  //      products of each tile in separate accumulators
+  // ---- 3. D2V tiles on the tensor cores
   const int lane = tid & 31, warp = tid >> 5, gid = lane >> 2, tig = lane & 3;
-  constexpr int NT = MFD_TQ / 8;
-  for (int it = 0; it < 8; ++it) {
-    const int2 wi = a.witem[warp][it];
-    if (wi.x < 0) break;
+  for (int it = sioff[warp]; it < sioff[warp + 1]; ++it) {
+    const int4 wi = sitem[it];
     const MfdBlock B = sblk[wi.x];
-    const int mt = wi.y;
-    double acc[NT][4][2];
+    double acc[MFD_MI][2];
 #pragma unroll
-    for (int t = 0; t < NT; ++t)
+    for (int i = 0; i < MFD_MI; ++i) acc[i][0] = acc[i][1] = 0.0;
+    // m-tiles past the item's repeat its last one (their results are not stored)
+    const double* arow[MFD_MI];
 #pragma unroll
-      for (int h = 0; h < 4; ++h) acc[t][h][0] = acc[t][h][1] = 0.0;
-    const cplx* arow = sC + B.coff + (size_t)(mt * 8 + gid) * B.pa + tig;
-    for (int ks = 0; ks < B.kpad / 4; ++ks) {
-      const cplx av = arow[4 * ks];
-      const int2 pc = scol[B.col0 + 4 * ks + tig];
-      const cplx* wrow = sW + (size_t)pc.x * MFD_WP + gid;
+    for (int i = 0; i < MFD_MI; ++i) arow[i] = sC + B.coff + (size_t)((wi.y + min(i, wi.z - 1)) * 8 + gid) * B.pa + tig;
+    const double* wd = reinterpret_cast<const double*>(sW) + 2 * (wi.w * 8 + gid) + (tig & 1);
+    const int* col = scol + B.col0 + (tig >> 1);
+    const int ksn = B.kpad / 4;
+    if (wi.z == MFD_MI) {
+#pragma unroll 2
+      for (int ks = 0; ks < ksn; ++ks) {
+        const double bv = wd[(size_t)col[2 * ks] * (2 * MFD_WP)];
 #pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        const cplx bv = wrow[8 * t];
-        const double bi = pc.y ? -bv.y : bv.y;
-        mfd_dmma(acc[t][0][0], acc[t][0][1], av.x, bv.x);
-        mfd_dmma(acc[t][1][0], acc[t][1][1], av.y, -bi);
-        mfd_dmma(acc[t][2][0], acc[t][2][1], av.x, bi);
-        mfd_dmma(acc[t][3][0], acc[t][3][1], av.y, bv.x);
+        for (int i = 0; i < MFD_MI; ++i) mfd_dmma(acc[i][0], acc[i][1], arow[i][4 * ks], bv);
+      }
+    } else {
+#pragma unroll 2
+      for (int ks = 0; ks < ksn; ++ks) {
+        const double bv = wd[(size_t)col[2 * ks] * (2 * MFD_WP)];
+        mfd_dmma(acc[0][0], acc[0][1], arow[0][4 * ks], bv);
+        if (wi.z > 1) mfd_dmma(acc[1][0], acc[1][1], arow[1][4 * ks], bv);
       }
     }
-    const int r = mt * 8 + gid;
-    if (r < B.nr) {
 #pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        cplx* drow = sD + (size_t)(B.drow0 + r) * MFD_DP + t * 8 + 2 * tig;
-        drow[0] = mkc(acc[t][0][0] + acc[t][1][0], acc[t][2][0] + acc[t][3][0]);
-        drow[1] = mkc(acc[t][0][1] + acc[t][1][1], acc[t][2][1] + acc[t][3][1]);
+    for (int i = 0; i < MFD_MI; ++i) {
+      const int rr = (wi.y + i) * 8 + gid, r = rr >> 1;
+      if (i < wi.z && r < B.nr) {
+        double* drow = reinterpret_cast<double*>(sD + (size_t)(B.drow0 + r) * MFD_DP + wi.w * 8 + 2 * tig) + (rr & 1);
+        drow[0] = acc[i][0];
+        drow[2] = acc[i][1];
       }
     }
   }
@@ -369,6 +401,7 @@ __global__ void __launch_bounds__(MFD_NT) mfprod_dmma_kernel(MfprodArgs a) {
   for (int e = tid; e < nact * MFD_TQ; e += MFD_NT) {
     const int x = e / MFD_TQ, t = e % MFD_TQ;
     cplx tw = mkc(0, 0);
+#pragma unroll 4
     for (int k = seoff[x]; k < seoff[x + 1]; ++k) {
       const int2 en = sel[k];
       const cplx d = sD[(size_t)en.x * MFD_DP + t];
@@ -393,15 +426,15 @@ __global__ void __launch_bounds__(MFD_NT) mfprod_dmma_kernel(MfprodArgs a) {
 int launch_mfprod(const MfprodArgs& a, cudaStream_t st) {
   if (mfd_fits(a)) {
     const bool do_act2 = a.nelact >= 2 && a.nact > 0 && a.nblk_d > 0;
-    if (do_act2) act2_fill_kernel<<<(a.ncoef + 127) / 128, 128, 0, st>>>(a.ncoef, a.dmap, a.den2, a.dcoef);
-    const size_t smem = mfd_smem_bytes(a);
+    if (do_act2) mfd_fill_kernel<<<(a.nmap_d + 127) / 128, 128, 0, st>>>(a.nmap_d, a.dmap, a.den2, a.dcoef);
+    const size_t smem = mfd_smem(a).bytes();
     static bool attr = false;
     if (!attr) {
-      cudaFuncSetAttribute(mfprod_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      cudaFuncSetAttribute(mfprod_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
       attr = true;
     }
-    // persistent: as many CTAs as are resident at once (shared memory decides; at
-    // least 2 per SM), sized once per shared-memory footprint
+    // persistent: as many CTAs as are resident at once (shared memory decides),
+    // sized once per shared-memory footprint
     static int nsm = 0, cps = 0;
     static size_t cps_smem = 0;
     if (!nsm) {
@@ -410,8 +443,8 @@ int launch_mfprod(const MfprodArgs& a, cudaStream_t st) {
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     }
     if (cps_smem != smem) {
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cps, mfprod_dmma_kernel, MFD_NT, smem) != cudaSuccess) cps = 2;
-      cps = std::max(cps, 2);
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cps, mfprod_dmma_kernel, MFD_NT, smem) != cudaSuccess) cps = 1;
+      cps = std::max(cps, 1);
       cps_smem = smem;
     }
     const int ntile = (int)((a.ngrid + MFD_TQ - 1) / MFD_TQ);

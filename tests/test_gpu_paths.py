@@ -63,6 +63,25 @@ def test_folded_and_dense_transforms(cuda_ok, lmax, nlat):
     assert rel_err(folded, dense) < TOL
 
 
+ORBITAL_SETS = {
+    "two": ([(1, 0, 0, 1), (2, 0, 0, 1)], 1, 1, 0, 1),
+    "three_m": ([(2, 1, -1, 1), (2, 1, 0, 1), (2, 1, 1, 1)], 2, 1, 1, 2),
+    "d_shell": ([(1, 0, 0, -1), (2, 0, 0, 1)] + [(3, 2, m, 1) for m in (-2, -1, 0, 1, 2)], 3, 3, 0, 1),
+    "two_dynamic_cores": ([(1, 0, 0, 0), (2, 0, 0, 0), (2, 1, 0, 1), (3, 1, 0, 1), (3, 0, 0, 1), (3, 2, 0, 1), (4, 0, 0, 1)], 4, 4, 0, 1),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", sorted(ORBITAL_SETS))
+@pytest.mark.parametrize("nfe,ndvr", [(1, 10), (2, 7), (5, 12), (9, 8)])
+def test_pair_products_and_elements(cuda_ok, name, nfe, ndvr):
+    """Orbital sets with |Delta m| up to 4 and partial tiles, on one element (no bridge), two, and element
+    sizes with and without unrolled rows."""
+    orbitals, na, nb, mtot, smul = ORBITAL_SETS[name]
+    _rhs_parity(dict(W.MIXED_SMALL, name=name, orbitals=orbitals, nela=na, nelb=nb, mtot=mtot, smul=smul, znuc=float(na + nb),
+                     nfe=nfe, ndvr=ndvr, rmax=2.0 * nfe, rmask=1.6 * nfe, igauge=1))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("igauge", [0, 1])
 @pytest.mark.parametrize("nfe,ndvr,dtime", [(1, 10, 0.01), (2, 7, 0.01), (9, 7, 0.005), (9, 8, 3.0), (14, 6, 0.2), (14, 6, 2.0), (6, 20, 0.004)])
