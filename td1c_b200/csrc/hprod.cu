@@ -150,9 +150,8 @@ struct Ctx {
   std::vector<int4> h_ent;
   int* ent_index = nullptr;  // [5][nfun][nfun] -> entry id or -1 (A, B, C, E, GV)
   Int2eArgs i2{};
-  int i2_nsplit = 128;
+  int i2_nsplit = 1, i2t_nsplit = 1;  // K slices of the FP64 and of the split-TF32 kernel
   I2dArgs i2d{};          // int2e on the FP64 tensor cores
-  bool i2_dmma = false;   // the DMMA plan fits in shared memory
   I2tArgs i2t{};          // int2e in split TF32 on tcgen05 (mixed-precision form)
   bool i2_tc = false;     // its plan fits (at most 64 stored active pairs)
   // act2 blocks
@@ -1006,6 +1005,44 @@ int build_batches(Ctx& c) {
   return 0;
 }
 
+int sm_count() {
+  int dev = 0, nsm = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return nsm;
+}
+// the items of one block of mt x nt tiles: rectangles of up to 2 x 4
+void dot_product_items(std::vector<DotProdItem>& items, int compa, int compb, int mt, int nt, int tile0) {
+  const int gm = (mt + 1) / 2, gn = (nt + 3) / 4;
+  for (int x = 0; x < gm; ++x)
+    for (int y = 0; y < gn; ++y) {
+      const int m0 = mt * x / gm, m1 = mt * (x + 1) / gm, n0 = nt * y / gn, n1 = nt * (y + 1) / gn;
+      items.push_back(DotProdItem{compa, compb, m0, m1 - m0, n0, n1 - n0, tile0, nt});
+    }
+}
+// the items spread over the warps, largest first to the warp with the least work (I2D_MAXG each, then
+// further sets of warps), the row list and the buffers; returns the number of K slices
+int dot_product_plan(DotProdArgs& a, const std::vector<const cplx*>& row, const std::vector<int>& comp,
+                     std::vector<DotProdItem> items, int ntile, size_t K) {
+  std::stable_sort(items.begin(), items.end(), [](const DotProdItem& x, const DotProdItem& y) { return x.nm * x.nn > y.nm * y.nn; });
+  const int slots = I2D_NW * I2D_MAXG, nsets = std::max(1, ((int)items.size() + slots - 1) / slots);
+  std::vector<DotProdItem> wi((size_t)nsets * slots, DotProdItem{0, 0, 0, 0, 0, 0, 0, 0});
+  std::vector<int> load((size_t)nsets * I2D_NW, 0), used((size_t)nsets * I2D_NW, 0);
+  for (const DotProdItem& it : items) {
+    int best = -1;
+    for (int w = 0; w < nsets * I2D_NW; ++w)
+      if (used[w] < I2D_MAXG && (best < 0 || load[w] < load[best])) best = w;
+    wi[(size_t)best * I2D_MAXG + used[best]++] = it;
+    load[best] += it.nm * it.nn;
+  }
+  a.nrow = (int)row.size(); a.nent = 64 * ntile; a.nsets = nsets; a.K = K;
+  a.row = dupload(row); a.comp = dupload(comp); a.items = dupload(wi);
+  const int ns = dot_products_nsplit(a, sm_count());
+  a.partial = dalloc<double>((size_t)ns * std::max(1, a.nent));
+  a.sum = dalloc<double>(std::max(1, a.nent));
+  return ns;
+}
+
 int build_reductions(Ctx& c) {
   // orbdots entries: kind 0 (A) and 1 (B) for dynamic j, i of equal m (and the
   // frozen j for kind 2 (C) and 4 (<phi_j|(g+v2) phi_i>)); kind 3 (E) for dynamic cores
@@ -1030,166 +1067,91 @@ int build_reductions(Ctx& c) {
   c.od.result = dalloc<cplx>(std::max(1, c.od.nent));
   // int2e blocks by delta = m_i - m_j
   const int n = c.nact, nc = c.ncore;
-  std::vector<Int2eBlock> blocks;
-  std::vector<int> rows;
-  std::vector<int2> cols;
-  std::vector<int4> dst;
-  if (n > 0) {
-    int dmax = 0;
-    for (int a = 0; a < n; ++a) for (int b = 0; b < n; ++b) dmax = std::max(dmax, std::abs(c.mval[nc + a] - c.mval[nc + b]));
-    for (int d = -dmax; d <= dmax; ++d) {
-      std::vector<int> r_ij; std::vector<std::pair<int, int>> rr;
-      for (int ia = 0; ia < n; ++ia)
-        for (int ja = 0; ja <= ia; ++ja)
-          if (c.mval[nc + ia] - c.mval[nc + ja] == d) rr.push_back({ia, ja});
-      std::vector<std::pair<int, int>> cc;
-      for (int ka = 0; ka < n; ++ka)
-        for (int la = 0; la < n; ++la)
-          if (c.mval[nc + la] - c.mval[nc + ka] == d) cc.push_back({ka, la});
-      if (rr.empty() || cc.empty()) continue;
-      // split into chunks: rows <= 24, cols <= 36 (the int2e kernel's CTA tile)
-      const int cchunk = std::min((int)cc.size(), 36);
-      const int rchunk = 24;
-      for (size_t r0 = 0; r0 < rr.size(); r0 += rchunk)
-        for (size_t c0 = 0; c0 < cc.size(); c0 += cchunk) {
-          int nr = (int)std::min((size_t)rchunk, rr.size() - r0), ncl = (int)std::min((size_t)cchunk, cc.size() - c0);
-          Int2eBlock bk{};
-          bk.row0 = (int)rows.size(); bk.nrow = nr; bk.col0 = (int)cols.size(); bk.ncol = ncl; bk.ent0 = (int)dst.size();
-          for (int x = 0; x < nr; ++x) {
-            int ia = rr[r0 + x].first, ja = rr[r0 + x].second;
-            rows.push_back(c.pair_of ? 0 : 0);
-            // stored pair of (i, j): a = i >= b = j
-            int p = -1;
-            for (int q = 0; q < c.npair; ++q) if (c.pa[q] == nc + ia && c.pb[q] == nc + ja) p = q;
-            rows.back() = p;
-          }
-          for (int y = 0; y < ncl; ++y) {
-            int ka = cc[c0 + y].first, la = cc[c0 + y].second;
-            int kf = nc + ka, lf = nc + la, p = -1, cj = 0;
-            for (int q = 0; q < c.npair; ++q) {
-              if (c.pa[q] == kf && c.pb[q] == lf) { p = q; cj = 0; }
-              if (c.pa[q] == lf && c.pb[q] == kf) { p = q; cj = 1; }
-            }
-            cols.push_back(make_int2(p, cj));
-          }
-          for (int x = 0; x < nr; ++x)
-            for (int y = 0; y < ncl; ++y)
-              dst.push_back(make_int4(rr[r0 + x].first, rr[r0 + x].second, cc[c0 + y].first, cc[c0 + y].second));
-          blocks.push_back(bk);
-        }
-    }
-  }
-  c.i2.nact = n; c.i2.nblocks = (int)blocks.size(); c.i2.nblkent = (int)dst.size(); c.i2.K = c.nbas2;
-  c.i2.blocks = dupload(blocks); c.i2.row_pair = dupload(rows); c.i2.col_pair = dupload(cols); c.i2.ent_dst = dupload(dst);
-  c.i2.rho2 = c.rho2; c.i2.v2sph = c.v2sph;
   c.int2e = dalloc<cplx>((size_t)std::max(1, n * n * n * n));
-  c.i2.int2e = c.int2e;
-  // the same entries as DMMA tiles: per Delta the rows ij (i >= j) padded to
-  // m-tiles of 8 pairs, the columns kl padded to n-tiles of 8, the entry of
-  // (row r, column y) at ent0 + r ncol + y in the (i outer, j inner) x
-  // (k outer, l inner) order of the block list above; groups (m-tile x up
-  // to I2D_NTMAX n-tiles) are spread over the warps so that the four
-  // schedulers of an SM get similar numbers of n-tiles
   {
-    std::vector<int> a_pair, a_ent, b_col;
-    std::vector<int2> b_pair;
-    std::vector<I2dGroup> groups;
-    std::vector<int4> dst2;
-    int dmax = 0;
-    for (int x = 0; x < n; ++x) for (int y = 0; y < n; ++y) dmax = std::max(dmax, std::abs(c.mval[nc + x] - c.mval[nc + y]));
-    for (int d = -dmax; d <= dmax && n > 0; ++d) {
-      std::vector<std::pair<int, int>> rr, cc;
-      for (int ia = 0; ia < n; ++ia)
-        for (int ja = 0; ja <= ia; ++ja)
-          if (c.mval[nc + ia] - c.mval[nc + ja] == d) rr.push_back({ia, ja});
-      for (int ka = 0; ka < n; ++ka)
-        for (int la = 0; la < n; ++la)
-          if (c.mval[nc + la] - c.mval[nc + ka] == d) cc.push_back({ka, la});
-      if (rr.empty() || cc.empty()) continue;
-      const int ent0 = (int)dst2.size(), ncl = (int)cc.size();
-      const int arow0 = (int)a_pair.size(), brow0 = (int)b_pair.size();
-      for (size_t r = 0; r < rr.size(); ++r) {
-        int p = -1;
-        for (int q = 0; q < c.npair; ++q) if (c.pa[q] == nc + rr[r].first && c.pb[q] == nc + rr[r].second) p = q;
-        a_pair.push_back(p); a_ent.push_back(ent0 + (int)r * ncl);
-        for (int y = 0; y < ncl; ++y) dst2.push_back(make_int4(rr[r].first, rr[r].second, cc[y].first, cc[y].second));
-      }
-      while ((a_pair.size() - arow0) % 8) { a_pair.push_back(-1); a_ent.push_back(-1); }
-      for (int y = 0; y < ncl; ++y) {
-        const int kf = nc + cc[y].first, lf = nc + cc[y].second;
-        int p = -1, cj = 0;
-        for (int q = 0; q < c.npair; ++q) {
-          if (c.pa[q] == kf && c.pb[q] == lf) { p = q; cj = 0; }
-          if (c.pa[q] == lf && c.pb[q] == kf) { p = q; cj = 1; }
+    std::vector<int> cpair, comp, cof(c.npair * 2, -1);  // cof: component of (pair, part) in its block
+    std::vector<DotProdItem> items;
+    int dmax = 0, ntile_all = 0, P = 0;
+    for (int a = 0; a < n; ++a) for (int b = 0; b < n; ++b) dmax = std::max(dmax, std::abs(c.mval[nc + a] - c.mval[nc + b]));
+    std::vector<int> blk_tile0(dmax + 1, 0), blk_nt(dmax + 1, 0);
+    auto dabs = [&](int q) { return std::abs(c.mval[c.pb[q]] - c.mval[c.pa[q]]); };
+    for (int q = 0; q < c.npair; ++q) P += c.pa[q] >= nc && c.pb[q] >= nc;
+    for (int d = 0; d <= dmax && n > 0; ++d) {
+      const int comp0 = (int)comp.size();
+      for (int q = 0; q < c.npair; ++q) {
+        if (c.pa[q] < nc || c.pb[q] < nc || dabs(q) != d) continue;
+        for (int part = 0; part < (c.pa[q] == c.pb[q] ? 1 : 2); ++part) {
+          cof[2 * q + part] = (int)comp.size() - comp0;
+          comp.push_back((int)cpair.size() | part << 16);
         }
-        b_pair.push_back(make_int2(p, cj)); b_col.push_back(y);
+        cpair.push_back(q);
       }
-      while ((b_pair.size() - brow0) % 8) { b_pair.push_back(make_int2(-1, 0)); b_col.push_back(-1); }
-      const int mtiles = ((int)a_pair.size() - arow0) / 8, ntiles = ((int)b_pair.size() - brow0) / 8;
-      for (int mt = 0; mt < mtiles; ++mt)
-        for (int nt = 0; nt < ntiles; nt += I2D_NTMAX)
-          groups.push_back(I2dGroup{arow0 + 8 * mt, brow0 + 8 * nt, std::min(I2D_NTMAX, ntiles - nt), 0});
+      if ((int)comp.size() == comp0) continue;
+      while ((comp.size() - comp0) % 8) comp.push_back(comp[comp0]);
+      const int nt = ((int)comp.size() - comp0) / 8, compb = (int)comp.size();
+      for (int k = 0; k < 8 * nt; ++k) comp.push_back(comp[comp0 + k] + P);  // the same components of v2sph
+      blk_tile0[d] = ntile_all; blk_nt[d] = nt;
+      dot_product_items(items, comp0, compb, nt, nt, ntile_all);
+      ntile_all += nt * nt;
     }
-    if (dst2.size() != dst.size()) return ST_CONFIG;
-    // warp slots: sets of I2D_NW warps x I2D_MAXG groups; within a set the
-    // largest groups go first to the scheduler (warp % 4) with the least work
-    std::vector<int> order(groups.size());
-    for (size_t g = 0; g < order.size(); ++g) order[g] = (int)g;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return groups[x].nnt > groups[y].nnt; });
-    const int slots = I2D_NW * I2D_MAXG;
-    const int nsets = std::max(1, ((int)groups.size() + slots - 1) / slots);
-    std::vector<int> wgrp((size_t)nsets * slots, -1);
-    for (int set = 0; set < nsets; ++set) {
-      int load[4] = {0, 0, 0, 0}, used[I2D_NW] = {0};
-      for (int k = set * slots; k < std::min((int)order.size(), (set + 1) * slots); ++k) {
-        const int g = order[k];
-        int best = -1;
-        for (int w = 0; w < I2D_NW; ++w)
-          if (used[w] < I2D_MAXG && (best < 0 || load[w % 4] < load[best % 4])) best = w;
-        wgrp[((size_t)set * I2D_NW + best) * I2D_MAXG + used[best]++] = g;
-        load[best % 4] += groups[g].nnt;
-      }
-    }
+    // the products of int2e(i, j, k, l): i < j from the conjugate of (j, i, l, k)
+    std::vector<int4> form((size_t)std::max(1, n * n * n * n), make_int4(-1, -1, -1, -1));
+    std::vector<unsigned char> flag(form.size(), 0);
+    std::vector<int> stored(c.nfun * c.nfun, -1);
+    for (int q = 0; q < c.npair; ++q) stored[c.pa[q] * c.nfun + c.pb[q]] = q;
+    for (int i = 0; i < n; ++i)
+      for (int j = 0; j < n; ++j)
+        for (int k = 0; k < n; ++k)
+          for (int l = 0; l < n; ++l) {
+            if (c.mval[nc + i] + c.mval[nc + k] != c.mval[nc + j] + c.mval[nc + l]) continue;
+            const bool sw = i < j;
+            const int p = stored[(nc + std::max(i, j)) * c.nfun + nc + std::min(i, j)];
+            const int k2 = sw ? l : k, l2 = sw ? k : l;
+            const bool cj = k2 < l2;
+            const int q = stored[(nc + std::max(k, l)) * c.nfun + nc + std::min(k, l)];
+            const int d = dabs(p), nt = blk_nt[d];
+            auto ent = [&](int x, int y) {
+              const int cx = cof[2 * p + x], cy = cof[2 * q + y];
+              return cx < 0 || cy < 0 ? -1 : (blk_tile0[d] + cx / 8 * nt + cy / 8) * 64 + cx % 8 * 8 + cy % 8;
+            };
+            const size_t t = i + n * (j + n * (k + (size_t)n * l));
+            form[t] = make_int4(ent(0, 0), ent(0, 1), ent(1, 0), ent(1, 1));
+            flag[t] = (cj ? 1 : 0) | (sw ? 2 : 0);
+          }
     I2dArgs& d2 = c.i2d;
-    d2.nra = (int)a_pair.size(); d2.nrb = (int)b_pair.size(); d2.ngroups = (int)groups.size(); d2.nblkent = (int)dst2.size();
-    d2.K = c.nbas2; d2.rho2 = c.rho2; d2.v2sph = c.v2sph; d2.nsets = nsets;
-    d2.a_pair = dupload(a_pair); d2.a_ent = dupload(a_ent); d2.b_pair = dupload(b_pair); d2.b_col = dupload(b_col);
-    d2.groups = dupload(groups); d2.warp_group = dupload(wgrp);
-    c.i2_dmma = n > 0 && int2e_dmma_fits(d2);
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (c.i2_dmma) {
-      // the DMMA plan's entries replace the block list's (same count, its own order)
-      c.i2_nsplit = nsm;
-      c.i2.ent_dst = dupload(dst2);
-    }
-    c.i2.partial = dalloc<cplx>((size_t)c.i2_nsplit * std::max(1, c.i2.nblkent));
-    d2.partial = reinterpret_cast<double*>(c.i2.partial);
-    // the split-TF32 plan: the stored active pairs in compact order and, per entry of the
-    // DMMA plan, its row pair, column pair and conjugation (the DMMA plan's choice)
-    if (c.i2_dmma) {
-      std::vector<int> cpair, compact(c.npair, -1);
-      for (int q = 0; q < c.npair; ++q)
-        if (c.pa[q] >= nc && c.pb[q] >= nc) { compact[q] = (int)cpair.size(); cpair.push_back(q); }
-      std::vector<int4> ent(dst2.size());
-      bool okp = !cpair.empty() && cpair.size() <= 64;
-      for (size_t e = 0; e < dst2.size() && okp; ++e) {
-        const int4 d4 = dst2[e];
-        int pr = -1, pc = -1, cj = 0;
-        for (int q = 0; q < c.npair; ++q) {
-          if (c.pa[q] == nc + d4.x && c.pb[q] == nc + d4.y) pr = q;
-          if (c.pa[q] == nc + d4.z && c.pb[q] == nc + d4.w) { pc = q; cj = 0; }
-          if (c.pa[q] == nc + d4.w && c.pb[q] == nc + d4.z) { pc = q; cj = 1; }
-        }
-        if (pr < 0 || pc < 0 || compact[pr] < 0 || compact[pc] < 0) { okp = false; break; }
-        ent[e] = make_int4(compact[pr], compact[pc], cj, 0);
-      }
+    std::vector<const cplx*> row;
+    for (int q : cpair) row.push_back(c.rho2 + (size_t)q * c.nbas2);
+    for (int q : cpair) row.push_back(c.v2sph + (size_t)q * c.nbas2);
+    d2.nact = n; d2.int2e = c.int2e; d2.form = dupload(form); d2.flag = dupload(flag);
+    c.i2_nsplit = dot_product_plan(d2.prod, row, comp, items, ntile_all, c.nbas2);
+    // the split-TF32 plan: the stored active pairs in compact order and, per entry (i >= j, all k, l of the m
+    // rule), its row pair, column pair and conjugation
+    c.i2_tc = false;
+    if (n > 0 && cpair.size() <= 64) {
+      std::vector<int> compact(c.npair, -1);
+      for (size_t k = 0; k < cpair.size(); ++k) compact[cpair[k]] = (int)k;
+      std::vector<int4> dst, ent;
+      for (int i = 0; i < n; ++i)
+        for (int j = 0; j <= i; ++j)
+          for (int k = 0; k < n; ++k)
+            for (int l = 0; l < n; ++l) {
+              if (c.mval[nc + i] + c.mval[nc + k] != c.mval[nc + j] + c.mval[nc + l]) continue;
+              const int p = stored[(nc + i) * c.nfun + nc + j], q = stored[(nc + std::max(k, l)) * c.nfun + nc + std::min(k, l)];
+              dst.push_back(make_int4(i, j, k, l));
+              ent.push_back(make_int4(compact[p], compact[q], k < l ? 1 : 0, 0));
+            }
       I2tArgs& t = c.i2t;
       t.P = (int)cpair.size(); t.NB = (t.P + 15) / 16 * 16; t.K = c.nbas2; t.nent = (int)ent.size();
-      t.rho2 = c.rho2; t.v2sph = c.v2sph; t.partial = c.i2.partial; t.status = c.d_status;
-      c.i2_tc = okp && int2e_tc_fits(t);
-      if (c.i2_tc) { t.pair = dupload(cpair); t.ent = dupload(ent); }
+      t.rho2 = c.rho2; t.v2sph = c.v2sph; t.status = c.d_status;
+      c.i2_tc = int2e_tc_fits(t);
+      if (c.i2_tc) {
+        c.i2t_nsplit = sm_count();
+        c.i2.nact = n; c.i2.nblkent = t.nent; c.i2.int2e = c.int2e;
+        c.i2.ent_dst = dupload(dst);
+        c.i2.partial = dalloc<cplx>((size_t)c.i2t_nsplit * t.nent);
+        t.partial = c.i2.partial;
+        t.pair = dupload(cpair); t.ent = dupload(ent);
+      }
     }
   }
   // act2 dense blocks: rows ij (i >= j, m_i - m_j = d) in the reference's
@@ -1447,9 +1409,9 @@ int gemm(Ctx& c, const LegGemmBatch* b, int nb, int M, int K, bool to_l, bool pa
   return launch_legendre_gemm_mt(b, nb, M, K, 2 * c.Nr, pair, c.tune_mt, c.st);
 }
 // the int2e K split: the tuned value where one is set (at most the allocated split)
-int i2_split(const Ctx& c) {
+int i2_split(const Ctx& c, int most) {
   const int k = c.tune_i2_split < 0 ? -c.tune_i2_split : c.tune_i2_split;
-  return k > 1 || (k == 1 && c.tune_i2_split > 0) ? std::min(k, c.i2_nsplit) : c.i2_nsplit;
+  return k > 1 || (k == 1 && c.tune_i2_split > 0) ? std::min(k, most) : most;
 }
 // the condensed Poisson solve's arguments: in mixed mode 3 the element pass's interior products
 // run in split TF32
@@ -1458,11 +1420,10 @@ PsCondArgs ps_args(const Ctx& c) {
   a.tf32 = c.mixed == 3 ? 1 : 0;
   return a;
 }
-// int2e: split TF32 on tcgen05 in mixed mode 3, else FP64 DMMA (or the FFMA blocks)
+// int2e: split TF32 on tcgen05 in mixed mode 3, else FP64 DMMA
 int int2e_run(Ctx& c, cudaStream_t s) {
-  if (c.mixed == 3 && c.i2_tc) return launch_int2e_tc(c.i2t, c.i2, i2_split(c), s);
-  if (c.i2_dmma) return launch_int2e_dmma(c.i2d, c.i2, i2_split(c), s);
-  return launch_int2e(c.i2, i2_split(c), s);
+  if (c.mixed == 3 && c.i2_tc) return launch_int2e_tc(c.i2t, c.i2, i2_split(c, c.i2t_nsplit), s);
+  return launch_int2e_dmma(c.i2d, i2_split(c, c.i2_nsplit), s);
 }
 int mfprod_run(Ctx& c, cudaStream_t st) {
   MfprodArgs m = c.mf;
@@ -3484,7 +3445,7 @@ int td1c_gpu_mixed_int2e_selftest(const void* d_wfn, const void* d_cic, const do
       rc |= run_htot(c, c.dip_lfd, (const cplx*)d_wfn, (const cplx*)d_cic, c.hwfn_io, c.hcic_io, 1.0);
     } else {
       // the FP64 DMMA kernel on the mixed RHS's own pair densities and potentials
-      rc |= launch_int2e_dmma(c.i2d, c.i2, i2_split(c), st);
+      rc |= launch_int2e_dmma(c.i2d, i2_split(c, c.i2_nsplit), st);
     }
     i2[k].resize(n4);
     cudaMemcpyAsync(i2[k].data(), c.int2e, n4 * sizeof(cplx), cudaMemcpyDeviceToHost, st);

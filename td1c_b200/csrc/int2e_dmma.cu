@@ -2,32 +2,39 @@
 // on the FP64 tensor cores.
 //
 // int2e(i,j,k,l) = sum_x rho2_ij[x] v2sph_kl[x] over x in [0, K), K =
-// Nr (lmax2 + 1), for i >= j and m_i + m_k = m_j + m_l.  For every Delta =
-// m_i - m_j the rows ij and the columns kl form a dense complex product
-// C = A B^T, computed with four real products per complex depth step:
-//   Re C += Re A Re B + Im A (-Im B),   Im C += Re A Im B + Im A Re B
-// on mma.sync.m8n8k4.f64 tiles of 8 rows x 8 columns x 4 complex depths,
-// each of the four products in its own accumulator (independent chains).
-// Lane (g, t) of a fragment handles depth x = 4 s + t, so one 128-bit
-// shared-memory load gives it both parts of its A (row g) or B (column g)
-// element; a conjugated column flips the sign of Im B in the same lane.
+// Nr (lmax2 + 1), for m_i + m_k = m_j + m_l.  Pairs (a, b) and (b, a) are a
+// stored field and its conjugate, so every integral is a sign combination of
+// the four real products of two stored pairs p, q,
+//   RR = sum Re rho_p Re v_q, II, RI = sum Re rho_p Im v_q, IR:
+//   v_q plain (RR - II, RI + IR), v_q conjugated (RR + II, IR - RI),
+// and the pairs of one |Delta m| need only each other: per |Delta m| one real
+// product S = A B^T of the pairs' components (re, im; the diagonal pairs are
+// real), on mma.sync.m8n8k4.f64 tiles of 8 x 8 components x 4 points.  For
+// CAS(8e,9o) that is 51 tiles where the complex form over ordered pairs
+// needed 116 tile products, and each stored row is staged once instead of once
+// per order.
 //
-// One CTA owns a slice of K and every block: the slice of each A row (rho2
-// of the block rows) and each B row (v2sph of the block columns) is staged
-// in shared memory by cp.async in a 4-stage ring (each thread's copy
-// addresses computed once); the 16 warps run the groups (m-tile x up to 3
-// n-tiles) the host assigned to them.  Each CTA writes its partial sums;
-// int2e_sum_kernel adds them in a fixed order.
+// One CTA owns a slice of K: the slice of every stored pair's rho2 and v2sph
+// rows passes through shared memory in a cp.async ring of NS stages of I2D_KC
+// points; each of the 8 warps keeps the accumulators of up to I2D_MAXG items
+// (up to 2 x 4 tiles, which share their fragments).  Each CTA writes its
+// partial sums; dot_sum_kernel adds them in a fixed order and
+// int2e_form_kernel forms the integrals.
+//
+// What bounds it: staging (60 rows of 16 points a stage, 8 warps waiting for
+// it together) and the tensor pipe in turn.  Ne, CAS(8e,9o), K = 127260:
+// 93 + 8 us (complex tiles) -> 42 + 3; 66 before the item shapes were unrolled
+// one by one (dp_item).
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "reductions.cuh"
 
 namespace td1c {
 
-constexpr int I2D_KC = 16;                 // complex depth per stage
-constexpr int I2D_PITCH = 2 * I2D_KC + 8;  // doubles per staged row: rows 2g, 2g+1 fall in opposite bank halves
-constexpr int I2D_NS = 4;                  // stages
-constexpr int I2D_LMAX = 8;                // staged 16-byte copies per thread and stage (nrows KC <= 8 NW 32)
+constexpr int I2D_KC = 16;                 // points per stage
+constexpr int I2D_PITCH = 2 * I2D_KC + 8;  // doubles per staged row: 8 mod 16, so 2 rows x 2 parts x 4 points fall in distinct banks
 
 __device__ __forceinline__ void dmma_8x8x4(double& c0, double& c1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
@@ -41,16 +48,32 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-size_t int2e_dmma_smem(const I2dArgs& a) {
-  return sizeof(double) * (size_t)I2D_NS * (a.nra + a.nrb) * I2D_PITCH;
-}
-bool int2e_dmma_fits(const I2dArgs& a) {
-  return int2e_dmma_smem(a) <= 227 * 1024 && (size_t)(a.nra + a.nrb) * I2D_KC <= (size_t)I2D_LMAX * I2D_NW * 32;
+static size_t dp_smem(int nrow, int ns) { return sizeof(double) * (size_t)ns * nrow * I2D_PITCH; }
+// three stages where they fit in shared memory, else two
+static int dp_stages(int nrow) { return dp_smem(nrow, 3) <= 224 * 1024 ? 3 : 2; }
+
+// one stage of an item of NM x NN tiles
+template <int NM, int NN>
+__device__ __forceinline__ void dp_item(const double* sm, const int (&aoff)[2], const int (&boff)[4], double (&acc)[2][4][2]) {
+#pragma unroll
+  for (int s = 0; s < I2D_KC / 4; ++s) {
+    double av[NM], bv[NN];
+#pragma unroll
+    for (int i = 0; i < NM; ++i) av[i] = sm[aoff[i] + 8 * s];
+#pragma unroll
+    for (int j = 0; j < NN; ++j) bv[j] = sm[boff[j] + 8 * s];
+#pragma unroll
+    for (int i = 0; i < NM; ++i)
+#pragma unroll
+      for (int j = 0; j < NN; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], av[i], bv[j]);
+  }
 }
 
-__global__ void __launch_bounds__(I2D_NW * 32, 1) int2e_dmma_kernel(I2dArgs a) {
-  extern __shared__ __align__(16) double i2d_smem[];
-  const int nrows = a.nra + a.nrb;
+// S = A B^T over a slice of K: A and B components (row | part << 16) of the row list, in the items' tiles
+template <int NS>
+__global__ void __launch_bounds__(I2D_NW * 32, 2) dot_products_kernel(DotProdArgs a) {
+  extern __shared__ __align__(16) double i2d_sm[];
+  const int nrows = a.nrow;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3;
   const size_t K = a.K;
@@ -58,146 +81,150 @@ __global__ void __launch_bounds__(I2D_NW * 32, 1) int2e_dmma_kernel(I2dArgs a) {
   const size_t k0 = (size_t)blockIdx.x * kper, k1 = min(K, k0 + kper);
   const int nchunk = k1 > k0 ? (int)((k1 - k0 + I2D_KC - 1) / I2D_KC) : 0;
   const unsigned stage_bytes = (unsigned)(sizeof(double) * nrows * I2D_PITCH);
-  const unsigned smem0 = (unsigned)__cvta_generic_to_shared(i2d_smem);
+  const unsigned smem0 = (unsigned)__cvta_generic_to_shared(i2d_sm);
 
-  // padding rows hold zeros in every stage and are never loaded
-  for (int row = warp; row < nrows; row += I2D_NW) {
-    const int pr = row < a.nra ? a.a_pair[row] : a.b_pair[row - a.nra].x;
-    if (pr < 0)
-      for (int e = lane; e < I2D_NS * I2D_PITCH; e += 32)
-        i2d_smem[(size_t)(e / I2D_PITCH) * nrows * I2D_PITCH + (size_t)row * I2D_PITCH + e % I2D_PITCH] = 0.0;
-  }
-  // this thread's copies: element e = tid + i blockDim (row e / KC, depth e % KC)
-  const cplx* src[I2D_LMAX];
-  unsigned dst[I2D_LMAX];
-  int kofs[I2D_LMAX];
-#pragma unroll
-  for (int i = 0; i < I2D_LMAX; ++i) {
-    const int e = tid + i * blockDim.x;
-    src[i] = nullptr; dst[i] = 0; kofs[i] = 0;
-    if (e < nrows * I2D_KC) {
-      const int row = e / I2D_KC, kk = e % I2D_KC;
-      const int pr = row < a.nra ? a.a_pair[row] : a.b_pair[row - a.nra].x;
-      if (pr >= 0) {
-        src[i] = (row < a.nra ? a.rho2 : a.v2sph) + (size_t)pr * K + k0 + kk;
-        dst[i] = smem0 + (unsigned)(sizeof(double) * ((size_t)row * I2D_PITCH + 2 * kk));
-        kofs[i] = kk;
-      }
-    }
-  }
+  // this thread copies point kk of the rows row0, row0 + NW 32 / KC, ...
+  const int kk = tid % I2D_KC, row0 = tid / I2D_KC;
   auto load = [&](int chunk) {
     if (chunk >= nchunk) return;
-    const size_t kb = (size_t)chunk * I2D_KC;
-    const unsigned so = (unsigned)(chunk % I2D_NS) * stage_bytes;
-    const bool tail = k0 + kb + I2D_KC > k1;
-#pragma unroll
-    for (int i = 0; i < I2D_LMAX; ++i) {
-      if (!src[i]) continue;
-      if (!tail) {
-        cp_async_16(dst[i] + so, src[i] + kb, 16u);
-      } else {  // past k1: zero fill, reading nothing, from the slice's first (valid) element
-        const bool in = k0 + kb + kofs[i] < k1;
-        cp_async_16(dst[i] + so, in ? src[i] + kb : src[i] - kofs[i], in ? 16u : 0u);
-      }
-    }
+    const size_t k = k0 + (size_t)chunk * I2D_KC + kk;
+    const bool in = k < k1;
+    const unsigned dst = smem0 + (unsigned)(chunk % NS) * stage_bytes + (unsigned)(2 * sizeof(double) * kk);
+    for (int row = row0; row < nrows; row += I2D_NW * 32 / I2D_KC)
+      cp_async_16(dst + (unsigned)(sizeof(double) * I2D_PITCH * row), a.row[row] + (in ? k : 0), in ? 16u : 0u);
   };
 
-  // this warp's groups with the lane's fragment offsets (in double2 units)
-  int nnt[I2D_MAXG], aoff[I2D_MAXG], boff[I2D_MAXG][I2D_NTMAX];
-  unsigned bcj[I2D_MAXG];  // bit t: n-tile t of the lane's column is conjugated
-  // [g][t][chain][c0|c1]: Re A Re B, Im A (-Im B), Re A Im B, Im A Re B as
-  // four independent accumulator chains, added at the end
-  double acc[I2D_MAXG][I2D_NTMAX][4][2];
-  const int* wg = a.warp_group + ((size_t)blockIdx.y * I2D_NW + warp) * I2D_MAXG;
+  // this warp's items and the lane's fragment offsets (doubles); tiles past the item repeat its first
+  int nm[I2D_MAXG], nn[I2D_MAXG], shape[I2D_MAXG], aoff[I2D_MAXG][2], boff[I2D_MAXG][4];
+  double acc[I2D_MAXG][2][4][2];
+  const DotProdItem* wi = a.items + ((size_t)blockIdx.y * I2D_NW + warp) * I2D_MAXG;
 #pragma unroll
   for (int g = 0; g < I2D_MAXG; ++g) {
-    const int gi = wg[g];
-    const I2dGroup G = gi >= 0 ? a.groups[gi] : I2dGroup{0, 0, 0, 0};
-    nnt[g] = G.nnt;
-    aoff[g] = (G.arow0 + gid) * (I2D_PITCH / 2) + tig;
-    bcj[g] = 0;
+    const DotProdItem G = wi[g];
+    nm[g] = G.nm;
+    nn[g] = G.nn;
+    shape[g] = G.nm ? 4 * G.nm + G.nn - 1 : 0;
 #pragma unroll
-    for (int t = 0; t < I2D_NTMAX; ++t) {
-      const int brow = G.brow0 + 8 * t + gid;
-      boff[g][t] = (a.nra + brow) * (I2D_PITCH / 2) + tig;
-      if (t < G.nnt && a.b_pair[brow].y) bcj[g] |= 1u << t;
-#pragma unroll
-      for (int h = 0; h < 4; ++h) acc[g][t][h][0] = acc[g][t][h][1] = 0.0;
+    for (int i = 0; i < 2; ++i) {
+      const int q = a.comp[G.compa + 8 * (G.mt + (i < G.nm ? i : 0)) + gid];
+      aoff[g][i] = (q & 0xffff) * I2D_PITCH + (q >> 16) + 2 * tig;
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int q = a.comp[G.compb + 8 * (G.nt + (j < G.nn ? j : 0)) + gid];
+      boff[g][j] = (q & 0xffff) * I2D_PITCH + (q >> 16) + 2 * tig;
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[g][i][j][0] = acc[g][i][j][1] = 0.0;
   }
 
 #pragma unroll
-  for (int s = 0; s < I2D_NS - 1; ++s) { load(s); cp_async_commit(); }
+  for (int s = 0; s < NS - 1; ++s) { load(s); cp_async_commit(); }
   for (int chunk = 0; chunk < nchunk; ++chunk) {
-    cp_async_wait<I2D_NS - 2>();
+    cp_async_wait<NS - 2>();
     __syncthreads();  // stage chunk % NS complete for every thread; stage (chunk - 1) % NS free
-    load(chunk + I2D_NS - 1);
+    load(chunk + NS - 1);
     cp_async_commit();
-    const double2* sm = reinterpret_cast<const double2*>(i2d_smem + (size_t)(chunk % I2D_NS) * nrows * I2D_PITCH);
+    const double* sm = i2d_sm + (size_t)(chunk % NS) * nrows * I2D_PITCH;
 #pragma unroll
     for (int g = 0; g < I2D_MAXG; ++g) {
-      if (nnt[g] == 0) continue;
-#pragma unroll
-      for (int s = 0; s < I2D_KC / 4; ++s) {
-        const double2 av = sm[aoff[g] + 4 * s];
-#pragma unroll
-        for (int t = 0; t < I2D_NTMAX; ++t) {
-          if (t < nnt[g]) {
-            const double2 bv = sm[boff[g][t] + 4 * s];
-            const double bi = ((bcj[g] >> t) & 1) ? -bv.y : bv.y;
-            dmma_8x8x4(acc[g][t][0][0], acc[g][t][0][1], av.x, bv.x);
-            dmma_8x8x4(acc[g][t][1][0], acc[g][t][1][1], av.y, -bi);
-            dmma_8x8x4(acc[g][t][2][0], acc[g][t][2][1], av.x, bi);
-            dmma_8x8x4(acc[g][t][3][0], acc[g][t][3][1], av.y, bv.x);
-          }
-        }
+      switch (shape[g]) {  // one branch per item and stage
+        case 4 * 1 + 0: dp_item<1, 1>(sm, aoff[g], boff[g], acc[g]); break;
+        case 4 * 1 + 1: dp_item<1, 2>(sm, aoff[g], boff[g], acc[g]); break;
+        case 4 * 1 + 2: dp_item<1, 3>(sm, aoff[g], boff[g], acc[g]); break;
+        case 4 * 1 + 3: dp_item<1, 4>(sm, aoff[g], boff[g], acc[g]); break;
+        case 4 * 2 + 0: dp_item<2, 1>(sm, aoff[g], boff[g], acc[g]); break;
+        case 4 * 2 + 1: dp_item<2, 2>(sm, aoff[g], boff[g], acc[g]); break;
+        case 4 * 2 + 2: dp_item<2, 3>(sm, aoff[g], boff[g], acc[g]); break;
+        case 4 * 2 + 3: dp_item<2, 4>(sm, aoff[g], boff[g], acc[g]); break;
+        default: break;
       }
     }
   }
   cp_async_wait<0>();
-  // partial sums: C(row gid, col 2 tig + i) of each tile
-  double2* out = reinterpret_cast<double2*>(a.partial) + (size_t)blockIdx.x * a.nblkent;
+  // partial sums: S(row gid, columns 2 tig, 2 tig + 1) of each tile
+  double* out = a.partial + (size_t)blockIdx.x * a.nent;
 #pragma unroll
   for (int g = 0; g < I2D_MAXG; ++g) {
-    if (nnt[g] == 0) continue;
-    const I2dGroup G = a.groups[wg[g]];
-    const int ae = a.a_ent[G.arow0 + gid];
+    const DotProdItem G = wi[g];
 #pragma unroll
-    for (int t = 0; t < I2D_NTMAX; ++t) {
-      if (t >= nnt[g]) continue;
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int bc = a.b_col[G.brow0 + 8 * t + 2 * tig + i];
-        if (ae >= 0 && bc >= 0)
-          out[ae + bc] = make_double2(acc[g][t][0][i] + acc[g][t][1][i], acc[g][t][2][i] + acc[g][t][3][i]);
-      }
-    }
+      for (int j = 0; j < 4; ++j)
+        if (i < nm[g] && j < nn[g])
+          *reinterpret_cast<double2*>(out + (size_t)(G.tile0 + (G.mt + i) * G.ntile + G.nt + j) * 64 + gid * 8 + 2 * tig) =
+              make_double2(acc[g][i][j][0], acc[g][i][j][1]);
   }
 }
 
-int launch_int2e_dmma(const I2dArgs& d, const Int2eArgs& sum, int nsplit, cudaStream_t st) {
-  const int n = sum.nact, n4 = n * n * n * n;
-  if (n4 == 0) return 0;
-  cudaError_t e = cudaMemsetAsync(sum.int2e, 0, sizeof(cplx) * n4, st);
-  if (e != cudaSuccess) return (int)e;
-  if (d.ngroups > 0) {
-    if (!int2e_dmma_fits(d)) return (int)cudaErrorInvalidValue;
-    const size_t smem = int2e_dmma_smem(d);
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(int2e_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-      attr = true;
-    }
-    dim3 grid(nsplit, d.nsets);
-    int2e_dmma_kernel<<<grid, I2D_NW * 32, smem, st>>>(d);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) {
-      fprintf(stderr, "td1c_b200: int2e DMMA kernel (grid %d x %d, smem %zu): %s\n", nsplit, d.nsets, smem,
-              cudaGetErrorString(e));
-      return (int)e;
-    }
+// fixed-order sums over the K slices: 32 entries x 32 slice groups per CTA (every load of a thread in
+// flight at once; with 8 groups the 37 loads of each took 9 us where the data fits in 1)
+__global__ void __launch_bounds__(1024) dot_sum_kernel(const double* __restrict__ partial, int nsplit, int nent,
+                                                       double* __restrict__ sum) {
+  __shared__ double part[32][33];
+  const int lane = threadIdx.x & 31, gq = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
+  double s = 0.0;
+  if (e < nent) {
+#pragma unroll 10
+    for (int c = gq; c < nsplit; c += 32) s += partial[(size_t)c * nent + e];
   }
-  return launch_int2e_sum_fill(sum, nsplit, st);
+  part[gq][lane] = s;
+  __syncthreads();
+  double t = part[lane][gq];  // warp gq adds the groups of entry gq by a fixed tree
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0 && blockIdx.x * 32 + gq < nent) sum[blockIdx.x * 32 + gq] = t;
+}
+
+// int2e(i, j, k, l) from the sums: form = (RR, RI, IR, II) entries (-1: zero), flag 1 the column is
+// conjugated, flag 2 the integral is the conjugate of int2e(j, i, l, k)
+__global__ void int2e_form_kernel(int n4, const int4* __restrict__ form, const unsigned char* __restrict__ flag,
+                                  const double* __restrict__ sum, cplx* __restrict__ int2e) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n4) return;
+  const int4 f = form[t];
+  cplx v = mkc(0, 0);
+  if (f.x >= 0) {
+    const double rr = sum[f.x], ri = f.y >= 0 ? sum[f.y] : 0.0, ir = f.z >= 0 ? sum[f.z] : 0.0, ii = f.w >= 0 ? sum[f.w] : 0.0;
+    const int fl = flag[t];
+    v = (fl & 1) ? mkc(rr + ii, ir - ri) : mkc(rr - ii, ri + ir);
+    if (fl & 2) v.y = -v.y;
+  }
+  int2e[t] = v;
+}
+
+// K slices: two CTAs per SM where they fit, and at least four stages of points each
+int dot_products_nsplit(const DotProdArgs& a, int nsm) {
+  const int per = 2 * dp_smem(a.nrow, dp_stages(a.nrow)) <= 224 * 1024 ? 2 : 1;
+  return std::max(1, std::min(per * nsm, (int)(a.K / (4 * I2D_KC))));
+}
+
+int launch_dot_products(const DotProdArgs& a, int nsplit, cudaStream_t st) {
+  if (a.nent <= 0) return 0;
+  const int ns = dp_stages(a.nrow);
+  const size_t smem = dp_smem(a.nrow, ns);
+  if (smem > 227 * 1024 || nsplit < 1) return (int)cudaErrorInvalidValue;
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(dot_products_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(dot_products_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    attr = true;
+  }
+  const dim3 grid(nsplit, a.nsets);
+  if (ns == 3) dot_products_kernel<3><<<grid, I2D_NW * 32, smem, st>>>(a);
+  else dot_products_kernel<2><<<grid, I2D_NW * 32, smem, st>>>(a);
+  dot_sum_kernel<<<(a.nent + 31) / 32, 1024, 0, st>>>(a.partial, nsplit, a.nent, a.sum);
+  return (int)cudaGetLastError();
+}
+
+int launch_int2e_dmma(const I2dArgs& d, int nsplit, cudaStream_t st) {
+  const int n4 = d.nact * d.nact * d.nact * d.nact;
+  if (n4 == 0) return 0;
+  const int rc = launch_dot_products(d.prod, nsplit, st);
+  if (rc) return rc;
+  int2e_form_kernel<<<(n4 + 255) / 256, 256, 0, st>>>(n4, d.form, d.flag, d.prod.sum, d.int2e);
+  return (int)cudaGetLastError();
 }
 
 }  // namespace td1c

@@ -11,94 +11,13 @@
 // order sum), the race-free pattern of the reference's per-thread partial
 // arrays.
 //
-// int2e (hprod_mkint2_sph.F90:2-100): int2e(i,j,k,l) = sum_{r,L} rho2_ij v2sph_kl
-// for i >= j active and m_i + m_k = m_j + m_l.  The m rule splits the
-// (ij) x (kl) matrix into dense blocks by delta = m_i - m_j; each block is a
-// complex GEMM over K = Nr (lmax2 + 1) split across CTAs, with A/B chunks
-// staged in shared memory; partials are summed in a fixed order and the
-// i < j half is filled by int2e(i,j,k,l) = conj(int2e(j,i,l,k)).
+// Also the fixed-order sum of the split-TF32 int2e's K slices (int2e_tc.cu) and
+// the i < j half, int2e(i,j,k,l) = conj(int2e(j,i,l,k)).
 #include "common.cuh"
 #include "kernels.cuh"
 #include "reductions.cuh"
 
 namespace td1c {
-
-constexpr int OD_CHUNK = 128;
-
-__global__ void __launch_bounds__(256) orbdots_kernel(OrbdotsArgs a) {
-  extern __shared__ cplx sm[];
-  const int nfun = a.nfun, C = OD_CHUNK;
-  cplx* so = sm;                       // [nfun][C] orb
-  cplx* sf = so + (size_t)nfun * C;    // [nfun][C] g + h1 + h0
-  cplx* sv = sf + (size_t)nfun * C;    // [nfun][C] v2
-  cplx* sh = sv + (size_t)nfun * C;    // [nfun][C] h0 + h1
-  cplx* sgv = sh + (size_t)nfun * C;   // [nfun][C] g + v2
-  const size_t base = (size_t)blockIdx.x * C;
-  for (int e = threadIdx.x; e < nfun * C; e += blockDim.x) {
-    int f = e / C, k = e % C;
-    size_t g = base + k;
-    cplx o = mkc(0, 0), fv = mkc(0, 0), v = mkc(0, 0), h = mkc(0, 0), gv = mkc(0, 0);
-    if (g < (size_t)a.nbas) {
-      size_t idx = (size_t)f * a.nbas + g;
-      o = a.orb[idx];
-      cplx h0 = a.h0orb[idx], h1 = a.h1orb[idx], gg = a.gorb[idx];
-      fv = cadd(cadd(gg, h1), h0);
-      v = a.v2orb[idx];
-      h = cadd(h0, h1);
-      gv = cadd(gg, v);
-    }
-    so[e] = o; sf[e] = fv; sv[e] = v; sh[e] = h; sgv[e] = gv;
-  }
-  __syncthreads();
-  cplx* out = a.partial + (size_t)blockIdx.x * a.nent;
-  // one warp per entry, lanes over the chunk (conflict-free), fixed-order
-  // shuffle reduction
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int t = wid; t < a.nent; t += nw) {
-    const int4 en = a.ent[t];  // (kind, j, i, 0)
-    const int kind = en.x, j = en.y, i = en.z;
-    const cplx* x; const cplx* y;
-    if (kind == 0) { x = so + j * C; y = sf + i * C; }        // A
-    else if (kind == 1) { x = so + j * C; y = sv + i * C; }   // B
-    else if (kind == 2) { x = sh + j * C; y = so + i * C; }   // C
-    else if (kind == 3) { x = so + i * C; y = sh + i * C; }   // E
-    else { x = so + j * C; y = sgv + i * C; }                 // <phi_j|(g+v2) phi_i>
-    cplx s = mkc(0, 0);
-    for (int k = lane; k < C; k += 32) {
-      cplx xv = x[k], yv = y[k];
-      s.x = fma(xv.x, yv.x, fma(xv.y, yv.y, s.x));
-      s.y = fma(xv.x, yv.y, fma(-xv.y, yv.x, s.y));
-    }
-    for (int o = 16; o > 0; o >>= 1) { s.x += __shfl_xor_sync(0xffffffff, s.x, o); s.y += __shfl_xor_sync(0xffffffff, s.y, o); }
-    if (lane == 0) out[t] = s;
-  }
-}
-
-// fixed-order sum of the per-chunk partials: one warp per entry, lane l adds
-// chunks l, l + 32, ... in order, then a fixed xor tree combines the lanes
-__global__ void sum_partials_kernel(const cplx* __restrict__ partial, int nchunk, int nent, cplx* __restrict__ out) {
-  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (t >= nent) return;
-  cplx s = mkc(0, 0);
-  for (int c = lane; c < nchunk; c += 32) s = cadd(s, partial[(size_t)c * nent + t]);
-  for (int o = 16; o > 0; o >>= 1) { s.x += __shfl_xor_sync(0xffffffffu, s.x, o); s.y += __shfl_xor_sync(0xffffffffu, s.y, o); }
-  if (lane == 0) out[t] = s;
-}
-
-int orbdots_nchunk(size_t nbas) { return (int)((nbas + OD_CHUNK - 1) / OD_CHUNK); }
-
-int launch_orbdots(const OrbdotsArgs& a, cudaStream_t st) {
-  const int nchunk = orbdots_nchunk((size_t)a.nbas);
-  size_t smem = sizeof(cplx) * 5 * (size_t)a.nfun * OD_CHUNK;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(orbdots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr = true;
-  }
-  orbdots_kernel<<<nchunk, 256, smem, st>>>(a);
-  sum_partials_kernel<<<(a.nent + 7) / 8, 256, 0, st>>>(a.partial, nchunk, a.nent, a.result);
-  return (int)cudaGetLastError();
-}
 
 // ---------------------------------------------------------------------------
 // int2e block GEMM: C(ij, kl) = sum_x A_ij[x] B_kl[x] over x in [0, K)
@@ -193,6 +112,83 @@ __global__ void __launch_bounds__(I2_NT) int2e_block_kernel(Int2eArgs a) {
           a.partial[((size_t)blockIdx.x * a.nblkent) + blk.ent0 + r * nc + c] = cadd(acc[i][j], sred[tt][i * 3 + j]);
       }
   }
+}
+
+constexpr int OD_CHUNK = 128;
+
+__global__ void __launch_bounds__(256) orbdots_kernel(OrbdotsArgs a) {
+  extern __shared__ cplx sm[];
+  const int nfun = a.nfun, C = OD_CHUNK;
+  cplx* so = sm;                       // [nfun][C] orb
+  cplx* sf = so + (size_t)nfun * C;    // [nfun][C] g + h1 + h0
+  cplx* sv = sf + (size_t)nfun * C;    // [nfun][C] v2
+  cplx* sh = sv + (size_t)nfun * C;    // [nfun][C] h0 + h1
+  cplx* sgv = sh + (size_t)nfun * C;   // [nfun][C] g + v2
+  const size_t base = (size_t)blockIdx.x * C;
+  for (int e = threadIdx.x; e < nfun * C; e += blockDim.x) {
+    int f = e / C, k = e % C;
+    size_t g = base + k;
+    cplx o = mkc(0, 0), fv = mkc(0, 0), v = mkc(0, 0), h = mkc(0, 0), gv = mkc(0, 0);
+    if (g < (size_t)a.nbas) {
+      size_t idx = (size_t)f * a.nbas + g;
+      o = a.orb[idx];
+      cplx h0 = a.h0orb[idx], h1 = a.h1orb[idx], gg = a.gorb[idx];
+      fv = cadd(cadd(gg, h1), h0);
+      v = a.v2orb[idx];
+      h = cadd(h0, h1);
+      gv = cadd(gg, v);
+    }
+    so[e] = o; sf[e] = fv; sv[e] = v; sh[e] = h; sgv[e] = gv;
+  }
+  __syncthreads();
+  cplx* out = a.partial + (size_t)blockIdx.x * a.nent;
+  // one warp per entry, lanes over the chunk (conflict-free), fixed-order
+  // shuffle reduction
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int t = wid; t < a.nent; t += nw) {
+    const int4 en = a.ent[t];  // (kind, j, i, 0)
+    const int kind = en.x, j = en.y, i = en.z;
+    const cplx* x; const cplx* y;
+    if (kind == 0) { x = so + j * C; y = sf + i * C; }        // A
+    else if (kind == 1) { x = so + j * C; y = sv + i * C; }   // B
+    else if (kind == 2) { x = sh + j * C; y = so + i * C; }   // C
+    else if (kind == 3) { x = so + i * C; y = sh + i * C; }   // E
+    else { x = so + j * C; y = sgv + i * C; }                 // <phi_j|(g+v2) phi_i>
+    cplx s = mkc(0, 0);
+    for (int k = lane; k < C; k += 32) {
+      cplx xv = x[k], yv = y[k];
+      s.x = fma(xv.x, yv.x, fma(xv.y, yv.y, s.x));
+      s.y = fma(xv.x, yv.y, fma(-xv.y, yv.x, s.y));
+    }
+    for (int o = 16; o > 0; o >>= 1) { s.x += __shfl_xor_sync(0xffffffff, s.x, o); s.y += __shfl_xor_sync(0xffffffff, s.y, o); }
+    if (lane == 0) out[t] = s;
+  }
+}
+
+// fixed-order sum of the per-chunk partials: one warp per entry, lane l adds
+// chunks l, l + 32, ... in order, then a fixed xor tree combines the lanes
+__global__ void sum_partials_kernel(const cplx* __restrict__ partial, int nchunk, int nent, cplx* __restrict__ out) {
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= nent) return;
+  cplx s = mkc(0, 0);
+  for (int c = lane; c < nchunk; c += 32) s = cadd(s, partial[(size_t)c * nent + t]);
+  for (int o = 16; o > 0; o >>= 1) { s.x += __shfl_xor_sync(0xffffffffu, s.x, o); s.y += __shfl_xor_sync(0xffffffffu, s.y, o); }
+  if (lane == 0) out[t] = s;
+}
+
+int orbdots_nchunk(size_t nbas) { return (int)((nbas + OD_CHUNK - 1) / OD_CHUNK); }
+
+int launch_orbdots(const OrbdotsArgs& a, cudaStream_t st) {
+  const int nchunk = orbdots_nchunk((size_t)a.nbas);
+  size_t smem = sizeof(cplx) * 5 * (size_t)a.nfun * OD_CHUNK;
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(orbdots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    attr = true;
+  }
+  orbdots_kernel<<<nchunk, 256, smem, st>>>(a);
+  sum_partials_kernel<<<(a.nent + 7) / 8, 256, 0, st>>>(a.partial, nchunk, a.nent, a.result);
+  return (int)cudaGetLastError();
 }
 
 // one warp per entry: lane l adds splits l, l + 32, ... in order, then a

@@ -14,6 +14,26 @@ struct OrbdotsArgs {
 int orbdots_nchunk(size_t nbas);  // chunks (CTAs) of the orbdots pass; the partial buffer holds nchunk x nent
 int launch_orbdots(const OrbdotsArgs& a, cudaStream_t st);
 
+// Real products over K points of the components (re, im) of a list of complex
+// rows, on the FP64 tensor cores (int2e_dmma.cu): S[x][y] = sum_k A_x[k] B_y[k]
+// in 8 x 8 tiles.  An item is up to 2 x 4 tiles of one block; the host assigns
+// at most I2D_MAXG items to each warp (nm = 0: none).
+constexpr int I2D_NW = 8, I2D_MAXG = 2;
+// block's first A and B component; tiles mt .. mt + nm - 1, nt .. nt + nn - 1; block's first tile, tiles per row
+struct DotProdItem { int compa, compb, mt, nm, nt, nn, tile0, ntile; };
+struct DotProdArgs {
+  int nrow, nent, nsets;
+  size_t K;
+  const cplx* const* row;    // [nrow]
+  const int* comp;           // row | part << 16
+  const DotProdItem* items;  // [nsets][I2D_NW][I2D_MAXG]
+  double* partial;           // [nsplit][nent]
+  double* sum;               // [nent]
+};
+int dot_products_nsplit(const DotProdArgs& a, int nsm);
+int launch_dot_products(const DotProdArgs& a, int nsplit, cudaStream_t st);
+
+// int2e as FFMA blocks (the no-allocation call) and the entries of the split-TF32 int2e
 struct Int2eBlock { int row0, nrow, col0, ncol, ent0, pad0, pad1, pad2; };
 struct Int2eArgs {
   int nact, nblocks, nblkent;
@@ -29,30 +49,17 @@ struct Int2eArgs {
 };
 int launch_int2e(const Int2eArgs& a, int nsplit, cudaStream_t st);
 
-// int2e on the FP64 tensor cores (DMMA m8n8k4), split over K.  Every
-// Delta-m block is padded to m-tiles of 8 row pairs (rho2) and n-tiles of 8
-// columns (v2sph); a group is one m-tile x up to I2D_NTMAX n-tiles, and the
-// host assigns at most I2D_MAXG groups to each warp (-1: none).
-constexpr int I2D_NW = 16, I2D_MAXG = 1, I2D_NTMAX = 3;
-struct I2dGroup { int arow0, brow0, nnt, pad; };  // 8 A rows x nnt n-tiles (8 B rows each)
+// int2e on the FP64 tensor cores: the products of the stored active pairs' rho2
+// and v2sph rows per |Delta m| block, K = Nr (lmax2 + 1)
 struct I2dArgs {
-  int nra, nrb, ngroups, nblkent;
-  size_t K;
-  const int* a_pair;     // [nra] stored pair of the padded A row (-1: padding)
-  const int* a_ent;      // [nra] first entry of the row (ent0 + r ncol), -1 for padding
-  const int2* b_pair;    // [nrb] (stored pair, conj) of the padded B row ((-1, 0): padding)
-  const int* b_col;      // [nrb] column index inside its block, -1 for padding
-  const I2dGroup* groups;
-  const int* warp_group;  // [nsets][I2D_NW][I2D_MAXG] group of each warp slot, -1: none
-  int nsets;
-  const cplx* rho2;
-  const cplx* v2sph;
-  double* partial;       // [nsplit][nblkent][2]
+  DotProdArgs prod;
+  int nact;
+  const int4* form;           // [nact^4] entries (RR, RI, IR, II) of each integral, -1: zero
+  const unsigned char* flag;  // [nact^4] 1 conjugated column, 2 conjugated integral
+  cplx* int2e;                // [nact^4]
 };
 int launch_int2e_sum_fill(const Int2eArgs& a, int nsplit, cudaStream_t st);
-size_t int2e_dmma_smem(const I2dArgs& a);
-bool int2e_dmma_fits(const I2dArgs& a);
-int launch_int2e_dmma(const I2dArgs& d, const Int2eArgs& sum, int nsplit, cudaStream_t st);
+int launch_int2e_dmma(const I2dArgs& d, int nsplit, cudaStream_t st);
 
 // int2e in split TF32 on tcgen05 (the mixed-precision form): every product of
 // the P stored active pairs in one 128 x 2NB GEMM per K slice, entries formed
