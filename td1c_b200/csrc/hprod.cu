@@ -116,6 +116,7 @@ struct Ctx {
   // ---- hprod_bind_ outputs
   double *p_ene_fcore = nullptr, *p_ene_dcore = nullptr, *p_ene_core = nullptr, *p_ene_act = nullptr, *p_ene_tot = nullptr;
   // ---- device tables
+  double* ob_tab = nullptr;  // one-body blocks of the elements
   double *xrad = nullptr, *mask = nullptr, *radk = nullptr, *radk0 = nullptr, *radp = nullptr, *cost = nullptr;
   double *legf1 = nullptr, *legb1 = nullptr, *legf2 = nullptr, *legb2 = nullptr, *alph = nullptr;
   // parity halves of the same tables (null when the bound theta grid is not symmetric)
@@ -875,6 +876,8 @@ int build_tables(Ctx& c) {
     cudaMemcpy(&hst, dstat, sizeof(int), cudaMemcpyDeviceToHost);
     if (hst) { fprintf(stderr, "td1c_b200: condensed Poisson factorisation failed\n"); return ST_CHOLESKY; }
   }
+  c.ob_tab = dalloc<double>(onebody_table_size(c.nd, c.nfe));
+  if (launch_onebody_tables(c.nfe, c.nd, Nr, c.radk, c.radk0, c.radp, c.ob_tab, 0)) return ST_CUDA;
   c.tdiag = dalloc<double>((size_t)Nr * c.L1);
   c.v2jfc = dalloc<double>(Nr);
   tdiag_kernel<<<(Nr * c.L1 + 255) / 256, 256>>>(Nr, c.L1, c.nd, c.znuc, c.xrad, c.radk, c.radk0, nullptr, c.tdiag);
@@ -1517,7 +1520,7 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
   // one-body
   OneBodyArgs ob{};
   ob.Nr = c.Nr; ob.L1 = c.L1; ob.nd = c.nd; ob.nfun = c.nfun; ob.nfcore = c.nfcore; ob.mmax1 = c.mmax1; ob.igauge = c.igauge;
-  ob.radk = c.radk; ob.radk0 = c.radk0; ob.radp = c.radp; ob.tdiag = c.tdiag; ob.xrad = c.xrad; ob.alph = c.alph;
+  ob.tab = c.ob_tab; ob.tdiag = c.tdiag; ob.xrad = c.xrad; ob.alph = c.alph;
   ob.mval = c.d_mval; ob.orb = c.orb; ob.h0orb = c.h0orb; ob.h1orb = c.h1orb; ob.lfield = d_lf;
   // the one-body stencil reads only the orbitals and the field: it runs on
   // the third stream, overlapping the mean-field chain, and joins before
@@ -2201,7 +2204,7 @@ int h1rat_run(Ctx& c, const Etd4Fun& F, const double* d_lf, cplx* w, int maxcyc,
   zaxpby(c, nd, w + nf, w + nf, w + nf, F.n[0], mkc(0, 0));
   OneBodyArgs ob{};
   ob.Nr = c.Nr; ob.L1 = c.L1; ob.nd = c.nd; ob.nfun = c.nfun; ob.nfcore = c.nfcore; ob.mmax1 = c.mmax1; ob.igauge = c.igauge;
-  ob.radk = c.radk; ob.radk0 = c.radk0; ob.radp = c.radp; ob.tdiag = c.tdiag; ob.xrad = c.xrad; ob.alph = c.alph;
+  ob.tab = c.ob_tab; ob.tdiag = c.tdiag; ob.xrad = c.xrad; ob.alph = c.alph;
   ob.mval = c.d_mval; ob.orb = t; ob.h0orb = c.h0orb; ob.h1orb = c.h1orb; ob.lfield = d_lf;
   for (int k = 1; k <= 2; ++k) {
     rc |= launch_onebody(ob, st);
@@ -2867,7 +2870,7 @@ void hprod_set_wfn0_(const double* wfn, const double* cic, const char* v2xfc_typ
   // with h0 from the bare kinetic table (before v2jfc is added)
   OneBodyArgs ob{};
   ob.Nr = c.Nr; ob.L1 = c.L1; ob.nd = c.nd; ob.nfun = c.nfcore; ob.nfcore = c.nfcore; ob.mmax1 = c.mmax1; ob.igauge = 0;
-  ob.radk = c.radk; ob.radk0 = c.radk0; ob.radp = c.radp; ob.tdiag = c.tdiag; ob.xrad = c.xrad; ob.alph = c.alph;
+  ob.tab = c.ob_tab; ob.tdiag = c.tdiag; ob.xrad = c.xrad; ob.alph = c.alph;
   ob.mval = c.d_mval; ob.orb = c.orb; ob.h0orb = c.h0orb; ob.h1orb = c.h1orb; ob.lfield = c.lfield;
   cudaMemsetAsync(c.lfield, 0, 9 * sizeof(double), st);
   launch_onebody(ob, st);
@@ -3089,7 +3092,7 @@ int td1c_gpu_dipole3(const void* d_wfn, const void* d_cic, const double* lfield,
   // p_z phi: the velocity coupling of the one-body kernel (igauge 1, unit field); z phi (igauge 0)
   OneBodyArgs ob{};
   ob.Nr = c.Nr; ob.L1 = c.L1; ob.nd = c.nd; ob.nfun = c.nfun; ob.nfcore = 0; ob.mmax1 = c.mmax1; ob.igauge = 1;
-  ob.radk = c.radk; ob.radk0 = c.radk0; ob.radp = c.radp; ob.tdiag = c.tdiag; ob.xrad = c.xrad; ob.alph = c.alph;
+  ob.tab = c.ob_tab; ob.tdiag = c.tdiag; ob.xrad = c.xrad; ob.alph = c.alph;
   ob.mval = c.d_mval; ob.orb = w; ob.h0orb = fc ? c.dip_g : c.h0orb; ob.h1orb = fc ? c.dip_p : c.h1orb; ob.lfield = c.dip_lf;
   rc |= chk("onebody", launch_onebody(ob, st));
   const cplx* po = fc ? c.dip_p : c.h1orb;

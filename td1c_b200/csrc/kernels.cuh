@@ -104,9 +104,7 @@ int mlp_infer_prepare();
 // ---- one-body: tprod + zprod/pzprod (hprod_tprod.F90, hprod_zprod.F90, hprod_pzprod.F90)
 struct OneBodyArgs {
   int Nr, L1, nd, nfun, nfcore, mmax1, igauge;
-  const double* radk;    // (2nd+1) x (nrad+1) band, reference layout
-  const double* radk0;
-  const double* radp;
+  const double* tab;     // kinetic and derivative blocks of the elements (launch_onebody_tables)
   const double* tdiag;   // [L1][Nr] diagonal of tmat (centrifugal + nuclear + radk diag + v2jfc)
   const double* xrad;    // [nrad+1]
   const double* alph;    // [(2 mmax1 + 1)][L1]
@@ -116,6 +114,9 @@ struct OneBodyArgs {
   cplx* h1orb;
   const double* lfield;  // device: lfield(1:3,1:3) column-major (9 doubles)
 };
+size_t onebody_table_size(int nd, int nfe);  // doubles
+int launch_onebody_tables(int nfe, int nd, int Nr, const double* radk, const double* radk0, const double* radp, double* tab,
+                          cudaStream_t st);
 int launch_onebody(const OneBodyArgs& a, cudaStream_t st);
 
 // ---- Poisson (hprod_mkv2mf.F90:118-182): per (pair, l) banded Cholesky solve

@@ -66,6 +66,7 @@ def test_folded_and_dense_transforms(cuda_ok, lmax, nlat):
 ORBITAL_SETS = {
     "two": ([(1, 0, 0, 1), (2, 0, 0, 1)], 1, 1, 0, 1),
     "three_m": ([(2, 1, -1, 1), (2, 1, 0, 1), (2, 1, 1, 1)], 2, 1, 1, 2),
+    "five": ([(1, 0, 0, 0), (2, 0, 0, 1), (2, 1, -1, 1), (2, 1, 0, 1), (2, 1, 1, 1)], 3, 3, 0, 1),  # 15 pairs
     "d_shell": ([(1, 0, 0, -1), (2, 0, 0, 1)] + [(3, 2, m, 1) for m in (-2, -1, 0, 1, 2)], 3, 3, 0, 1),
     "two_dynamic_cores": ([(1, 0, 0, 0), (2, 0, 0, 0), (2, 1, 0, 1), (3, 1, 0, 1), (3, 0, 0, 1), (3, 2, 0, 1), (4, 0, 0, 1)], 4, 4, 0, 1),
 }
