@@ -937,6 +937,12 @@ int build_state(Ctx& c) {
     a.tpart = dalloc<cplx>(nl * c.nfe);
     a.xb = dalloc<cplx>(nl * std::max(1, c.nfe - 1));
     a.t = dalloc<cplx>(nl);
+    if (ps_few_fits(a.f, c.npair)) {
+      size_t nwf, nsf, nbi;
+      ps_few_sizes(a.f, &nwf, &nsf, &nbi);
+      a.f.wfrag = dalloc<double>(nwf); a.f.sfrag = dalloc<double>(nsf); a.f.binv = dalloc<double>(nbi);
+      if (launch_ps_few_setup(a.f, 0)) return ST_CUDA;
+    }
   }
   return 0;
 }

@@ -160,6 +160,10 @@ struct PsCond {
   double* tm = nullptr;    // [L2][nb] LU of the bridge system: multipliers,
   double* tw = nullptr;    //   reciprocal pivots,
   double* tu = nullptr;    //   superdiagonal
+  // DMMA operands in fragment order of the passes for few pairs (poisson_few.cu); null for more
+  double* wfrag = nullptr; // per (l, element): element pass
+  double* sfrag = nullptr; // per (l, element): share pass
+  double* binv = nullptr;  // per l: inverse of the bridge matrix
 };
 struct PsCondArgs {
   PsCond f;
@@ -177,6 +181,11 @@ struct PsCondArgs {
 int launch_ps_cond_setup(PsCond& f, const double* xrad, const double* radk, const double* invr, const double* rpl0,
                          const double* rpl1, const double* fac2, int* status, cudaStream_t st);
 int launch_ps_cond(const PsCondArgs& a, cudaStream_t st);
+constexpr int PS_FEW = 16;
+bool ps_few_fits(const PsCond& f, int npair);
+void ps_few_sizes(const PsCond& f, size_t* wfrag, size_t* sfrag, size_t* binv);  // doubles
+int launch_ps_few_setup(const PsCond& f, cudaStream_t st);
+int launch_ps_few(const PsCondArgs& a, cudaStream_t st);
 
 // ---- mean-field action on the (r, theta) grid (hprod_mfprod2.F90)
 struct Act2Block {     // one dense (ij) x (kl) block of the 2-RDM contraction

@@ -601,6 +601,7 @@ int launch_ps_cond(const PsCondArgs& a, cudaStream_t st) {
   static_assert(PSE_NT == 64 * PSE_LC && PSE_PC == 32, "element pass: two warps of 16 pairs per multipole");
   static_assert(PSE_NT % PSE_LC == 0, "record staging: PSE_NT / LC threads per record");
   if (a.npair <= 0) return 0;
+  if (a.f.wfrag && !a.tf32) return launch_ps_few(a, st);  // up to PS_FEW pairs (poisson_few.cu)
   if (a.f.nd - 1 > 8 * PSE_MT || a.f.nd - 1 > 4 * PSE_KS) return ST_CONFIG;
   int rc = launch_ps_pass(a, true, st);
   if (rc) return rc;
