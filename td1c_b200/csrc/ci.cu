@@ -206,7 +206,9 @@ __global__ void __launch_bounds__(128) ci_sigma_kernel(CiArgs a) {
   cplx c = a.cic[J];
   sig = csub(sig, cscale(c, e));
   cplx fac = a.icomp == 1 ? mkc(0.0, -a.dtime) : mkc(-a.dtime, 0.0);
-  a.sigma[J] = cmul(sig, fac);
+  const cplx k = cmul(sig, fac);
+  if (a.rk.stage == 0) a.sigma[J] = k;
+  else rk_put(a.rk, J, k);
 }
 
 int launch_ci_dvec(const CiArgs& a, int maxsec, cudaStream_t st) {

@@ -705,30 +705,45 @@ __global__ void __launch_bounds__(256) smallmat_kernel(SmallArgs a) {
   }
 }
 
-// hwfn_i = tf2 (v2 + g [+ h1 [+ h0]])_i + sum_{j, m_j = m_i} orb_j X(j,i)
-// (hprod_htot_dtorb.F90:54-104); frozen-core rows are zero.
-__global__ void dtorb_kernel(int Nr, int L1, int nfun, int nfcore, int icomp, int isplit, double dtime, const int* __restrict__ mval,
-                             const cplx* __restrict__ orb, const cplx* __restrict__ h0, const cplx* __restrict__ h1,
-                             const cplx* __restrict__ gg, const cplx* __restrict__ v2, const cplx* __restrict__ xmat,
-                             cplx* __restrict__ hwfn) {
-  const size_t nb = (size_t)Nr * L1;
-  size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nb * nfun) return;
-  const int i = (int)(t / nb);
-  const size_t k = t % nb;
-  if (i < nfcore) { hwfn[t] = mkc(0, 0); return; }
-  const cplx tf2 = icomp == 0 ? mkc(-dtime, 0) : mkc(0, -dtime);
-  // isplit 0: v2 + g + h1 + h0; 2: without h0; 1: without h1 and h0 (hprod_htot_dtorb.F90:58-84)
-  cplx h = cadd(v2[t], gg[t]);
-  if (isplit != 1) h = cadd(h, h1[t]);
-  if (isplit == 0) h = cadd(h, h0[t]);
-  cplx o = cmul(h, tf2);
-  const int mi = mval[i];
-  for (int j = 0; j < nfun; ++j) {
-    if (mval[j] != mi) continue;
-    o = cadd(o, cmul(orb[(size_t)j * nb + k], xmat[j + nfun * i]));
+// k_i = tf2 (v2 + g [+ h1 [+ h0]])_i + sum_{j, m_j = m_i} orb_j X(j,i)
+// (hprod_htot_dtorb.F90:54-104); frozen-core rows are zero.  A CTA takes 32 basis functions, a warp per
+// orbital: the orbitals' values are read once into shared memory, so an RK4 stage can overwrite them with
+// the next stage's in place.
+__global__ void __launch_bounds__(512) dtorb_kernel(size_t nb, int nfun, int nfcore, int icomp, int isplit, double dtime,
+                                                    const int* __restrict__ mval, const cplx* orb, const cplx* __restrict__ h0,
+                                                    const cplx* __restrict__ h1, const cplx* __restrict__ gg,
+                                                    const cplx* __restrict__ v2, const cplx* __restrict__ xmat,
+                                                    cplx* __restrict__ hwfn, RkStage rk) {
+  __shared__ cplx so[16][32], sx[16 * 16];
+  __shared__ int sm[16];
+  const int i = threadIdx.x >> 5, lane = threadIdx.x & 31;  // blockDim = 32 nfun
+  const size_t k = (size_t)blockIdx.x * 32 + lane, t = (size_t)i * nb + k;
+  const bool in = k < nb, dyn = i >= nfcore;
+  cplx h = mkc(0, 0);
+  if (in) {
+    so[i][lane] = orb[t];
+    if (dyn) {
+      // isplit 0: v2 + g + h1 + h0; 2: without h0; 1: without h1 and h0 (hprod_htot_dtorb.F90:58-84)
+      h = cadd(v2[t], gg[t]);
+      if (isplit != 1) h = cadd(h, h1[t]);
+      if (isplit == 0) h = cadd(h, h0[t]);
+    }
   }
-  hwfn[t] = o;
+  for (int e = threadIdx.x; e < nfun * nfun; e += blockDim.x) sx[e] = xmat[e];
+  if (threadIdx.x < nfun) sm[threadIdx.x] = mval[threadIdx.x];
+  __syncthreads();
+  if (!in) return;
+  if (!dyn) {
+    if (rk.stage == 0) hwfn[t] = mkc(0, 0);
+    return;
+  }
+  const cplx tf2 = icomp == 0 ? mkc(-dtime, 0) : mkc(0, -dtime);
+  cplx o = cmul(h, tf2);
+  const int mi = sm[i];
+  for (int j = 0; j < nfun; ++j)
+    if (sm[j] == mi) o = cadd(o, cmul(so[j][lane], sx[j + nfun * i]));
+  if (rk.stage == 0) hwfn[t] = o;
+  else rk_put(rk, t, o);
 }
 
 // ===========================================================================
@@ -1472,22 +1487,27 @@ int chk(const char* what, int rc) {
   return rc;
 }
 
-// d_lf: device lfield[9]; wfn/cic device inputs; hwfn/hcic device outputs
-int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cplx* hwfn, cplx* hcic, double dtime) {
+// d_lf: device lfield[9]; wfn/cic device inputs (wfn null: the orbitals already stand in c.orb);
+// hwfn/hcic device outputs, or (rk) the RK4 stage that takes the value of the orbitals and of the CI vector
+int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cplx* hwfn, cplx* hcic, double dtime,
+             const RkStage* rk = nullptr, const RkStage* rk_ci = nullptr) {
   cudaStream_t st = c.st;
-  const size_t so = c.nbas * c.nfun, sg = c.ngrid * c.nfun;
+  const size_t so = c.nbas * c.nfun;
   int rc = 0;
   int iev = 0;
   auto mark = [&]() { if (c.profile && iev < 16) cudaEventRecord(c.ev[iev++], st); };
   mark();
-  // scratch initialisation (hprod_htot_init.F90)
-  (void)sg;  // gorbg / v2orbg rows of dynamic orbitals are fully written by mfprod
-  cudaMemsetAsync(c.gorb, 0, so * sizeof(cplx), st);
-  cudaMemsetAsync(c.v2orb, 0, so * sizeof(cplx), st);
+  // scratch initialisation (hprod_htot_init.F90): a mean field writes every dynamic row of gorb and v2orb
+  // (the frozen-core rows stay zero); without one they are zero
+  if (c.neltot < 2 || c.npair == 0) {
+    cudaMemsetAsync(c.gorb, 0, so * sizeof(cplx), st);
+    cudaMemsetAsync(c.v2orb, 0, so * sizeof(cplx), st);
+  }
   // RDMs (ormas_mkden1/2, hprod_invden)
   CiArgs ca{};
   ca.t = c.cit; ca.cic = cic_in; ca.Da = c.Da; ca.Db = c.Db; ca.T = c.T; ca.den1 = c.den1; ca.den2 = c.den2;
   ca.sigma = hcic; ca.int1e = c.int1e; ca.int2e = c.int2e; ca.ene_act = c.ene + 3; ca.dtime = dtime; ca.icomp = c.icomp;
+  if (rk_ci) ca.rk = *rk_ci;
   // The RDM chain reads only the CI vector, and its first consumer is
   // mfprod: it runs on the side stream, concurrently with the orbital
   // transform, the one-body stencil, the pair densities, the Poisson solve
@@ -1507,8 +1527,9 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
   }
   auto join = [&]() { if (fork) cudaStreamWaitEvent(st, c.ev_join, 0); };
   // orbitals (hprod_orbin.F90)
-  cudaMemcpyAsync(c.orb + c.nfcore * c.nbas, wfn + c.nfcore * c.nbas, (so - c.nfcore * c.nbas) * sizeof(cplx),
-                  cudaMemcpyDeviceToDevice, st);
+  if (wfn)
+    cudaMemcpyAsync(c.orb + c.nfcore * c.nbas, wfn + c.nfcore * c.nbas, (so - c.nfcore * c.nbas) * sizeof(cplx),
+                    cudaMemcpyDeviceToDevice, st);
   if (c.n_orbg) rc |= chk("orbg gemm", gemm(c, c.b_orbg, c.n_orbg, c.nlat, c.L1, false));
   if (c.nfcore > 0) {
     if (c.igauge == 0) {
@@ -1614,13 +1635,14 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
     rc |= chk("ci sigma", launch_ci_sigma(ca, c.st2));
     cudaEventRecord(c.ev_sig_join, c.st2);
     c.launches += 1;
-  } else {
+  } else if (!rk_ci) {
     cudaMemsetAsync(hcic, 0, sizeof(cplx), st);
   }
   mark();  // end ci_sigma (the sigma itself overlaps dtorb)
   // dtorb
-  dtorb_kernel<<<(unsigned)((so + 255) / 256), 256, 0, st>>>(c.Nr, c.L1, c.nfun, c.nfcore, c.icomp, c.isplit, dtime, c.d_mval, c.orb,
-                                                             c.h0orb, c.h1orb, c.gorb, c.v2orb, c.xmat, hwfn);
+  dtorb_kernel<<<(unsigned)((c.nbas + 31) / 32), 32 * c.nfun, 0, st>>>(
+      c.nbas, c.nfun, c.nfcore, c.icomp, c.isplit, dtime, c.d_mval, c.orb, c.h0orb, c.h1orb, c.gorb, c.v2orb, c.xmat, hwfn,
+      rk ? *rk : RkStage{});
   c.launches++;
   if (c.nact > 0) cudaStreamWaitEvent(st, c.ev_sig_join, 0);
   mark();  // end dtorb (and sigma)
@@ -1630,24 +1652,8 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
 }
 
 // ===========================================================================
-// RK4 (clcrk::prop, src/prop/clcrk.cpp:55-87; tableau set_coeff_04 221-235)
+// propagation kernels
 // ===========================================================================
-// y += wy k ;  ynext = y0 + wn k   (orbitals and CI handled as two segments)
-__global__ void rk_combine_kernel(size_t n, cplx* __restrict__ y, const cplx* __restrict__ y0, const cplx* __restrict__ k,
-                                  cplx* __restrict__ ynext, double wy, double wn, int do_next) {
-  size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  cplx kv = k[t];
-  cplx yv = y[t];
-  yv.x = fma(wy, kv.x, yv.x); yv.y = fma(wy, kv.y, yv.y);
-  y[t] = yv;
-  if (do_next) {
-    cplx a = y0[t];
-    a.x = fma(wn, kv.x, a.x); a.y = fma(wn, kv.y, a.y);
-    ynext[t] = a;
-  }
-}
-
 // wfn_mask (src/wfn/wfn_mask.F90:2-35): orb(irad, l, i) *= mask(irad) for
 // dynamic i, l >= |m_i|, irad >= min_irad
 __global__ void mask_kernel(int Nr, int L1, int nfun, int nfcore, int min_irad, const int* __restrict__ mval,
@@ -2032,26 +2038,25 @@ int h1_run(Ctx& c, bool pade, cplx fac, cplx zf0, bool allow_cycles, const doubl
   return rc ? ST_CUDA : 0;
 }
 
-// the four stages of clcrk::prop (clcrk.cpp:55-87, set_coeff_04 221-235)
-// from the state (y_orb, y_cic), stage fields lf[0..35] on the device
-int rk4_stages(Ctx& c, cplx* y_orb, cplx* y_cic, double dt, const double* lf) {
-  cudaStream_t st = c.st;
-  const size_t no = c.nbas * c.nfun, nc = c.lcic;
+// stage is (0 .. 3) of clcrk::prop (clcrk.cpp:55-87, set_coeff_04 221-235) from the state (y_orb, y_cic) at
+// the step's start with the stage field lf: the first stage copies the orbitals into the context, the
+// others find theirs there (and in b.yt) as the stage before left them
+int rk4_stage(Ctx& c, int is, cplx* y_orb, cplx* y_cic, double dt, const double* lf) {
+  const size_t no = c.nbas * c.nfun;
   RkBufs& b = c.rk;
-  const double wts[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
-  const double anext[4] = {0.5, 0.5, 1.0, 0.0};
-  cudaMemcpyAsync(b.y0, y_orb, no * sizeof(cplx), cudaMemcpyDeviceToDevice, st);
-  cudaMemcpyAsync(b.y0 + no, y_cic, nc * sizeof(cplx), cudaMemcpyDeviceToDevice, st);
+  static const double wts[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
+  static const double anext[4] = {0.5, 0.5, 1.0, 0.0};
+  RkStage so, sc;
+  so.stage = sc.stage = is + 1;
+  so.wt = sc.wt = dt * wts[is];
+  so.an = sc.an = dt * anext[is];
+  so.y = y_orb; so.acc = b.k; so.next = c.orb;
+  sc.y = y_cic; sc.acc = b.k + no; sc.next = b.yt + no;
+  return run_htot(c, lf, is == 0 ? y_orb : nullptr, is == 0 ? y_cic : b.yt + no, nullptr, nullptr, 1.0, &so, &sc);
+}
+int rk4_stages(Ctx& c, cplx* y_orb, cplx* y_cic, double dt, const double* lf) {
   int rc = 0;
-  for (int is = 0; is < 4; ++is) {
-    const cplx* in = (is == 0) ? b.y0 : b.yt;
-    rc |= run_htot(c, lf + 9 * is, in, in + no, b.k, b.k + no, 1.0);
-    const int nxt = is < 3 ? 1 : 0;
-    rk_combine_kernel<<<(unsigned)((no + 255) / 256), 256, 0, st>>>(no, y_orb, b.y0, b.k, b.yt, dt * wts[is], dt * anext[is], nxt);
-    rk_combine_kernel<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(nc, y_cic, b.y0 + no, b.k + no, b.yt + no, dt * wts[is],
-                                                                  dt * anext[is], nxt);
-    c.launches += 2;
-  }
+  for (int is = 0; is < 4; ++is) rc |= rk4_stage(c, is, y_orb, y_cic, dt, lf + 9 * is);
   return rc;
 }
 
@@ -2369,27 +2374,14 @@ int lp_j(Ctx& c, const cplx* y, const double* d_lf) {
 // exact W_n, int2e_n (the last J), stages 2 and 3 the c = 1/2 values, stage 4
 // the c = 1 values
 int lp_rk4_pred(Ctx& c, cplx* y_orb, cplx* y_cic, double dt, const double* lf) {
-  cudaStream_t st = c.st;
-  const size_t no = c.nbas * c.nfun, nc = c.lcic;
-  RkBufs& b = c.rk;
-  const double wts[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
-  const double anext[4] = {0.5, 0.5, 1.0, 0.0};
-  cudaMemcpyAsync(b.y0, y_orb, no * sizeof(cplx), cudaMemcpyDeviceToDevice, st);
-  cudaMemcpyAsync(b.y0 + no, y_cic, nc * sizeof(cplx), cudaMemcpyDeviceToDevice, st);
   int rc = 0;
   c.mf_external = 1;
   for (int is = 0; is < 4; ++is) {
     if (is == 1 || is == 3) {
-      rc |= chk("lp stage", launch_lp_stage(c.lp, is == 1 ? 1 : 0, st));
+      rc |= chk("lp stage", launch_lp_stage(c.lp, is == 1 ? 1 : 0, c.st));
       c.launches += 2;
     }
-    const cplx* in = (is == 0) ? b.y0 : b.yt;
-    rc |= run_htot(c, lf + 9 * is, in, in + no, b.k, b.k + no, 1.0);
-    const int nxt = is < 3 ? 1 : 0;
-    rk_combine_kernel<<<(unsigned)((no + 255) / 256), 256, 0, st>>>(no, y_orb, b.y0, b.k, b.yt, dt * wts[is], dt * anext[is], nxt);
-    rk_combine_kernel<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(nc, y_cic, b.y0 + no, b.k + no, b.yt + no, dt * wts[is],
-                                                                  dt * anext[is], nxt);
-    c.launches += 2;
+    rc |= rk4_stage(c, is, y_orb, y_cic, dt, lf + 9 * is);
   }
   c.mf_external = 0;
   return rc;
@@ -2891,6 +2883,7 @@ void hprod_set_wfn0_(const double* wfn, const double* cic, const char* v2xfc_typ
   cudaStreamSynchronize(st);
   c.ene_fcore = 2.0 * es[0] + es[1];
   cudaMemsetAsync(c.gorbg, 0, c.nfcore * c.ngrid * sizeof(cplx), st);  // scratch of the energy only
+  cudaMemsetAsync(c.gorb, 0, c.nfcore * c.nbas * sizeof(cplx), st);
   // hprod_addfc_tmat: add v2jfc to the kinetic diagonal; the one-body
   // propagator factors of the old T are stale
   tdiag_kernel<<<(c.Nr * c.L1 + 255) / 256, 256, 0, st>>>(c.Nr, c.L1, c.nd, c.znuc, c.xrad, c.radk, c.radk0, c.v2jfc, c.tdiag);
@@ -3112,6 +3105,7 @@ int td1c_gpu_dipole3(const void* d_wfn, const void* d_cic, const double* lfield,
     RowDotBufs bufs{{c.orb, c.dip_z, c.dip_p, c.dip_g}};
     rowdot_kernel<<<c.dip_rd_n, 256, 0, st>>>(c.nbas, bufs, c.dip_rd_ent, c.dip_rd);
     rc |= chk("gfock overlaps", (int)cudaGetLastError());
+    cudaMemsetAsync(c.gorb, 0, c.nfcore * c.nbas * sizeof(cplx), st);  // the RHS leaves the frozen-core rows zero
   }
   DipoleArgs da{};
   da.Nr = c.Nr; da.L1 = c.L1; da.mmax1 = c.mmax1; da.ncore = c.ncore; da.nact = c.nact; da.nent = c.dip_nent;

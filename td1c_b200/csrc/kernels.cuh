@@ -17,6 +17,26 @@
 
 namespace td1c {
 
+// What an RHS does with its value k: writes it out (stage 0), or makes it stage 1 .. 4 of an RK4 step
+// (clcrk::prop, src/prop/clcrk.cpp:55-87; tableau set_coeff_04 221-235): acc = or += wt k, the next stage's
+// state y + an k, and after stage 4 y += acc.  y is the state at the step's start until then.
+struct RkStage {
+  int stage = 0;
+  double wt = 0, an = 0;
+  cplx *y = nullptr, *acc = nullptr, *next = nullptr;
+};
+__device__ __forceinline__ void rk_put(const RkStage& s, size_t at, cplx k) {
+  cplx v = s.stage > 1 ? s.acc[at] : mkc(0, 0);
+  v.x = fma(s.wt, k.x, v.x); v.y = fma(s.wt, k.y, v.y);
+  const cplx y = s.y[at];
+  if (s.stage == 4) {
+    s.y[at] = cadd(y, v);
+  } else {
+    s.acc[at] = v;
+    s.next[at] = mkc(fma(s.an, k.x, y.x), fma(s.an, k.y, y.y));
+  }
+}
+
 struct LegGemmBatch {
   const double* A;   // real table, M x K row-major, row pitch lda (16-byte aligned rows, zero past K up to lda)
   const double* B0;  // slab (K rows x ldb reals) or conj operand for pair mode
@@ -303,6 +323,7 @@ struct CiArgs {
   const cplx* int2e;
   const double* ene_act;  // device scalar
   double dtime; int icomp;
+  RkStage rk;             // stage > 0: sigma goes into an RK4 stage of the CI vector instead of out
 };
 int launch_ci_dvec(const CiArgs& a, int maxsec, cudaStream_t st);
 int launch_ci_rdm(const CiArgs& a, cudaStream_t st);
