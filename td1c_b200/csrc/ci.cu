@@ -56,17 +56,18 @@ __global__ void ci_dvec_kernel(CiArgs a) {
   const long o = t.dvec_off[pq];
   const int ka = t.sec_detA[t.sec_base[sec] + K], kb = t.sec_detB[t.sec_base[sec] + K];
   const int sec0 = t.mtot - t.smin;
+  const cplx* __restrict__ cic = a.io ? a.io->cic : a.cic;
   cplx da = mkc(0, 0), db = mkc(0, 0);
   int sg;
   unsigned ia = excite_str(t.stra[ka], q, p, sg);
   if (ia != ~0u) {
     int I = det_in_sector(t, sec0, t.idx_a[ia], kb);
-    if (I >= 0) da = cscale(a.cic[I], (double)sg);
+    if (I >= 0) da = cscale(cic[I], (double)sg);
   }
   unsigned ib = excite_str(t.strb[kb], q, p, sg);
   if (ib != ~0u) {
     int I = det_in_sector(t, sec0, ka, t.idx_b[ib]);
-    if (I >= 0) db = cscale(a.cic[I], (double)sg);
+    if (I >= 0) db = cscale(cic[I], (double)sg);
   }
   a.Da[o + K] = da;
   a.Db[o + K] = db;
@@ -92,9 +93,10 @@ __global__ void __launch_bounds__(256) ci_den1_kernel(CiArgs a) {
   if (t.orb_m[x] != t.orb_m[y]) { if (threadIdx.x == 0) a.den1[x + n * y] = mkc(0, 0); return; }
   const int yx = y + n * x;
   const long o = t.dvec_off[yx];
+  const cplx* __restrict__ cic = a.io ? a.io->cic : a.cic;
   cplx s = mkc(0, 0);
   for (int J = threadIdx.x; J < t.lcic; J += blockDim.x) {
-    cplx c = a.cic[J];
+    cplx c = cic[J];
     cplx d = t.spin_sym ? cscale(a.Db[o + J], 2.0) : cadd(a.Da[o + J], a.Db[o + J]);
     s = cadd(s, cmulc(c, d));
   }
@@ -203,11 +205,11 @@ __global__ void __launch_bounds__(128) ci_sigma_kernel(CiArgs a) {
   for (int o = 16; o > 0; o >>= 1) { sig.x += __shfl_xor_sync(0xffffffff, sig.x, o); sig.y += __shfl_xor_sync(0xffffffff, sig.y, o); }
   if (lane != 0) return;
   const double e = *a.ene_act;
-  cplx c = a.cic[J];
+  cplx c = a.io ? a.io->cic[J] : a.cic[J];
   sig = csub(sig, cscale(c, e));
   cplx fac = a.icomp == 1 ? mkc(0.0, -a.dtime) : mkc(-a.dtime, 0.0);
   const cplx k = cmul(sig, fac);
-  if (a.rk.stage == 0) a.sigma[J] = k;
+  if (a.rk.stage == 0) (a.io ? a.io->hcic : a.sigma)[J] = k;
   else rk_put(a.rk, J, k);
 }
 

@@ -94,7 +94,9 @@ struct Etd4Bufs {
   cplx *w1 = nullptr, *w2 = nullptr, *w3 = nullptr, *h2 = nullptr, *h3 = nullptr, *tmp = nullptr;
   size_t cap = 0;
 };
+struct RhsGraph;  // the captured RHS (rhs_call)
 struct Ctx {
+  RhsGraph* rhs = nullptr;
   std::vector<void*> allocs;  // device allocations of this context
   RkBufs rk;                  // propagation buffers and cached step graphs
   Etd4Bufs e4;
@@ -713,7 +715,7 @@ __global__ void __launch_bounds__(512) dtorb_kernel(size_t nb, int nfun, int nfc
                                                     const int* __restrict__ mval, const cplx* orb, const cplx* __restrict__ h0,
                                                     const cplx* __restrict__ h1, const cplx* __restrict__ gg,
                                                     const cplx* __restrict__ v2, const cplx* __restrict__ xmat,
-                                                    cplx* __restrict__ hwfn, RkStage rk) {
+                                                    cplx* __restrict__ hwfn_arg, RkStage rk, const RhsIo* io, int no_ci) {
   __shared__ cplx so[16][32], sx[16 * 16];
   __shared__ int sm[16];
   const int i = threadIdx.x >> 5, lane = threadIdx.x & 31;  // blockDim = 32 nfun
@@ -731,6 +733,8 @@ __global__ void __launch_bounds__(512) dtorb_kernel(size_t nb, int nfun, int nfc
   }
   for (int e = threadIdx.x; e < nfun * nfun; e += blockDim.x) sx[e] = xmat[e];
   if (threadIdx.x < nfun) sm[threadIdx.x] = mval[threadIdx.x];
+  cplx* hwfn = io ? io->hwfn : hwfn_arg;
+  if (io && no_ci && blockIdx.x == 0 && threadIdx.x == 0) io->hcic[0] = mkc(0, 0);  // no active space: hcic = 0
   __syncthreads();
   if (!in) return;
   if (!dyn) {
@@ -744,6 +748,18 @@ __global__ void __launch_bounds__(512) dtorb_kernel(size_t nb, int nfun, int nfc
     if (sm[j] == mi) o = cadd(o, cmul(so[j][lane], sx[j + nfun * i]));
   if (rk.stage == 0) hwfn[t] = o;
   else rk_put(rk, t, o);
+}
+
+// lfield[9] (and the caller's buffers) by value into device memory
+struct Lf9 { double v[9]; };
+__global__ void lfield_kernel(Lf9 f, double* __restrict__ out, RhsIo io, RhsIo* io_out) {
+  if (threadIdx.x < 9) out[threadIdx.x] = f.v[threadIdx.x];
+  if (io_out && threadIdx.x == 9) *io_out = io;
+}
+// the dynamic orbitals of the caller's state into the context
+__global__ void orbin_kernel(const RhsIo* io, size_t n0, size_t n, cplx* __restrict__ orb) {
+  const size_t t = n0 + (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) orb[t] = io->wfn[t];
 }
 
 // ===========================================================================
@@ -1488,9 +1504,10 @@ int chk(const char* what, int rc) {
 }
 
 // d_lf: device lfield[9]; wfn/cic device inputs (wfn null: the orbitals already stand in c.orb);
-// hwfn/hcic device outputs, or (rk) the RK4 stage that takes the value of the orbitals and of the CI vector
+// hwfn/hcic device outputs, or (rk) the RK4 stage that takes the value of the orbitals and of the CI vector,
+// or (io) all four buffers as they stand in the device copy
 int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cplx* hwfn, cplx* hcic, double dtime,
-             const RkStage* rk = nullptr, const RkStage* rk_ci = nullptr) {
+             const RkStage* rk = nullptr, const RkStage* rk_ci = nullptr, const RhsIo* io = nullptr) {
   cudaStream_t st = c.st;
   const size_t so = c.nbas * c.nfun;
   int rc = 0;
@@ -1508,6 +1525,7 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
   ca.t = c.cit; ca.cic = cic_in; ca.Da = c.Da; ca.Db = c.Db; ca.T = c.T; ca.den1 = c.den1; ca.den2 = c.den2;
   ca.sigma = hcic; ca.int1e = c.int1e; ca.int2e = c.int2e; ca.ene_act = c.ene + 3; ca.dtime = dtime; ca.icomp = c.icomp;
   if (rk_ci) ca.rk = *rk_ci;
+  ca.io = io;
   // The RDM chain reads only the CI vector, and its first consumer is
   // mfprod: it runs on the side stream, concurrently with the orbital
   // transform, the one-body stencil, the pair densities, the Poisson solve
@@ -1527,7 +1545,11 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
   }
   auto join = [&]() { if (fork) cudaStreamWaitEvent(st, c.ev_join, 0); };
   // orbitals (hprod_orbin.F90)
-  if (wfn)
+  if (io) {
+    const size_t n0 = c.nfcore * c.nbas;
+    orbin_kernel<<<(unsigned)((so - n0 + 255) / 256), 256, 0, st>>>(io, n0, so, c.orb);
+    c.launches++;
+  } else if (wfn)
     cudaMemcpyAsync(c.orb + c.nfcore * c.nbas, wfn + c.nfcore * c.nbas, (so - c.nfcore * c.nbas) * sizeof(cplx),
                     cudaMemcpyDeviceToDevice, st);
   if (c.n_orbg) rc |= chk("orbg gemm", gemm(c, c.b_orbg, c.n_orbg, c.nlat, c.L1, false));
@@ -1635,20 +1657,90 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
     rc |= chk("ci sigma", launch_ci_sigma(ca, c.st2));
     cudaEventRecord(c.ev_sig_join, c.st2);
     c.launches += 1;
-  } else if (!rk_ci) {
+  } else if (!rk_ci && !io) {
     cudaMemsetAsync(hcic, 0, sizeof(cplx), st);
   }
   mark();  // end ci_sigma (the sigma itself overlaps dtorb)
   // dtorb
   dtorb_kernel<<<(unsigned)((c.nbas + 31) / 32), 32 * c.nfun, 0, st>>>(
       c.nbas, c.nfun, c.nfcore, c.icomp, c.isplit, dtime, c.d_mval, c.orb, c.h0orb, c.h1orb, c.gorb, c.v2orb, c.xmat, hwfn,
-      rk ? *rk : RkStage{});
+      rk ? *rk : RkStage{}, io, c.nact == 0);
   c.launches++;
   if (c.nact > 0) cudaStreamWaitEvent(st, c.ev_sig_join, 0);
   mark();  // end dtorb (and sigma)
   c.nev = iev;
   rc |= chk("rhs tail", (int)cudaGetLastError());
   return rc;
+}
+
+// One RHS on the caller's device buffers.  An eager RHS is some twenty launches and events on three
+// streams, more host time than the small workloads' kernels take; the second call in a row with the same
+// settings captures it once (reading the buffers and the field from device memory, so the capture holds
+// for any buffers), and later calls replay it.  The capture goes with the context, or when a setting changes.
+struct RhsKey {
+  double dtime = 0, ene_fcore = 0;
+  int set[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  bool operator==(const RhsKey& k) const { return memcmp(this, &k, sizeof(RhsKey)) == 0; }
+};
+struct RhsGraph {
+  cudaGraphExec_t exec = nullptr;
+  RhsIo* io = nullptr;
+  RhsKey key, last;
+  bool have_last = false;
+  long launches = 0;
+};
+int rhs_call(Ctx& c, RhsGraph& g, const double* lf, const RhsIo& io, double dtime) {
+  if (!g.io) g.io = dalloc<RhsIo>(1);
+  Lf9 f;
+  for (int k = 0; k < 9; ++k) f.v[k] = lf[k];
+  lfield_kernel<<<1, 32, 0, c.st>>>(f, c.lfield, io, g.io);
+  c.launches++;
+  RhsKey key;
+  memset(&key, 0, sizeof(key));
+  key.dtime = dtime; key.ene_fcore = c.ene_fcore;
+  const int set[8] = {c.icomp, c.igauge, c.isplit, c.mixed, c.mf_external, c.tune_mt, c.tune_mf_cap, c.tune_i2_split};
+  memcpy(key.set, set, sizeof(set));
+  cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(c.st, &cst);
+  auto eager = [&]() { return run_htot(c, c.lfield, io.wfn, io.cic, io.hwfn, io.hcic, dtime); };
+  if (cst != cudaStreamCaptureStatusNone || c.profile) return eager();
+  if (g.exec && !(g.key == key)) {
+    cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
+  }
+  if (!g.exec) {
+    const bool again = g.have_last && g.last == key;
+    g.last = key;
+    g.have_last = true;
+    if (!again) return eager();
+    const long l0 = c.launches;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamBeginCapture(c.st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return ST_CUDA;
+    const int rc = run_htot(c, c.lfield, nullptr, nullptr, nullptr, nullptr, dtime, nullptr, nullptr, g.io);
+    const cudaError_t e = cudaStreamEndCapture(c.st, &graph);
+    g.launches = c.launches - l0;
+    c.launches = l0;
+    if (!rc && e == cudaSuccess && cudaGraphInstantiate(&g.exec, graph, cudaGraphInstantiateFlagUseNodePriority) != cudaSuccess)
+      g.exec = nullptr;
+    if (graph) cudaGraphDestroy(graph);
+    if (rc || !g.exec) {  // no memory for the graph, say: the eager RHS needs none
+      cudaGetLastError();
+      g.have_last = false;
+      return eager();
+    }
+    g.key = key;
+  }
+  c.launches += g.launches;
+  return cudaGraphLaunch(g.exec, c.st) == cudaSuccess ? 0 : ST_CUDA;
+}
+int rhs_call(Ctx& c, const double* lf, const cplx* wfn, const cplx* cic, cplx* hwfn, cplx* hcic, double dtime) {
+  if (!c.rhs) c.rhs = new RhsGraph();
+  return rhs_call(c, *c.rhs, lf, RhsIo{wfn, cic, hwfn, hcic}, dtime);
+}
+void rhs_free(Ctx& c) {
+  if (c.rhs && c.rhs->exec) cudaGraphExecDestroy(c.rhs->exec);
+  delete c.rhs;
+  c.rhs = nullptr;
 }
 
 // ===========================================================================
@@ -2822,6 +2914,9 @@ void hprod_init_(void) {
     make_stream(&c.st, true); make_stream(&c.st2, false); make_stream(&c.st3, false); make_stream(&c.st4, true);
     c.own_streams = true;
   }
+  // a second init of a context: what was captured over the old buffers goes
+  if (c.st) cudaStreamSynchronize(c.st);
+  rhs_free(c);
   for (cudaEvent_t* e : {&c.ev_fork, &c.ev_join, &c.ev_ob_fork, &c.ev_ob_join, &c.ev_i2_fork, &c.ev_i2_join,
                          &c.ev_sig_fork, &c.ev_sig_join})
     cudaEventCreateWithFlags(e, cudaEventDisableTiming);
@@ -2900,7 +2995,7 @@ void hprod_htot_(const double* dtime, const double* lfield, const double* wfn, c
   cudaMemcpyAsync(c.lfield, lfield, 9 * sizeof(double), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(c.wfn_io, wfn, so * sizeof(cplx), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(c.cic_io, cic, c.lcic * sizeof(cplx), cudaMemcpyHostToDevice, st);
-  int rc = run_htot(c, c.lfield, c.wfn_io, c.cic_io, c.hwfn_io, c.hcic_io, *dtime);
+  int rc = rhs_call(c, lfield, c.wfn_io, c.cic_io, c.hwfn_io, c.hcic_io, *dtime);
   // the reference stops on a failed solve (hprod_mkv2mf.F90:167-170); here a
   // non-finite output (a NaN in the input, a diverged state) is reported in
   // the status word instead
@@ -2928,6 +3023,7 @@ void hprod_final_(void) {
   for (auto& ge : c.graph_exec) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
   for (auto& ge : c.lp_exec) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
   if (c.st) cudaStreamSynchronize(c.st);
+  rhs_free(c);
   if (c.st2) cudaStreamSynchronize(c.st2);
   if (c.st3) cudaStreamSynchronize(c.st3);
   for (cudaEvent_t e : {c.ev_fork, c.ev_join, c.ev_ob_fork, c.ev_ob_join, c.ev_i2_fork, c.ev_i2_join, c.ev_sig_fork,
@@ -2974,8 +3070,7 @@ int td1c_gpu_energies(double* e) {
 int td1c_gpu_htot_dev(double dtime, const double* lfield, const void* d_wfn, const void* d_cic, void* d_hwfn, void* d_hcic) {
   Ctx& c = ctx();
   if (!c.initialized) return ST_CONFIG;
-  cudaMemcpyAsync(c.lfield, lfield, 9 * sizeof(double), cudaMemcpyHostToDevice, c.st);
-  int rc = run_htot(c, c.lfield, (const cplx*)d_wfn, (const cplx*)d_cic, (cplx*)d_hwfn, (cplx*)d_hcic, dtime);
+  int rc = rhs_call(c, lfield, (const cplx*)d_wfn, (const cplx*)d_cic, (cplx*)d_hwfn, (cplx*)d_hcic, dtime);
   return rc ? ST_CUDA : 0;
 }
 
@@ -3200,10 +3295,9 @@ int td1c_gpu_relax(void* d_wfn, void* d_cic, double dt, int ncyc, double* ene) {
   double* d_trace = nullptr;
   if (cudaMalloc(&d_trace, sizeof(double) * std::max(1, ncyc)) != cudaSuccess) return ST_CUDA;
   const double lf0[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  cudaMemcpyAsync(c.lfield, lf0, 9 * sizeof(double), cudaMemcpyHostToDevice, st);
   int rc = 0;
   for (int s = 0; s < ncyc && !rc; ++s) {
-    rc |= run_htot(c, c.lfield, (const cplx*)d_wfn, (const cplx*)d_cic, c.relax_hw, c.relax_hc, 1.0);
+    rc |= rhs_call(c, lf0, (const cplx*)d_wfn, (const cplx*)d_cic, c.relax_hw, c.relax_hc, 1.0);
     cudaMemcpyAsync(d_trace + s, c.ene + 4, sizeof(double), cudaMemcpyDeviceToDevice, st);
     rc |= td1c_gpu_rk4(d_wfn, d_cic, 0.0, dt, 1, 0.0, 800.0, 1.0, 0.0, 1);
     rc |= launch_orth(c.Nr, c.L1, c.nfun, c.nfcore, c.lcic, c.d_mval, (cplx*)d_wfn, (cplx*)d_cic, st);
@@ -3278,8 +3372,7 @@ int td1c_gpu_relax_etdrk2(void* d_wfn, void* d_cic, double dt, int ncyc, int max
   const double lf0[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   int rc = 0;
   for (int s = 0; s < ncyc && !rc; ++s) {
-    cudaMemcpyAsync(c.lfield, lf0, 9 * sizeof(double), cudaMemcpyHostToDevice, st);
-    rc |= run_htot(c, c.lfield, (const cplx*)d_wfn, (const cplx*)d_cic, c.relax_hw, c.relax_hc, 1.0);
+    rc |= rhs_call(c, lf0, (const cplx*)d_wfn, (const cplx*)d_cic, c.relax_hw, c.relax_hc, 1.0);
     cudaMemcpyAsync(d_trace + s, c.ene + 4, sizeof(double), cudaMemcpyDeviceToDevice, st);
     rc |= prop_run(2, d_wfn, d_cic, 0.0, dt, 1, 0.0, 800.0, 1.0, 0.0, maxcyc, thresh, 1, false);
     rc |= launch_orth(c.Nr, c.L1, c.nfun, c.nfcore, c.lcic, c.d_mval, (cplx*)d_wfn, (cplx*)d_cic, st);

@@ -17,6 +17,13 @@
 
 namespace td1c {
 
+// The caller's buffers of one RHS, in device memory: a captured RHS reads them from here, so one capture
+// serves any buffers (the field stands in the context's lfield)
+struct RhsIo {
+  const cplx *wfn, *cic;
+  cplx *hwfn, *hcic;
+};
+
 // What an RHS does with its value k: writes it out (stage 0), or makes it stage 1 .. 4 of an RK4 step
 // (clcrk::prop, src/prop/clcrk.cpp:55-87; tableau set_coeff_04 221-235): acc = or += wt k, the next stage's
 // state y + an k, and after stage 4 y += acc.  y is the state at the step's start until then.
@@ -324,6 +331,7 @@ struct CiArgs {
   const double* ene_act;  // device scalar
   double dtime; int icomp;
   RkStage rk;             // stage > 0: sigma goes into an RK4 stage of the CI vector instead of out
+  const RhsIo* io = nullptr;  // non-null: the CI vector and sigma are its buffers
 };
 int launch_ci_dvec(const CiArgs& a, int maxsec, cudaStream_t st);
 int launch_ci_rdm(const CiArgs& a, cudaStream_t st);

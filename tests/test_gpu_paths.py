@@ -123,3 +123,40 @@ def test_correction_cycle_limits(cuda_ok, maxcyc, thresh):
             assert rel_err(x.cpu().numpy(), wo) < TOL and rel_err(c.cpu().numpy(), co) < TOL
     finally:
         h.final()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("wl", [W.HE_SMALL, W.NE_SMALL, W.LENGTH_SMALL], ids=lambda w: w["name"])
+def test_rhs_replay(cuda_ok, wl):
+    """The captured RHS on other buffers, other fields, and after changes of a setting: bitwise the eager one."""
+    import torch
+    o, h, orb, cic = _pair(wl)
+    try:
+        def call(x, c, lf, dt=1.0):
+            y, yc = torch.full_like(x, float("nan")), torch.full_like(c, float("nan"))
+            torch.cuda.synchronize()
+            h.htot_dev(dt, lf, x.data_ptr(), c.data_ptr(), y.data_ptr(), yc.data_ptr())
+            h.sync()
+            return y.cpu().numpy(), yc.cpu().numpy()
+        xs = [torch.from_numpy((orb * s).reshape(-1).copy()).cuda() for s in (1.0, 0.5)]
+        cs = [torch.from_numpy(cic.copy()).cuda() for _ in xs]
+        lfs = [_field(wl), 0.5 * _field(wl)]
+        split = wl.get("split_type", 0)
+        first = {}
+        for k in range(2):  # alternating settings never repeat, so these are eager
+            for sp in (1, split):
+                h.set_split(sp)
+                first[k, sp] = call(xs[k], cs[k], lfs[k])
+        for sp in (1, split, 2):
+            h.set_split(sp)
+            for rep in range(4):
+                got = call(xs[rep % 2], cs[rep % 2], lfs[rep % 2])
+                if sp != 2:
+                    for a, b in zip(got, first[rep % 2, sp]):
+                        assert np.array_equal(a, b)
+        h.set_split(split)
+        for dt in (0.25, 0.25, 0.25, 1.0, 1.0, 1.0):
+            a = call(xs[0], cs[0], lfs[0], dt)[0]
+            assert rel_err(a, dt * first[0, split][0]) < 1e-14
+    finally:
+        h.final()
