@@ -190,6 +190,8 @@ struct Ctx {
   int4* dip_rd_ent = nullptr;
   int dip_rd_n = 0;
   std::vector<int> dip_ia, dip_ib, dip_if, dip_isz, dip_isp;
+  double* relax_trace = nullptr;  // energies of the cycles of a relaxation call
+  int relax_cap = 0;
   cplx *relax_hw = nullptr, *relax_hc = nullptr;  // RHS outputs of the energy evaluation in td1c_gpu_relax
   // one-body propagators: condensed factors of 1 + c T per c, and scratch
   struct H1Slot { double cre = 0, cim = 0; H1Fac f; };
@@ -3282,6 +3284,15 @@ int td1c_gpu_orth(void* d_wfn, void* d_cic) {
 int td1c_gpu_rk4(void* d_wfn, void* d_cic, double t0, double dt, int nstep, double fint, double wlen, double numcyc,
                  double cep, int use_graph);
 
+// the energy trace of a relaxation call, kept with the context and grown when a call needs more
+static double* relax_trace(Ctx& c, int ncyc) {
+  if (ncyc > c.relax_cap || !c.relax_trace) {
+    c.relax_cap = std::max(1024, ncyc);
+    c.relax_trace = dalloc<double>(c.relax_cap);
+  }
+  return c.relax_trace;
+}
+
 // imaginary-time relaxation in the form of init_prop12 (init.cpp:250-319):
 // per cycle the total energy of the current state (ene[s], host), one
 // zero-field RK4 step of dt (wfn_mask included) and wfn_orth; needs a
@@ -3292,8 +3303,8 @@ int td1c_gpu_relax(void* d_wfn, void* d_cic, double dt, int ncyc, double* ene) {
   cudaStream_t st = c.st;
   const size_t so = c.nbas * c.nfun;
   if (!c.relax_hw) { c.relax_hw = dalloc<cplx>(so); c.relax_hc = dalloc<cplx>(std::max(1, c.lcic)); }
-  double* d_trace = nullptr;
-  if (cudaMalloc(&d_trace, sizeof(double) * std::max(1, ncyc)) != cudaSuccess) return ST_CUDA;
+  double* d_trace = relax_trace(c, ncyc);
+  if (!d_trace) return ST_CUDA;
   const double lf0[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   int rc = 0;
   for (int s = 0; s < ncyc && !rc; ++s) {
@@ -3304,7 +3315,6 @@ int td1c_gpu_relax(void* d_wfn, void* d_cic, double dt, int ncyc, double* ene) {
   }
   if (ene && ncyc > 0) cudaMemcpyAsync(ene, d_trace, ncyc * sizeof(double), cudaMemcpyDeviceToHost, st);
   cudaError_t e = cudaStreamSynchronize(st);
-  cudaFree(d_trace);
   int dst = 0;
   cudaMemcpy(&dst, c.d_status, sizeof(int), cudaMemcpyDeviceToHost);
   return (rc || e != cudaSuccess) ? ST_CUDA : dst;
@@ -3367,8 +3377,8 @@ int td1c_gpu_relax_etdrk2(void* d_wfn, void* d_cic, double dt, int ncyc, int max
   cudaStream_t st = c.st;
   const size_t so = c.nbas * c.nfun;
   if (!c.relax_hw) { c.relax_hw = dalloc<cplx>(so); c.relax_hc = dalloc<cplx>(std::max(1, c.lcic)); }
-  double* d_trace = nullptr;
-  if (cudaMalloc(&d_trace, sizeof(double) * std::max(1, ncyc)) != cudaSuccess) return ST_CUDA;
+  double* d_trace = relax_trace(c, ncyc);
+  if (!d_trace) return ST_CUDA;
   const double lf0[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   int rc = 0;
   for (int s = 0; s < ncyc && !rc; ++s) {
@@ -3379,7 +3389,6 @@ int td1c_gpu_relax_etdrk2(void* d_wfn, void* d_cic, double dt, int ncyc, int max
   }
   if (ene && ncyc > 0) cudaMemcpyAsync(ene, d_trace, ncyc * sizeof(double), cudaMemcpyDeviceToHost, st);
   cudaError_t e = cudaStreamSynchronize(st);
-  cudaFree(d_trace);
   int dst = 0;
   cudaMemcpy(&dst, c.d_status, sizeof(int), cudaMemcpyDeviceToHost);
   return (rc || e != cudaSuccess) ? ST_CUDA : dst;

@@ -92,54 +92,78 @@ int dipole_partial_size(int Nr, int nent) { return ((Nr + DIP_CHUNK - 1) / DIP_C
 // ecs_flag = 0): normalise the CI vector; then modified Gram-Schmidt of every
 // non-frozen orbital against all earlier orbitals of equal m (each overlap
 // with the already projected orbital), then normalisation, over l >= |m|.
-// One CTA; every sum is a fixed-order block reduction.
+// One cluster of 8 CTAs, each with its slice of every orbital; a sum is a block
+// reduction per CTA and then, in rank order, over the cluster's distributed
+// shared memory (two slots in turn, so one cluster barrier per sum is enough).
+// The chain of dependent sums is what bounds it: one CTA alone streamed each
+// orbital pair through a single SM (Ne's 25 sums took 10 times longer).
 // ---------------------------------------------------------------------------
-constexpr int ORTH_NT = 1024;
+constexpr int ORTH_NT = 1024, ORTH_CTAS = 8;
 
-__device__ cplx orth_block_sum(cplx v, cplx* red) {
+struct OrthSum {
+  cplx warp[ORTH_NT / 32];
+  cplx slot[2];
+};
+__device__ __forceinline__ cplx orth_sum(cplx v, OrthSum& s, int& turn) {
   const int tid = threadIdx.x;
-  red[tid] = v;
+  for (int o = 16; o > 0; o >>= 1) { v.x += __shfl_xor_sync(0xffffffffu, v.x, o); v.y += __shfl_xor_sync(0xffffffffu, v.y, o); }
+  if ((tid & 31) == 0) s.warp[tid >> 5] = v;
   __syncthreads();
-  for (int st = ORTH_NT / 2; st > 0; st >>= 1) {
-    if (tid < st) red[tid] = cadd(red[tid], red[tid + st]);
-    __syncthreads();
+  if (tid < 32) {
+    cplx w = s.warp[tid];
+    for (int o = 16; o > 0; o >>= 1) { w.x += __shfl_xor_sync(0xffffffffu, w.x, o); w.y += __shfl_xor_sync(0xffffffffu, w.y, o); }
+    if (tid == 0) s.slot[turn] = w;
   }
-  const cplx r = red[0];
-  __syncthreads();
-  return r;
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+  const unsigned mine = (unsigned)__cvta_generic_to_shared(&s.slot[turn]);
+  cplx t = mkc(0, 0);
+#pragma unroll
+  for (int r = 0; r < ORTH_CTAS; ++r) {
+    unsigned at;
+    cplx w;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(mine), "r"(r));
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(w.x), "=d"(w.y) : "r"(at) : "memory");
+    t = cadd(t, w);
+  }
+  turn ^= 1;
+  return t;
 }
 
-__global__ void __launch_bounds__(ORTH_NT) orth_kernel(int Nr, int L1, int nfun, int nfcore, int lcic,
-                                                       const int* __restrict__ mval, cplx* wfn, cplx* cic) {
-  __shared__ cplx red[ORTH_NT];
-  const int tid = threadIdx.x;
+__global__ void __cluster_dims__(ORTH_CTAS, 1, 1) __launch_bounds__(ORTH_NT)
+    orth_kernel(int Nr, int L1, int nfun, int nfcore, int lcic, const int* __restrict__ mval, cplx* wfn, cplx* cic) {
+  __shared__ OrthSum sum;
+  int turn = 0;
+  const int t0 = blockIdx.x * ORTH_NT + threadIdx.x, step = ORTH_CTAS * ORTH_NT;  // a thread's elements are its own throughout
   cplx s = mkc(0, 0);
-  for (int d = tid; d < lcic; d += ORTH_NT) s.x += cabs2(cic[d]);
-  const double cn = 1.0 / sqrt(orth_block_sum(s, red).x);
-  for (int d = tid; d < lcic; d += ORTH_NT) cic[d] = cscale(cic[d], cn);
+  for (int d = t0; d < lcic; d += step) s.x += cabs2(cic[d]);
+  const double cn = 1.0 / sqrt(orth_sum(s, sum, turn).x);
+  for (int d = t0; d < lcic; d += step) cic[d] = cscale(cic[d], cn);
   for (int i = nfcore; i < nfun; ++i) {
     const int mi = mval[i], l0 = mi < 0 ? -mi : mi;
-    cplx* pi = wfn + (size_t)i * L1 * Nr;
     const int n = (L1 - l0) * Nr;  // the l >= |m| rows are contiguous
+    cplx* pi = wfn + ((size_t)i * L1 + l0) * Nr;
     for (int j = 0; j < i; ++j) {
       if (mval[j] != mi) continue;
-      const cplx* pj = wfn + (size_t)j * L1 * Nr;
+      const cplx* pj = wfn + ((size_t)j * L1 + l0) * Nr;
       cplx ov = mkc(0, 0);
-      for (int e = tid; e < n; e += ORTH_NT) ov = cadd(ov, cmulc(pj[(size_t)l0 * Nr + e], pi[(size_t)l0 * Nr + e]));
-      ov = orth_block_sum(ov, red);
-      for (int e = tid; e < n; e += ORTH_NT) pi[(size_t)l0 * Nr + e] = csub(pi[(size_t)l0 * Nr + e], cmul(pj[(size_t)l0 * Nr + e], ov));
-      __syncthreads();
+#pragma unroll 4
+      for (int e = t0; e < n; e += step) ov = cadd(ov, cmulc(pj[e], pi[e]));
+      ov = orth_sum(ov, sum, turn);
+#pragma unroll 4
+      for (int e = t0; e < n; e += step) pi[e] = csub(pi[e], cmul(pj[e], ov));
     }
     cplx nr = mkc(0, 0);
-    for (int e = tid; e < n; e += ORTH_NT) nr.x += cabs2(pi[(size_t)l0 * Nr + e]);
-    const double inv = 1.0 / sqrt(orth_block_sum(nr, red).x);
-    for (int e = tid; e < n; e += ORTH_NT) pi[(size_t)l0 * Nr + e] = cscale(pi[(size_t)l0 * Nr + e], inv);
-    __syncthreads();
+#pragma unroll 4
+    for (int e = t0; e < n; e += step) nr.x += cabs2(pi[e]);
+    const double inv = 1.0 / sqrt(orth_sum(nr, sum, turn).x);
+    for (int e = t0; e < n; e += step) pi[e] = cscale(pi[e], inv);
   }
+  // no CTA leaves while another may still read its slot
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
 
 int launch_orth(int Nr, int L1, int nfun, int nfcore, int lcic, const int* mval, cplx* wfn, cplx* cic, cudaStream_t st) {
-  orth_kernel<<<1, ORTH_NT, 0, st>>>(Nr, L1, nfun, nfcore, lcic, mval, wfn, cic);
+  orth_kernel<<<ORTH_CTAS, ORTH_NT, 0, st>>>(Nr, L1, nfun, nfcore, lcic, mval, wfn, cic);
   return (int)cudaGetLastError();
 }
 
