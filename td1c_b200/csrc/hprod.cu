@@ -95,7 +95,10 @@ struct Etd4Bufs {
   size_t cap = 0;
 };
 struct RhsGraph;  // the captured RHS (rhs_call)
+unsigned long g_epoch = 0;
 struct Ctx {
+  unsigned long epoch = ++g_epoch;  // renewed by every change of what a captured step was built from
+  cplx* ens_y = nullptr;  // this job's state inside an ensemble call (orbitals, then CI)
   RhsGraph* rhs = nullptr;
   std::vector<void*> allocs;  // device allocations of this context
   RkBufs rk;                  // propagation buffers and cached step graphs
@@ -1906,6 +1909,7 @@ int h1_factor(Ctx& c, cplx fac, H1Fac* out) {
     sl = &c.h1slot[Ctx::kH1Slots - 1];
   }
   sl->cre = fac.x; sl->cim = fac.y;
+  c.epoch = ++g_epoch;  // captured steps may hold the slot's factors
   H1FacSrc src{};
   src.Nr = c.Nr; src.L1 = c.L1; src.nd = c.nd; src.nfe = c.nfe; src.c = fac;
   src.radk = c.radk; src.radk0 = c.radk0; src.tdiag = c.tdiag; src.status = c.d_status;
@@ -2878,12 +2882,14 @@ int td1c_gpu_bind_ormas(int nsub) {
 int td1c_gpu_bind_control(int icomp, int igauge) {
   Ctx& c = ctx();
   c.icomp = icomp; c.igauge = igauge;
+  ctx().epoch = ++g_epoch;
   return 0;
 }
 
 int td1c_gpu_bind_split(int split_type) {
   if (split_type < 0 || split_type > 2) return ST_CONFIG;
   ctx().isplit = split_type;
+  ctx().epoch = ++g_epoch;
   return 0;
 }
 
@@ -2919,6 +2925,7 @@ void hprod_init_(void) {
   // a second init of a context: what was captured over the old buffers goes
   if (c.st) cudaStreamSynchronize(c.st);
   rhs_free(c);
+  c.epoch = ++g_epoch;
   for (cudaEvent_t* e : {&c.ev_fork, &c.ev_join, &c.ev_ob_fork, &c.ev_ob_join, &c.ev_i2_fork, &c.ev_i2_join,
                          &c.ev_sig_fork, &c.ev_sig_join})
     cudaEventCreateWithFlags(e, cudaEventDisableTiming);
@@ -2936,6 +2943,7 @@ void hprod_init_(void) {
 
 void hprod_set_wfn0_(const double* wfn, const double* cic, const char* v2xfc_type, int len) {
   Ctx& c = ctx();
+  c.epoch = ++g_epoch;
   (void)cic; (void)v2xfc_type; (void)len;
   if (!c.initialized) { c.status |= ST_CONFIG; return; }
   cudaStream_t st = c.st;
@@ -3019,9 +3027,11 @@ void hprod_htot_(const double* dtime, const double* lfield, const double* wfn, c
   if (c.p_ene_tot) *c.p_ene_tot = c.h_ene[4];
 }
 
+static void ens_forget(int id);
 void hprod_final_(void) {
   if (!g) return;
   Ctx& c = *g;
+  ens_forget(g_cur);
   for (auto& ge : c.graph_exec) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
   for (auto& ge : c.lp_exec) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
   if (c.st) cudaStreamSynchronize(c.st);
@@ -3489,6 +3499,7 @@ int td1c_gpu_set_mixed(int on) {
   if (on < 0 || on > 3) return ST_CONFIG;
   c.mixed = on;
   if (c.mixed) build_tc_plans(c);
+  ctx().epoch = ++g_epoch;
   return 0;
 }
 
@@ -3698,6 +3709,7 @@ int td1c_gpu_ctx_destroy(int id) {
 
 int td1c_gpu_set_tuning(int mt, int mf_cap, int i2_split_) {
   Ctx& c = ctx();
+  c.epoch = ++g_epoch;
   if ((mt != 0 && mt != 3 && mt != 6) || mf_cap < 0) return ST_CONFIG;
   c.tune_mt = mt; c.tune_mf_cap = mf_cap; c.tune_i2_split = i2_split_;
   for (auto& ge : c.graph_exec) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }  // recaptured with the new shapes
@@ -3715,7 +3727,45 @@ int td1c_gpu_get_tuning(int* out4) {
 // nstep split2 steps of every job of an ensemble in one CUDA graph per step:
 // the step of job j is captured on job j's own streams, forked from one
 // stream and joined back, so the jobs' kernels have no order between them and
-// the GPU runs them side by side.  *ms = device time of the nstep replays.
+// the GPU runs them side by side.  The step works on a state buffer of each
+// context (the callers' states are copied in and out), so its graph holds for
+// any state buffers and is kept: up to EnsPlans of them, the least recently
+// used one makes room, and a plan goes with any of its contexts.  Capturing and
+// instantiating a small ensemble's step takes longer than its steps.
+// *ms = device time of the nstep replays.
+struct EnsPlan {
+  std::vector<int> ids;
+  std::vector<unsigned long> epoch;
+  std::vector<double> dt;
+  std::vector<const void*> tab;
+  int maxcyc = 0;
+  double thresh = 0;
+  std::vector<cudaGraphExec_t> exec;  // of each job
+  unsigned long used = 0;
+  void destroy() {
+    for (cudaGraphExec_t e : exec) cudaGraphExecDestroy(e);
+    exec.clear();
+  }
+  bool same(const EnsPlan& k) const {
+    return ids == k.ids && epoch == k.epoch && dt == k.dt && tab == k.tab && maxcyc == k.maxcyc && thresh == k.thresh;
+  }
+};
+static constexpr size_t kEnsPlans = 8;
+static std::vector<EnsPlan>& ens_plans() {
+  static std::vector<EnsPlan> p;
+  return p;
+}
+static void ens_forget(int id) {  // context id ends: its plans go
+  auto& P = ens_plans();
+  for (size_t k = 0; k < P.size();)
+    if (std::find(P[k].ids.begin(), P[k].ids.end(), id) != P[k].ids.end()) {
+      P[k].destroy();
+      P.erase(P.begin() + k);
+    } else {
+      ++k;
+    }
+}
+
 int td1c_gpu_ensemble_split2(int njob, const int* ids, void* const* d_wfn, void* const* d_cic, const double* t0,
                              const double* dt, int nstep, const double* fint, const double* wlen, const double* numcyc,
                              const double* cep, int maxcyc, double thresh, double* ms) {
@@ -3724,6 +3774,7 @@ int td1c_gpu_ensemble_split2(int njob, const int* ids, void* const* d_wfn, void*
   const int keep = g_cur;
   static cudaStream_t master = nullptr;
   static std::vector<cudaEvent_t> evs;
+  static unsigned long clock = 0;
   if (!master) make_stream(&master, true);
   while ((int)evs.size() < 2 * njob + 2) {
     cudaEvent_t e;
@@ -3731,7 +3782,10 @@ int td1c_gpu_ensemble_split2(int njob, const int* ids, void* const* d_wfn, void*
     evs.push_back(e);
   }
   int rc = 0;
-  // per job: the field table, buffers and first-call set-up (outside any capture)
+  EnsPlan key;
+  key.maxcyc = maxcyc;
+  key.thresh = thresh;
+  // per job: the field table, buffers and the state
   for (int j = 0; j < njob && !rc; ++j) {
     if (td1c_gpu_ctx_select(ids[j]) || !g || !g->initialized || g->isplit != 1) { rc = ST_CONFIG; break; }
     Ctx& c = *g;
@@ -3742,6 +3796,7 @@ int td1c_gpu_ensemble_split2(int njob, const int* ids, void* const* d_wfn, void*
       if (!b.lf_cur) { b.lf_cur = dalloc<double>(54); b.counter = dalloc<int>(2); }
       b.cap = no + nc;
     }
+    if (!c.ens_y) c.ens_y = dalloc<cplx>(no + nc);
     b.reset_orb = nullptr; b.reset_cic = nullptr;
     Pulse pl;
     pl.famp = std::sqrt(fint[j] / 3.50944506E+16); pl.freq = 1239.84190 / (wlen[j] * 27.2113845);
@@ -3758,47 +3813,92 @@ int td1c_gpu_ensemble_split2(int njob, const int* ids, void* const* d_wfn, void*
     cudaMemcpyAsync(c.field_tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, c.st);
     b.h_counter[0] = 0; b.h_counter[1] = nstep;
     cudaMemcpyAsync(b.counter, b.h_counter, 2 * sizeof(int), cudaMemcpyHostToDevice, c.st);
-    // warm-up on a copy of the state: the one-body factors, scratch and kernel attributes
-    cudaMemcpyAsync(b.yt, d_wfn[j], no * sizeof(cplx), cudaMemcpyDeviceToDevice, c.st);
-    cudaMemcpyAsync(b.yt + no, d_cic[j], nc * sizeof(cplx), cudaMemcpyDeviceToDevice, c.st);
-    cudaMemcpyAsync(c.lfield, tab.data(), 9 * sizeof(double), cudaMemcpyHostToDevice, c.st);
-    rc |= h1_apply(c, false, c.lfield, b.yt, 0.5 * dt[j], mkc(0, 0), maxcyc, thresh);
-    rc |= run_htot(c, c.lfield, b.yt, b.yt + no, b.k, b.k + no, 1.0);
-    if (cudaStreamSynchronize(c.st) != cudaSuccess) rc |= ST_CUDA;
+    cudaMemcpyAsync(c.ens_y, d_wfn[j], no * sizeof(cplx), cudaMemcpyDeviceToDevice, c.st);
+    cudaMemcpyAsync(c.ens_y + no, d_cic[j], nc * sizeof(cplx), cudaMemcpyDeviceToDevice, c.st);
+    key.ids.push_back(ids[j]);
+    key.dt.push_back(dt[j]);
+    key.tab.push_back(c.field_tab);
+    key.epoch.push_back(c.epoch);
   }
-  cudaGraphExec_t exec = nullptr;
-  if (!rc && nstep > 0) {
-    cudaGraph_t graph = nullptr;
-    if (cudaStreamBeginCapture(master, cudaStreamCaptureModeThreadLocal) != cudaSuccess) rc = ST_CUDA;
+  EnsPlan* plan = nullptr;
+  for (EnsPlan& q : ens_plans())
+    if (!rc && q.same(key)) plan = &q;
+  if (!rc && nstep > 0 && !plan) {
+    // warm-up on a copy of each state: the one-body factors, scratch and kernel attributes (outside the capture)
+    for (int j = 0; j < njob; ++j) {
+      td1c_gpu_ctx_select(ids[j]);
+      Ctx& c = *g;
+      const size_t no = c.nbas * c.nfun, nc = c.lcic;
+      RkBufs& b = c.rk;
+      cudaMemcpyAsync(b.yt, c.ens_y, (no + nc) * sizeof(cplx), cudaMemcpyDeviceToDevice, c.st);
+      cudaMemcpyAsync(c.lfield, c.field_tab, 9 * sizeof(double), cudaMemcpyDeviceToDevice, c.st);
+      rc |= h1_apply(c, false, c.lfield, b.yt, 0.5 * dt[j], mkc(0, 0), std::min(maxcyc, 1), thresh);
+      rc |= run_htot(c, c.lfield, b.yt, b.yt + no, b.k, b.k + no, 1.0);
+      if (cudaStreamSynchronize(c.st) != cudaSuccess) rc |= ST_CUDA;
+      key.epoch[j] = c.epoch;
+    }
     for (int j = 0; j < njob && !rc; ++j) {
       td1c_gpu_ctx_select(ids[j]);
       Ctx& c = *g;
-      cudaEventRecord(evs[2 * j], master);
-      cudaStreamWaitEvent(c.st, evs[2 * j], 0);
-      rc |= split2_step(c, (cplx*)d_wfn[j], (cplx*)d_cic[j], dt[j], maxcyc, thresh, true);
-      cudaEventRecord(evs[2 * j + 1], c.st);
+      cudaGraph_t graph = nullptr;
+      cudaGraphExec_t exec = nullptr;
+      if (cudaStreamBeginCapture(c.st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { rc = ST_CUDA; break; }
+      rc |= split2_step(c, c.ens_y, c.ens_y + c.nbas * c.nfun, dt[j], maxcyc, thresh, true);
+      if (cudaStreamEndCapture(c.st, &graph) != cudaSuccess) rc |= ST_CUDA;
+      if (!rc && cudaGraphInstantiate(&exec, graph, cudaGraphInstantiateFlagUseNodePriority) != cudaSuccess) rc |= ST_CUDA;
+      if (graph) cudaGraphDestroy(graph);
+      if (!rc) key.exec.push_back(exec);
+    }
+    if (rc) key.destroy();
+    if (!rc) {
+      auto& P = ens_plans();
+      if (P.size() >= kEnsPlans) {
+        size_t old = 0;
+        for (size_t k = 1; k < P.size(); ++k)
+          if (P[k].used < P[old].used) old = k;
+        P[old].destroy();
+        P.erase(P.begin() + old);
+      }
+      P.push_back(key);
+      plan = &P.back();
+    }
+  }
+  if (!rc && plan) {
+    plan->used = ++clock;
+    for (int j = 0; j < njob; ++j) {  // the copies on the jobs' streams come first
+      td1c_gpu_ctx_select(ids[j]);
+      cudaEventRecord(evs[2 * j], g->st);
+      cudaStreamWaitEvent(master, evs[2 * j], 0);
+    }
+    static cudaEvent_t e0 = nullptr, e1 = nullptr;
+    if (!e0) { cudaEventCreate(&e0); cudaEventCreate(&e1); }
+    cudaEventRecord(e0, master);
+    std::vector<cudaStream_t> sj(njob);
+    for (int j = 0; j < njob; ++j) {
+      td1c_gpu_ctx_select(ids[j]);
+      sj[j] = g->st;
+      cudaStreamWaitEvent(sj[j], e0, 0);
+    }
+    for (int s = 0; s < nstep && !rc; ++s)
+      for (int j = 0; j < njob && !rc; ++j)
+        if (cudaGraphLaunch(plan->exec[j], sj[j]) != cudaSuccess) rc |= ST_CUDA;
+    for (int j = 0; j < njob; ++j) {
+      cudaEventRecord(evs[2 * j + 1], sj[j]);
       cudaStreamWaitEvent(master, evs[2 * j + 1], 0);
     }
-    if (cudaStreamEndCapture(master, &graph) != cudaSuccess) rc |= ST_CUDA;
-    if (!rc && cudaGraphInstantiate(&exec, graph, cudaGraphInstantiateFlagUseNodePriority) != cudaSuccess) rc |= ST_CUDA;
-    if (graph) cudaGraphDestroy(graph);
-  }
-  if (!rc && exec) {
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    cudaEventRecord(e0, master);
-    for (int s = 0; s < nstep && !rc; ++s)
-      if (cudaGraphLaunch(exec, master) != cudaSuccess) rc |= ST_CUDA;
     cudaEventRecord(e1, master);
-    if (cudaEventSynchronize(e1) != cudaSuccess) rc |= ST_CUDA;
+    for (int j = 0; j < njob; ++j) {
+      td1c_gpu_ctx_select(ids[j]);
+      Ctx& c = *g;
+      const size_t no = c.nbas * c.nfun, nc = c.lcic;
+      cudaMemcpyAsync(d_wfn[j], c.ens_y, no * sizeof(cplx), cudaMemcpyDeviceToDevice, master);
+      cudaMemcpyAsync(d_cic[j], c.ens_y + no, nc * sizeof(cplx), cudaMemcpyDeviceToDevice, master);
+    }
+    if (cudaStreamSynchronize(master) != cudaSuccess) rc |= ST_CUDA;
     float t = 0;
     cudaEventElapsedTime(&t, e0, e1);
     if (ms) *ms = t;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
   }
-  if (exec) cudaGraphExecDestroy(exec);
   for (int j = 0; j < njob; ++j) {
     td1c_gpu_ctx_select(ids[j]);
     if (!g) continue;
@@ -3806,6 +3906,11 @@ int td1c_gpu_ensemble_split2(int njob, const int* ids, void* const* d_wfn, void*
     const size_t no = c.nbas * c.nfun, nc = c.lcic;
     check_finite(c, d_wfn[j], 2 * no, c.st);
     check_finite(c, d_cic[j], 2 * nc, c.st);
+  }
+  for (int j = 0; j < njob; ++j) {
+    td1c_gpu_ctx_select(ids[j]);
+    if (!g) continue;
+    Ctx& c = *g;
     int dst = 0;
     cudaMemcpyAsync(&dst, c.d_status, sizeof(int), cudaMemcpyDeviceToHost, c.st);
     if (cudaStreamSynchronize(c.st) != cudaSuccess) rc |= ST_CUDA;
@@ -3872,6 +3977,7 @@ int td1c_gpu_set_mf_external(int on) {
   Ctx& c = ctx();
   if (!c.initialized) return ST_CONFIG;
   c.mf_external = on ? 1 : 0;
+  ctx().epoch = ++g_epoch;
   return 0;
 }
 

@@ -160,3 +160,34 @@ def test_rhs_replay(cuda_ok, wl):
             assert rel_err(a, dt * first[0, split][0]) < 1e-14
     finally:
         h.final()
+
+
+@pytest.mark.gpu
+def test_ensemble_plan_is_reused_and_renewed(cuda_ok):
+    """Ensemble steps on other buffers (the kept step graph), after a new frozen core of one job (a new graph),
+    and beside another ensemble of the same jobs: each bitwise the jobs' own steps."""
+    import torch
+    from td1c_b200.ensemble import DeviceEnsemble
+    jobs = [dict(W.HE_SMALL, dt=0.01), dict(W.NE_SMALL, dt=0.01)]
+    ens = [DeviceEnsemble(jobs, relax_cycles=0) for _ in range(2)]
+    try:
+        def check(e, scale):
+            a = [[x.clone() for x in e.orb], [x.clone() for x in e.cic]]
+            for x in a[0]:
+                x *= scale
+            b = [[x.clone() for x in v] for v in a]
+            torch.cuda.synchronize()
+            e.run(3, t0=20.0, orb=a[0], cic=a[1])
+            e.run_sequential(3, t0=20.0, orb=b[0], cic=b[1])
+            for u, v in zip(a[0] + a[1], b[0] + b[1]):
+                assert torch.equal(u, v)
+        for e, s in ((ens[0], 1.0), (ens[1], 1.0), (ens[0], 0.9), (ens[0], 1.0), (ens[1], 0.8)):
+            check(e, s)
+        wfn = ens[0].orb[1].cpu().numpy().copy()
+        ens[0].h[1].set_wfn0(0.7 * wfn, ens[0].cic[1].cpu().numpy())
+        check(ens[0], 1.0)
+        ens[1].final()
+        check(ens[0], 0.9)
+    finally:
+        for e in ens:
+            e.final()
