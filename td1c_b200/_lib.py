@@ -12,7 +12,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "_lib")
 LIB_PATH = os.path.join(LIB_DIR, "libtd1c_b200.so")
-SOURCES = ["hprod.cu", "legendre_gemm.cu", "legendre_par.cu", "onebody.cu", "poisson.cu", "mfprod.cu", "reductions.cu", "ci.cu",
+SOURCES = ["hprod.cu", "hostcopy.cu", "legendre_gemm.cu", "legendre_par.cu", "onebody.cu", "poisson.cu", "mfprod.cu", "reductions.cu", "ci.cu",
            "int2e_static.cu", "int2e_dmma.cu", "observables.cu", "h1prop.cu", "h1cycle.cu", "poisson_cond.cu", "poisson_few.cu",
            "legendre_tf32.cu", "legendre_tc.cu", "int2e_tc.cu", "mlp.cu",
            "predictor.cu"]

@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "hostcopy.cuh"
 #include "kernels.cuh"
 #include "reductions.cuh"
 #include "tma.cuh"
@@ -3002,8 +3003,9 @@ void hprod_htot_(const double* dtime, const double* lfield, const double* wfn, c
   if (!c.initialized) { c.status |= ST_CONFIG; return; }
   cudaStream_t st = c.st;
   const size_t so = c.nbas * c.nfun;
-  cudaMemcpyAsync(c.lfield, lfield, 9 * sizeof(double), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(c.wfn_io, wfn, so * sizeof(cplx), cudaMemcpyHostToDevice, st);
+  // the frozen-core rows of wfn are not read, and those of hwfn are zero
+  const size_t nf = c.nfcore * c.nbas;
+  cudaError_t e = host_to_device(c.wfn_io + nf, wfn + 2 * nf, (so - nf) * sizeof(cplx), st);
   cudaMemcpyAsync(c.cic_io, cic, c.lcic * sizeof(cplx), cudaMemcpyHostToDevice, st);
   int rc = rhs_call(c, lfield, c.wfn_io, c.cic_io, c.hwfn_io, c.hcic_io, *dtime);
   // the reference stops on a failed solve (hprod_mkv2mf.F90:167-170); here a
@@ -3012,12 +3014,14 @@ void hprod_htot_(const double* dtime, const double* lfield, const double* wfn, c
   check_finite(c, c.hwfn_io, 2 * so, st);
   check_finite(c, c.hcic_io, 2 * (size_t)c.lcic, st);
   check_finite(c, c.ene, 5, st);
-  cudaMemcpyAsync(hwfn, c.hwfn_io, so * sizeof(cplx), cudaMemcpyDeviceToHost, st);
+  memset(hwfn, 0, nf * sizeof(cplx));
+  if (e == cudaSuccess) e = device_to_host(hwfn + 2 * nf, c.hwfn_io + nf, (so - nf) * sizeof(cplx), st);
   cudaMemcpyAsync(hcic, c.hcic_io, c.lcic * sizeof(cplx), cudaMemcpyDeviceToHost, st);
   cudaMemcpyAsync(c.h_ene, c.ene, 5 * sizeof(double), cudaMemcpyDeviceToHost, st);
   int dst = 0;
   cudaMemcpyAsync(&dst, c.d_status, sizeof(int), cudaMemcpyDeviceToHost, st);
-  cudaError_t e = cudaStreamSynchronize(st);
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = es;
   if (rc || e != cudaSuccess) c.status |= ST_CUDA;
   c.status |= dst;
   if (c.p_ene_fcore) *c.p_ene_fcore = c.h_ene[0];
@@ -3049,6 +3053,7 @@ void hprod_final_(void) {
   delete g;
   g = nullptr;
   g_ctxs[g_cur] = nullptr;
+  if (std::all_of(g_ctxs.begin(), g_ctxs.end(), [](const Ctx* q) { return q == nullptr; })) host_copy_release();
 }
 
 int td1c_gpu_last_status(void) { return g ? g->status : 0; }

@@ -136,8 +136,8 @@ class HProd:
         wfn = np.ascontiguousarray(wfn, dtype=np.complex128)
         cic = np.ascontiguousarray(cic, dtype=np.complex128)
         lf = np.ascontiguousarray(lfield, dtype=np.float64)
-        hw = np.zeros_like(wfn)
-        hc = np.zeros_like(cic)
+        hw = np.empty_like(wfn)  # both are written whole
+        hc = np.empty_like(cic)
         dt = ctypes.c_double(dtime)
         self.lib.hprod_htot_(ctypes.byref(dt), _dp(lf), _dp(wfn.view(np.float64)), _dp(cic.view(np.float64)),
                              _dp(hw.view(np.float64)), _dp(hc.view(np.float64)))

@@ -163,6 +163,36 @@ def test_rhs_replay(cuda_ok, wl):
 
 
 @pytest.mark.gpu
+def test_host_call_of_a_large_state(cuda_ok):
+    """A state above the size from which host copies go through the pinned ring (and not a multiple of its
+    pieces): bitwise the device call, frozen-core rows zero, repeated calls included."""
+    import torch
+    wl = W.small(W.NE_CAS, rmax=30.0, ndvr=20, nfe=21, lmax1=19, lmax2=38, rmask=24.0)
+    from td1c_b200 import basis
+    from td1c_b200.hprod import HProd
+    from td1c_b200.wfn import seeded_orbitals, seeded_cic
+    rad, ang = basis.build(wl)
+    h = HProd(wl, rad, ang)
+    try:
+        tb = h.ci_tables()
+        orb = seeded_orbitals(wl, rad["xrad"], rad["wrad"], rad["mask"])
+        cic = seeded_cic(wl, h.dims["lcic"], tb["stra"], tb["strb"], tb["detoff"], tb["afirst"], tb["acount"])
+        h.set_wfn0(orb, cic)
+        lf = _field(wl)
+        x, c = torch.from_numpy(orb.reshape(-1).copy()).cuda(), torch.from_numpy(cic.copy()).cuda()
+        y, yc = torch.empty_like(x), torch.empty_like(c)
+        torch.cuda.synchronize()
+        h.htot_dev(1.0, lf, x.data_ptr(), c.data_ptr(), y.data_ptr(), yc.data_ptr())
+        h.sync()
+        for _ in range(3):
+            hw, hc = h.htot(1.0, lf, orb, cic)
+            assert np.array_equal(hw.reshape(-1), y.cpu().numpy()) and np.array_equal(hc, yc.cpu().numpy())
+            assert not np.any(hw[0])
+    finally:
+        h.final()
+
+
+@pytest.mark.gpu
 def test_ensemble_plan_is_reused_and_renewed(cuda_ok):
     """Ensemble steps on other buffers (the kept step graph), after a new frozen core of one job (a new graph),
     and beside another ensemble of the same jobs: each bitwise the jobs' own steps."""
