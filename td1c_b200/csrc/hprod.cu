@@ -2939,6 +2939,8 @@ void hprod_init_(void) {
   cudaDeviceSynchronize();
   rc |= (int)cudaGetLastError();
   if (rc) { c.status |= ST_CUDA; return; }
+  c.rhs = new RhsGraph();
+  c.rhs->io = dalloc<RhsIo>(1);
   c.initialized = true;
 }
 
