@@ -1301,24 +1301,26 @@ int build_reductions(Ctx& c) {
       }
     }
     eoff[n] = (int)elist.size();
-    // items (block, up to MFD_MI m-tiles, n-tile) over the warps of a CTA, longest first to the least loaded
+    // items (block, up to MFD_MI m-tiles) over the warps of a CTA, longest first to the least loaded quarter of
+    // the SM (warp index mod 4) and in it to the least loaded warp
     std::vector<std::pair<int, int4>> items;
     for (size_t b = 0; b < dblk.size(); ++b) {
       const int ng = (dblk[b].mt + MFD_MI - 1) / MFD_MI;
       for (int gq = 0; gq < ng; ++gq) {
         const int m0 = dblk[b].mt * gq / ng, m1 = dblk[b].mt * (gq + 1) / ng;
-        for (int t = 0; t < MFD_TQ / 8; ++t) items.push_back({(m1 - m0) * dblk[b].kpad / 4, make_int4((int)b, m0, m1 - m0, t)});
+        items.push_back({(m1 - m0) * dblk[b].kpad / 4, make_int4((int)b, m0, m1 - m0, 0)});
       }
     }
     std::stable_sort(items.begin(), items.end(), [](const std::pair<int, int4>& x, const std::pair<int, int4>& y) { return x.first > y.first; });
     std::vector<std::vector<int4>> wl(MFD_NT / 32);
-    std::vector<int> wload(MFD_NT / 32, 0), ioff;
+    std::vector<int> wload(MFD_NT / 32, 0), qload(4, 0), ioff;
     for (auto& it : items) {
       int best = 0;
       for (int w = 1; w < MFD_NT / 32; ++w)
-        if (wload[w] < wload[best]) best = w;
+        if (std::make_pair(qload[w % 4], wload[w]) < std::make_pair(qload[best % 4], wload[best])) best = w;
       wl[best].push_back(it.second);
       wload[best] += it.first;
+      qload[best % 4] += it.first;
     }
     std::vector<int4> witem;
     for (auto& v : wl) {

@@ -264,7 +264,7 @@ struct MfprodArgs {
   double* dcoef;          // [ncoef_d]
   const int2* elist;      // per active target x: (D2V row, other orbital | conj << 16), in row order
   const int* eoff;        // [nact + 1] offsets into elist
-  const int4* witem;      // (block, first m-tile, m-tiles, n-tile) of every warp, in warp order
+  const int4* witem;      // (block, first m-tile, m-tiles, 0) of every warp, in warp order
   const int* ioff;        // [warps + 1] offsets into witem
 };
 int launch_mfprod(const MfprodArgs& a, cudaStream_t st);

@@ -211,7 +211,10 @@ __global__ void mfd_fill_kernel(int n, const MfdCoef* __restrict__ map, const cp
 // The contraction in real form: a row's two parts over the depth (Wr, Wi) of each stored pair, where the
 // complex form over ordered pairs did every product twice.  What bounds it: a tile's phases (DMMA, then the
 // FFMA twfn and v2orbg sums) follow one another inside a CTA, so its warps wait at the barriers between
-// them; three CTAs of 256 threads per SM fill part of that.  Ne, CAS(8e,9o), 136080 points: 112 -> 81 us.
+// them; three CTAs of 256 threads per SM fill part of that.  Ne, CAS(8e,9o), 113905 points: 112 -> 81 us.  An item
+// takes both n-tiles of its m-tiles, so a coefficient fragment is loaded once for two products (shared-memory loads are
+// the other thing the DMMA phase waits for), and the core terms go to the warps with the fewest items first: a Ne
+// right-hand side 453 -> 448 us, an open shell of 6 orbitals on 37 x 12 points 57.2 -> 55.6.
 struct MfdSmem {
   int nfun, nact, npair, nrow, ncoef, nelist, ndcol, nblk, nitem;
   __host__ __device__ size_t w() const { return 0; }                                       // complex units
@@ -311,7 +314,7 @@ __global__ void __launch_bounds__(MFD_NT, 3) mfprod_dmma_kernel(MfprodArgs a) {
   };
   const int ndcore = ncore - nfcore;
   // ---- 2. core terms (same sums and order as mfprod_kernel)
-  for (int e = tid; e < (nfun - nfcore) * MFD_TQ; e += MFD_NT) {
+  for (int e = MFD_NT - 1 - tid; e < (nfun - nfcore) * MFD_TQ; e += MFD_NT) {  // the last warps have the fewest items
     const int i = nfcore + e / MFD_TQ, t = e % MFD_TQ;
     if (q0 + t >= ng) continue;
     cplx g = mkc(0, 0);
@@ -360,38 +363,51 @@ __global__ void __launch_bounds__(MFD_NT, 3) mfprod_dmma_kernel(MfprodArgs a) {
   for (int it = sioff[warp]; it < sioff[warp + 1]; ++it) {
     const int4 wi = sitem[it];
     const MfdBlock B = sblk[wi.x];
-    double acc[MFD_MI][2];
+    double acc[MFD_MI][2][2];
 #pragma unroll
-    for (int i = 0; i < MFD_MI; ++i) acc[i][0] = acc[i][1] = 0.0;
+    for (int i = 0; i < MFD_MI; ++i) acc[i][0][0] = acc[i][0][1] = acc[i][1][0] = acc[i][1][1] = 0.0;
     // m-tiles past the item's repeat its last one (their results are not stored)
     const double* arow[MFD_MI];
 #pragma unroll
     for (int i = 0; i < MFD_MI; ++i) arow[i] = sC + B.coff + (size_t)((wi.y + min(i, wi.z - 1)) * 8 + gid) * B.pa + tig;
-    const double* wd = reinterpret_cast<const double*>(sW) + 2 * (wi.w * 8 + gid) + (tig & 1);
+    const double* wd = reinterpret_cast<const double*>(sW) + 2 * gid + (tig & 1);
     const int* col = scol + B.col0 + (tig >> 1);
     const int ksn = B.kpad / 4;
     if (wi.z == MFD_MI) {
 #pragma unroll 2
       for (int ks = 0; ks < ksn; ++ks) {
-        const double bv = wd[(size_t)col[2 * ks] * (2 * MFD_WP)];
+        const double* wr = wd + (size_t)col[2 * ks] * (2 * MFD_WP);
+        const double b0 = wr[0], b1 = wr[16];
 #pragma unroll
-        for (int i = 0; i < MFD_MI; ++i) mfd_dmma(acc[i][0], acc[i][1], arow[i][4 * ks], bv);
+        for (int i = 0; i < MFD_MI; ++i) {
+          const double av = arow[i][4 * ks];
+          mfd_dmma(acc[i][0][0], acc[i][0][1], av, b0);
+          mfd_dmma(acc[i][1][0], acc[i][1][1], av, b1);
+        }
       }
     } else {
 #pragma unroll 2
       for (int ks = 0; ks < ksn; ++ks) {
-        const double bv = wd[(size_t)col[2 * ks] * (2 * MFD_WP)];
-        mfd_dmma(acc[0][0], acc[0][1], arow[0][4 * ks], bv);
-        if (wi.z > 1) mfd_dmma(acc[1][0], acc[1][1], arow[1][4 * ks], bv);
+        const double* wr = wd + (size_t)col[2 * ks] * (2 * MFD_WP);
+        const double b0 = wr[0], b1 = wr[16], a0 = arow[0][4 * ks];
+        mfd_dmma(acc[0][0][0], acc[0][0][1], a0, b0);
+        mfd_dmma(acc[0][1][0], acc[0][1][1], a0, b1);
+        if (wi.z > 1) {
+          const double a1 = arow[1][4 * ks];
+          mfd_dmma(acc[1][0][0], acc[1][0][1], a1, b0);
+          mfd_dmma(acc[1][1][0], acc[1][1][1], a1, b1);
+        }
       }
     }
 #pragma unroll
     for (int i = 0; i < MFD_MI; ++i) {
       const int rr = (wi.y + i) * 8 + gid, r = rr >> 1;
       if (i < wi.z && r < B.nr) {
-        double* drow = reinterpret_cast<double*>(sD + (size_t)(B.drow0 + r) * MFD_DP + wi.w * 8 + 2 * tig) + (rr & 1);
-        drow[0] = acc[i][0];
-        drow[2] = acc[i][1];
+        double* drow = reinterpret_cast<double*>(sD + (size_t)(B.drow0 + r) * MFD_DP + 2 * tig) + (rr & 1);
+        drow[0] = acc[i][0][0];
+        drow[2] = acc[i][0][1];
+        drow[16] = acc[i][1][0];
+        drow[18] = acc[i][1][1];
       }
     }
   }
