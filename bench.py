@@ -43,7 +43,7 @@ import time
 
 import numpy as np
 
-# the ensemble leg forks one graph into four streams per job: give the device enough hardware
+# the ensemble leg runs a graph of four streams per job: give the device enough hardware
 # work queues that the jobs' streams do not share them (read when CUDA starts)
 if any(a.startswith("--ensemble") for a in sys.argv[1:]):
     os.environ.setdefault("CUDA_DEVICE_MAX_CONNECTIONS", "32")
@@ -752,7 +752,7 @@ def full_pulse(args, h, wl, dt, arms, set_arm, steps, placed, deviations, torch,
 
 
 def ensemble_leg(njob, seed=7, nstep=16, small=False):
-    """The seeded ensemble's jobs stepped together by one graph per step, against the same steps run
+    """The seeded ensemble's jobs stepped together (a step graph per job, side by side), against the same steps run
     job after job (fs/s summed over the jobs)."""
     from td1c_b200 import autotune
     from td1c_b200.ensemble import DeviceEnsemble, job_list

@@ -343,10 +343,10 @@ int td1c_gpu_set_tuning(int mt, int mf_cap, int i2_split);
 int td1c_gpu_get_tuning(int* out4);
 /* nstep split2 steps (td1c_gpu_split2 with its mask) of njob jobs at once:
  * job j is context ids[j] (bound with split_type 1) with state d_wfn[j],
- * d_cic[j] and its own pulse (t0, dt, fint, wlen, numcyc, cep per job).  One
- * CUDA graph holds one step of every job, each job's kernels on its own
- * streams forked from one stream, so the jobs run side by side; it is
- * replayed nstep times.  *ms (host, may be NULL) = device time of the
+ * d_cic[j] and its own pulse (t0, dt, fint, wlen, numcyc, cep per job).  A
+ * CUDA graph per job holds its step and is launched nstep times on the job's
+ * own stream, so the jobs run side by side; the graphs are kept for later
+ * calls.  *ms (host, may be NULL) = device time of the
  * replays.  Returns 0 or the status bits of the jobs. */
 int td1c_gpu_ensemble_split2(int njob, const int* ids, void* const* d_wfn, void* const* d_cic, const double* t0,
                              const double* dt, int nstep, const double* fint, const double* wlen, const double* numcyc,

@@ -9,7 +9,9 @@
 //
 // The ring and its threads belong to the process: four slots of 2 MB, made by
 // the first large copy and given back by host_copy_release (with the last
-// context).  A copy that finds the ring in use by another thread, a forked
+// context).  Ne's right-hand side from host buffers: 2700 -> 1480 us (the RHS itself 450).
+// From 512 KB on: below that a copy is a few tens of us on the plain path, about
+// what waking the threads costs.  A copy that finds the ring in use by another thread, a forked
 // child, a second device, or a failed allocation takes the plain path.
 #include <pthread.h>
 #include <unistd.h>

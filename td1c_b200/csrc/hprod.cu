@@ -4,13 +4,13 @@
 // kernels on one stream, all data resident in HBM:
 //   orbin        sph2ang1 GEMM (+ frozen-core gauge phase)   hprod_orbin.F90
 //   CI           D = E_pq c, 1-/2-RDM, regularised 1/D        ormas_mkden1/2, hprod_invden.F90
-//   one-body     tprod + zprod/pzprod stencil                 hprod_tprod/zprod/pzprod.F90
+//   one-body     tprod + zprod/pzprod, DMMA per element       hprod_tprod/zprod/pzprod.F90
 //   pair density fused into the theta->l GEMM                 hprod_mkrho2.F90, bas_ang2sph2.F90
-//   Poisson      banded Cholesky solves per (pair, l)         hprod_mkv2mf.F90
+//   Poisson      static condensation per (pair, l)            hprod_mkv2mf.F90
 //   l->theta     GEMM (Hermitian half read with conj)         bas_sph2ang2.F90
 //   mfprod       core J/K, active J/K, 2-RDM contraction      hprod_mfprod2.F90
 //   theta->l     GEMM for g and v2 orbitals                   bas_ang2sph1.F90
-//   integrals    orbital matrix elements, int2e block GEMM    hprod_mkint1/2_sph.F90
+//   integrals    orbital matrix elements, int2e products      hprod_mkint1/2_sph.F90
 //   small        int1e, energies, X matrix                    hprod_ene_*.F90, hprod_htot_mkxmat.F90
 //   sigma        CI sigma vector                              ormas_xact2/ormas_hcic
 //   dtorb        hwfn = -i dt (h0+h1+g+v2) phi + sum_j phi_j X_ji  hprod_htot_dtorb.F90
@@ -1682,7 +1682,8 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
 }
 
 // One RHS on the caller's device buffers.  An eager RHS is some twenty launches and events on three
-// streams, more host time than the small workloads' kernels take; the second call in a row with the same
+// streams, more host time than the small workloads' kernels take (us a call among others, eager and replayed: an
+// 8 x 8 box 46.0 and 15.2, He 45.7 and 22.3, Ne's 445 either way); the second call in a row with the same
 // settings captures it once (reading the buffers and the field from device memory, so the capture holds
 // for any buffers), and later calls replay it.  The capture goes with the context, or when a setting changes.
 struct RhsKey {
@@ -3733,14 +3734,16 @@ int td1c_gpu_get_tuning(int* out4) {
   return 0;
 }
 
-// nstep split2 steps of every job of an ensemble in one CUDA graph per step:
-// the step of job j is captured on job j's own streams, forked from one
-// stream and joined back, so the jobs' kernels have no order between them and
-// the GPU runs them side by side.  The step works on a state buffer of each
-// context (the callers' states are copied in and out), so its graph holds for
-// any state buffers and is kept: up to EnsPlans of them, the least recently
-// used one makes room, and a plan goes with any of its contexts.  Capturing and
-// instantiating a small ensemble's step takes longer than its steps.
+// nstep split2 steps of every job of an ensemble: one CUDA graph per job holds
+// its step, and the graphs are launched on the jobs' own streams, so the jobs'
+// kernels have no order between them and the GPU runs them side by side (one
+// graph with a branch per job took 2.5 times as long on six small jobs: its
+// branches hardly overlapped).  The step works on a state buffer of each
+// context (the callers' states are copied in and out), so the graphs hold for
+// any state buffers and are kept: up to kEnsPlans sets of them, the least recently
+// used one makes room, and a set goes with any of its contexts.  Capturing and
+// instantiating a small ensemble's step takes longer than its steps (six jobs,
+// four steps: 27 ms a call when it was done on each, 10 kept, 4 with a graph per job).
 // *ms = device time of the nstep replays.
 struct EnsPlan {
   std::vector<int> ids;

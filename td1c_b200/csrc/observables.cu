@@ -96,7 +96,8 @@ int dipole_partial_size(int Nr, int nent) { return ((Nr + DIP_CHUNK - 1) / DIP_C
 // reduction per CTA and then, in rank order, over the cluster's distributed
 // shared memory (two slots in turn, so one cluster barrier per sum is enough).
 // The chain of dependent sums is what bounds it: one CTA alone streamed each
-// orbital pair through a single SM (Ne's 25 sums took 10 times longer).
+// orbital pair through a single SM.  Three relaxation cycles of C (6 orbitals, 33
+// elements of 21 points, lmax 26): 1910 -> 1600 us with it.
 // ---------------------------------------------------------------------------
 constexpr int ORTH_NT = 1024, ORTH_CTAS = 8;
 

@@ -113,11 +113,11 @@ def gather(results, dist=None, dst=0):
 
 
 # ---------------------------------------------------------------------------
-# the ensemble on one GPU: a context per job, one captured graph per step
+# the ensemble on one GPU: a context and a captured step graph per job
 # ---------------------------------------------------------------------------
 class DeviceEnsemble:
     """Independent jobs, each in a context of its own (own tables, buffers and streams), stepped
-    together by td1c_gpu_ensemble_split2: one CUDA graph per step holds one split2 step of every job.
+    together by td1c_gpu_ensemble_split2: each job's split2 step is a CUDA graph on the job's own stream.
 
     tables(wl) -> (rad, ang) gives the grids and tables of a job (default: the package's builder);
     state(h, wl) -> (orb, cic) its initial state (default: seeded, orthonormalised and relaxed in
