@@ -428,7 +428,11 @@ int launch_h1loop_ctl(int* iter, const int* done, int maxcyc, cudaGraphCondition
 int launch_h1bridge(const H1ElemArgs& a, cudaStream_t st);
 // The folded passes of h1cycle.cu: one launch per pass, z in [l][element][orbital][point] and the bridge
 // shares in [l][element][side][orbital], two buffers of each by the cycle's parity
-constexpr int H1C_WMAX = 8;  // widest band of the bridge inverse the folded passes take
+// widest band of the bridge inverse the folded passes take.  Up to 4 the shares they stage (10 (2 w + 3) values per
+// orbital) fit where the coupled sums stand later; 8 adds 10 KB and costs the third CTA of an SM.  A time step's band
+// is 1 to 5 on elements of 9 to 21 points (a Ne cycle 42 us, the two-launch pass 64); long steps on fine grids, whose
+// inverse is no band, go there.
+constexpr int H1C_WMAX = 8;
 struct H1CycArgs {
   H1Fac fac;
   int Nr, L1, nfun, nfcore, mmax1, igauge;
