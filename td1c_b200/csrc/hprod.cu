@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <complex>
 #include <cstdio>
@@ -73,6 +74,20 @@ T* dupload(const std::vector<T>& v) {
   return p;
 }
 
+// What a captured step was built from: its buffers, its parameters, the settings it takes by value, and the
+// context's epoch, which stands for everything else it holds (tables, one-body factors)
+constexpr int kSettings = 8;
+struct StepKey {
+  const void *y = nullptr, *yc = nullptr, *tab = nullptr, *reset_orb = nullptr, *reset_cic = nullptr;
+  double dt = 0, thresh = 0;
+  int maxcyc = 0, mask = 0;
+  std::array<int, kSettings> set{};
+  unsigned long epoch = 0;
+  bool operator==(const StepKey& k) const {
+    return y == k.y && yc == k.yc && tab == k.tab && reset_orb == k.reset_orb && reset_cic == k.reset_cic && dt == k.dt &&
+           thresh == k.thresh && maxcyc == k.maxcyc && mask == k.mask && set == k.set && epoch == k.epoch;
+  }
+};
 struct RkBufs {
   cplx *y0 = nullptr, *yt = nullptr, *k = nullptr, *k2 = nullptr;  // orbitals then CI, contiguous
   double* lf_cur = nullptr;
@@ -80,16 +95,10 @@ struct RkBufs {
   size_t cap = 0;
   const cplx* reset_orb = nullptr;  // optional: every step starts from this state
   const cplx* reset_cic = nullptr;
-  // cached graph of one step and what it was captured with
-  const void* g_y = nullptr; const void* g_yc = nullptr; const void* g_tab = nullptr;
-  const void* g_ro = nullptr; double g_dt = 0; long g_per = 0;
   int h_counter[2] = {0, 0};
-  // cached graphs of one split2 / ETD-RK2 / ETD-RK4 step
-  const void* s_y[3] = {nullptr, nullptr, nullptr}; const void* s_yc[3] = {nullptr, nullptr, nullptr};
-  const void* s_tab[3] = {nullptr, nullptr, nullptr}; double s_dt[3] = {0, 0, 0}; int s_cyc[3] = {0, 0, 0};
-  double s_thr[3] = {0, 0, 0}; int s_split[3] = {-1, -1, -1}; int s_mask[3] = {-1, -1, -1}; long s_per[3] = {0, 0, 0};
-  const void* s_ro[3] = {nullptr, nullptr, nullptr};
-  int g_ctl = -1, s_ctl[3] = {-1, -1, -1};  // control flags (icomp, igauge) the graphs were captured with
+  // of the cached graphs of one RK4 / split2 / ETD-RK2 / ETD-RK4 step
+  StepKey key[4];
+  long per[4] = {0, 0, 0, 0};  // kernel launches
 };
 struct Etd4Bufs {
   cplx *w1 = nullptr, *w2 = nullptr, *w3 = nullptr, *h2 = nullptr, *h3 = nullptr, *tmp = nullptr;
@@ -98,7 +107,7 @@ struct Etd4Bufs {
 struct RhsGraph;  // the captured RHS (rhs_call)
 unsigned long g_epoch = 0;
 struct Ctx {
-  unsigned long epoch = ++g_epoch;  // renewed by every change of what a captured step was built from
+  unsigned long epoch = ++g_epoch;  // renewed by every change of what a captured step holds and its key does not name
   cplx* ens_y = nullptr;  // this job's state inside an ensemble call (orbitals, then CI)
   RhsGraph* rhs = nullptr;
   std::vector<void*> allocs;  // device allocations of this context
@@ -229,6 +238,8 @@ struct Ctx {
   cplx* lp_save = nullptr;  // the state at the start of a judged window (orbitals, then CI)
   cudaGraphExec_t lp_exec[3] = {nullptr, nullptr, nullptr};  // E, H, P steps
   long lp_exec_launch[3] = {0, 0, 0};
+  std::array<int, kSettings> lp_set{};  // settings and epoch the learned steps were captured with
+  unsigned long lp_epoch = 0;
   // what the captured steps and the window schedule belong to: a call that starts where the last
   // one ended (same state buffers, field and step) continues its history and schedule
   const void* lp_key_y = nullptr; const void* lp_key_yc = nullptr; const void* lp_key_tab = nullptr;
@@ -244,6 +255,11 @@ struct Ctx {
   cudaEvent_t ev_sig_fork = nullptr, ev_sig_join = nullptr;
   int nev = 0;
 };
+
+// the settings a captured right-hand side or step takes by value
+std::array<int, kSettings> settings(const Ctx& c) {
+  return {c.icomp, c.igauge, c.isplit, c.mixed, c.mf_external, c.tune_mt, c.tune_mf_cap, c.tune_i2_split};
+}
 
 // phases of run_htot, in order (td1c_gpu_profile reports their durations)
 const char* kPhaseNames[] = {"orbin", "ci_rdm", "onebody", "rho_gemm", "poisson", "w_gemm", "mfprod",
@@ -1688,8 +1704,10 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
 // for any buffers), and later calls replay it.  The capture goes with the context, or when a setting changes.
 struct RhsKey {
   double dtime = 0, ene_fcore = 0;
-  int set[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  bool operator==(const RhsKey& k) const { return memcmp(this, &k, sizeof(RhsKey)) == 0; }
+  std::array<int, kSettings> set{};
+  bool operator==(const RhsKey& k) const {
+    return memcmp(&dtime, &k.dtime, sizeof(double)) == 0 && memcmp(&ene_fcore, &k.ene_fcore, sizeof(double)) == 0 && set == k.set;
+  }
 };
 struct RhsGraph {
   cudaGraphExec_t exec = nullptr;
@@ -1705,10 +1723,7 @@ int rhs_call(Ctx& c, RhsGraph& g, const double* lf, const RhsIo& io, double dtim
   lfield_kernel<<<1, 32, 0, c.st>>>(f, c.lfield, io, g.io);
   c.launches++;
   RhsKey key;
-  memset(&key, 0, sizeof(key));
-  key.dtime = dtime; key.ene_fcore = c.ene_fcore;
-  const int set[8] = {c.icomp, c.igauge, c.isplit, c.mixed, c.mf_external, c.tune_mt, c.tune_mf_cap, c.tune_i2_split};
-  memcpy(key.set, set, sizeof(set));
+  key.dtime = dtime; key.ene_fcore = c.ene_fcore; key.set = settings(c);
   cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(c.st, &cst);
   auto eager = [&]() { return run_htot(c, c.lfield, io.wfn, io.cic, io.hwfn, io.hcic, dtime); };
@@ -1908,12 +1923,12 @@ int h1_factor(Ctx& c, cplx fac, H1Fac* out) {
     f.tdl = dalloc<cplx>(nbt); f.tdi = dalloc<cplx>(nbt); f.tdu = dalloc<cplx>(nbt); f.tdu2 = dalloc<cplx>(nbt);
     f.tpiv = dalloc<int>(nbt);
   } else {
-    // all slots taken: rebuild the oldest in place
+    // all slots taken: rebuild the oldest in place; captured steps may hold its factors
+    c.epoch = ++g_epoch;
     for (int i = 0; i < Ctx::kH1Slots - 1; ++i) std::swap(c.h1slot[i], c.h1slot[i + 1]);
     sl = &c.h1slot[Ctx::kH1Slots - 1];
   }
   sl->cre = fac.x; sl->cim = fac.y;
-  c.epoch = ++g_epoch;  // captured steps may hold the slot's factors
   H1FacSrc src{};
   src.Nr = c.Nr; src.L1 = c.L1; src.nd = c.nd; src.nfe = c.nfe; src.c = fac;
   src.radk = c.radk; src.radk0 = c.radk0; src.tdiag = c.tdiag; src.status = c.d_status;
@@ -2569,21 +2584,16 @@ int prop_run(int kind, void* d_wfn, void* d_cic, double t0, double dt, int nstep
   } else {
     int s0 = 0;
     cudaGraphExec_t& ge = c.graph_exec[kind];
-    bool cached;
-    const int ctl = c.icomp * 2 + c.igauge + 4 * c.mixed + 8 * c.mf_external;
-    if (kind == 0) {
-      cached = ge && b.g_y == y && b.g_yc == yc && b.g_tab == c.field_tab && b.g_dt == dt && b.g_ro == b.reset_orb &&
-               b.g_ctl == ctl;
-    } else {
-      const int q = kind - 1;
-      cached = ge && b.s_y[q] == y && b.s_yc[q] == yc && b.s_tab[q] == c.field_tab && b.s_dt[q] == dt &&
-               b.s_cyc[q] == maxcyc && b.s_thr[q] == thresh && b.s_split[q] == c.isplit &&
-               b.s_mask[q] == (int)do_mask && b.s_ro[q] == b.reset_orb && b.s_ctl[q] == ctl;
-    }
-    if (!cached) {
+    StepKey key;
+    key.y = y; key.yc = yc; key.tab = c.field_tab; key.reset_orb = b.reset_orb; key.reset_cic = b.reset_cic;
+    key.dt = dt; key.mask = do_mask;
+    if (kind != 0) { key.thresh = thresh; key.maxcyc = maxcyc; }
+    key.set = settings(c); key.epoch = c.epoch;
+    if (!(ge && b.key[kind] == key)) {
+      if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
       rc |= step();
       s0 = 1;
-      if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
+      key.epoch = c.epoch;  // the eager step may have built factors
       long l0 = c.launches;
       cudaGraph_t graph;
       if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return ST_CUDA;
@@ -2591,22 +2601,13 @@ int prop_run(int kind, void* d_wfn, void* d_cic, double t0, double dt, int nstep
       if (cudaStreamEndCapture(st, &graph) != cudaSuccess) return ST_CUDA;
       if (cudaGraphInstantiate(&ge, graph, cudaGraphInstantiateFlagUseNodePriority) != cudaSuccess) { cudaGraphDestroy(graph); return ST_CUDA; }
       cudaGraphDestroy(graph);
-      const long per_step = c.launches - l0;
+      b.per[kind] = c.launches - l0;
       c.launches = l0;
-      if (kind == 0) {
-        b.g_per = per_step; b.g_y = y; b.g_yc = yc; b.g_tab = c.field_tab; b.g_dt = dt; b.g_ro = b.reset_orb;
-        b.g_ctl = ctl;
-      } else {
-        const int q = kind - 1;
-        b.s_per[q] = per_step; b.s_y[q] = y; b.s_yc[q] = yc; b.s_tab[q] = c.field_tab; b.s_dt[q] = dt;
-        b.s_cyc[q] = maxcyc; b.s_thr[q] = thresh; b.s_split[q] = c.isplit; b.s_mask[q] = (int)do_mask;
-        b.s_ro[q] = b.reset_orb; b.s_ctl[q] = ctl;
-      }
+      b.key[kind] = key;
     }
-    const long per_step = kind == 0 ? b.g_per : b.s_per[kind - 1];
     for (int s = s0; s < nstep; ++s) {
       if (cudaGraphLaunch(ge, st) != cudaSuccess) return ST_CUDA;
-      c.launches += per_step;
+      c.launches += b.per[kind];
     }
   }
   check_finite(c, y, 2 * no, st);
@@ -2697,8 +2698,9 @@ int learned_run(void* d_wfn, void* d_cic, double t0, double dt, int nstep, doubl
   bool same = c.lp_key_y == y && c.lp_key_yc == yc && c.lp_key_tab == c.field_tab && !record;
   for (int i = 0; i < 8 && same; ++i) same = c.lp_key[i] == key[i];
   const bool cont = same && std::fabs(t0 - c.lp_t_end) <= 1e-9 * std::max(1.0, std::fabs(t0));
-  if (!same || record) {
+  if (!same || record || c.lp_epoch != c.epoch || c.lp_set != settings(c))
     for (auto& ge : c.lp_exec) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
+  if (!same || record) {
     c.lp_key_y = record ? nullptr : y; c.lp_key_yc = record ? nullptr : yc; c.lp_key_tab = c.field_tab;
     for (int i = 0; i < 8; ++i) c.lp_key[i] = key[i];
   }
@@ -2730,6 +2732,8 @@ int learned_run(void* d_wfn, void* d_cic, double t0, double dt, int nstep, doubl
     cudaGraphDestroy(graph);
     c.lp_exec_launch[kind] = c.launches - l0;
     c.launches = l0;
+    c.lp_set = settings(c);
+    c.lp_epoch = c.epoch;
     return 0;
   };
   auto step = [&](int kind) -> int {
@@ -2886,14 +2890,12 @@ int td1c_gpu_bind_ormas(int nsub) {
 int td1c_gpu_bind_control(int icomp, int igauge) {
   Ctx& c = ctx();
   c.icomp = icomp; c.igauge = igauge;
-  ctx().epoch = ++g_epoch;
   return 0;
 }
 
 int td1c_gpu_bind_split(int split_type) {
   if (split_type < 0 || split_type > 2) return ST_CONFIG;
   ctx().isplit = split_type;
-  ctx().epoch = ++g_epoch;
   return 0;
 }
 
@@ -3509,7 +3511,6 @@ int td1c_gpu_set_mixed(int on) {
   if (on < 0 || on > 3) return ST_CONFIG;
   c.mixed = on;
   if (c.mixed) build_tc_plans(c);
-  ctx().epoch = ++g_epoch;
   return 0;
 }
 
@@ -3719,11 +3720,9 @@ int td1c_gpu_ctx_destroy(int id) {
 
 int td1c_gpu_set_tuning(int mt, int mf_cap, int i2_split_) {
   Ctx& c = ctx();
-  c.epoch = ++g_epoch;
   if ((mt != 0 && mt != 3 && mt != 6) || mf_cap < 0) return ST_CONFIG;
   c.tune_mt = mt; c.tune_mf_cap = mf_cap; c.tune_i2_split = i2_split_;
-  for (auto& ge : c.graph_exec) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }  // recaptured with the new shapes
-  c.lp_key_y = nullptr;  // and so are the learned form's steps
+  c.lp_key_y = nullptr;  // the learned form's schedule starts afresh
   return 0;
 }
 
@@ -3748,6 +3747,7 @@ int td1c_gpu_get_tuning(int* out4) {
 struct EnsPlan {
   std::vector<int> ids;
   std::vector<unsigned long> epoch;
+  std::vector<std::array<int, kSettings>> set;
   std::vector<double> dt;
   std::vector<const void*> tab;
   int maxcyc = 0;
@@ -3759,7 +3759,7 @@ struct EnsPlan {
     exec.clear();
   }
   bool same(const EnsPlan& k) const {
-    return ids == k.ids && epoch == k.epoch && dt == k.dt && tab == k.tab && maxcyc == k.maxcyc && thresh == k.thresh;
+    return ids == k.ids && epoch == k.epoch && set == k.set && dt == k.dt && tab == k.tab && maxcyc == k.maxcyc && thresh == k.thresh;
   }
 };
 static constexpr size_t kEnsPlans = 8;
@@ -3831,6 +3831,7 @@ int td1c_gpu_ensemble_split2(int njob, const int* ids, void* const* d_wfn, void*
     key.dt.push_back(dt[j]);
     key.tab.push_back(c.field_tab);
     key.epoch.push_back(c.epoch);
+    key.set.push_back(settings(c));
   }
   EnsPlan* plan = nullptr;
   for (EnsPlan& q : ens_plans())
@@ -3989,7 +3990,6 @@ int td1c_gpu_set_mf_external(int on) {
   Ctx& c = ctx();
   if (!c.initialized) return ST_CONFIG;
   c.mf_external = on ? 1 : 0;
-  ctx().epoch = ++g_epoch;
   return 0;
 }
 
