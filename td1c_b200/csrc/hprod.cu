@@ -106,17 +106,11 @@ struct Etd4Bufs {
 };
 struct RhsGraph;  // the captured RHS (rhs_call)
 unsigned long g_epoch = 0;
-struct Ctx {
-  unsigned long epoch = ++g_epoch;  // renewed by every change of what a captured step holds and its key does not name
-  cplx* ens_y = nullptr;  // this job's state inside an ensemble call (orbitals, then CI)
-  RhsGraph* rhs = nullptr;
-  std::vector<void*> allocs;  // device allocations of this context
-  RkBufs rk;                  // propagation buffers and cached step graphs
-  Etd4Bufs e4;
+// What the caller bound to a context, its settings and its streams: all that outlives a second hprod_init_
+struct Bound {
   bool own_streams = false;   // contexts other than the default one own their streams
   int tune_mt = 0, tune_mf_cap = 0, tune_i2_split = 0;  // launch shapes (0: the built-in choice)
-  // ---- bound inputs
-  bool have_rad = false, have_sph = false, have_bas = false, initialized = false;
+  bool have_rad = false, have_sph = false, have_bas = false;
   int nfe = 0, nd = 0, nrad = 0, Nr = 0;
   double rmask = 0;
   std::vector<double> h_xrad, h_wrad, h_radp, h_radk, h_radk0, h_mask;
@@ -130,6 +124,28 @@ struct Ctx {
   int nsub = 1;  // ORMAS subspaces of the active space (ormas_bind_ nsub); 1 = CAS
   // ---- hprod_bind_ outputs
   double *p_ene_fcore = nullptr, *p_ene_dcore = nullptr, *p_ene_core = nullptr, *p_ene_act = nullptr, *p_ene_tot = nullptr;
+  int mixed = 0;  // 1: the mean field's pair-density and pair-potential transforms in split TF32 (tcgen05)
+  int mf_external = 0;  // 1: the RHS takes W and int2e as they stand (the learned form's predicted stages)
+  // learned form: the caller's network and policy
+  MlpInferArgs lp_mi{};
+  bool lp_has_net = false;
+  int lp_use_net = 0;
+  double lp_bound = 1e-6;
+  int lp_screen = 1;  // 1: predicted windows only after a fill window whose judge values pass
+  cudaStream_t st = nullptr;
+  cudaStream_t st2 = nullptr;  // side stream of the CI RDM chain (process lifetime, like st)
+  cudaStream_t st3 = nullptr;  // side stream of the one-body stencil and of int2e
+  cudaStream_t st4 = nullptr;  // stream on which graph-loop bodies are captured
+  int status = 0;
+};
+struct Ctx : Bound {
+  unsigned long epoch = ++g_epoch;  // renewed by every change of what a captured step holds and its key does not name
+  cplx* ens_y = nullptr;  // this job's state inside an ensemble call (orbitals, then CI)
+  RhsGraph* rhs = nullptr;
+  std::vector<void*> allocs;  // device allocations of this context
+  RkBufs rk;                  // propagation buffers and cached step graphs
+  Etd4Bufs e4;
+  bool initialized = false;
   // ---- device tables
   double* ob_tab = nullptr;  // one-body blocks of the elements
   double *xrad = nullptr, *mask = nullptr, *radk = nullptr, *radk0 = nullptr, *radp = nullptr, *cost = nullptr;
@@ -189,8 +205,6 @@ struct Ctx {
   cudaGraphExec_t graph_exec[4] = {nullptr, nullptr, nullptr, nullptr};
   long launches = 0;
   // ---- misc
-  cudaStream_t st = nullptr;
-  int status = 0;
   int* d_status = nullptr;  // device status word (ST_* bits)
   double* d_scalar = nullptr;
   int2* dip_ent = nullptr; int dip_nent = 0; cplx* dip_partial = nullptr;  // dipole entries and chunk sums
@@ -217,24 +231,17 @@ struct Ctx {
   double* h1_partial = nullptr;
   unsigned* h1_ticket = nullptr;
   int* h1_flags = nullptr;  // [0] done, [1] cycles of the last application, [2] cycle counter of a graph loop
-  cudaStream_t st4 = nullptr;  // stream on which graph-loop bodies are captured
   // phase timing (off during graph capture)
   bool profile = false;
-  int mixed = 0;  // 1: the mean field's pair-density and pair-potential transforms in split TF32 (tcgen05)
   // persistent split-TF32 plans of the two pair-field transforms (built on the first switch to mixed)
   std::vector<LegGemmBatch> h_b_rho, h_b_W;
   LegTcPlan tc_rho, tc_W;
   bool tc_built = false, tc_ok_rho = false, tc_ok_W = false;
-  int mf_external = 0;  // 1: the RHS takes W and int2e as they stand (the learned form's predicted stages)
-  // learned form: predictor data path (predictor.cu), the caller's network, and the captured steps
+  // learned form: predictor data path (predictor.cu) and the captured steps
   LpArgs lp{};
   bool lp_alloc = false;
-  MlpInferArgs lp_mi{};
-  bool lp_has_net = false;
   float* lp_out = nullptr;
   int* lp_mi_status = nullptr;
-  int lp_use_net = 0;
-  double lp_bound = 1e-6;
   cplx* lp_save = nullptr;  // the state at the start of a judged window (orbitals, then CI)
   cudaGraphExec_t lp_exec[3] = {nullptr, nullptr, nullptr};  // E, H, P steps
   long lp_exec_launch[3] = {0, 0, 0};
@@ -246,11 +253,8 @@ struct Ctx {
   double lp_key[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   double lp_t_end = -1e300;
   int lp_mode = 0, lp_backoff = 0, lp_plain_left = 0;
-  int lp_screen = 1;  // 1: predicted windows only after a fill window whose judge values pass
   cudaEvent_t ev[16] = {};
-  cudaStream_t st2 = nullptr;  // side stream of the CI RDM chain (process lifetime, like st)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  cudaStream_t st3 = nullptr;  // side stream of the one-body stencil and of int2e
   cudaEvent_t ev_ob_fork = nullptr, ev_ob_join = nullptr, ev_i2_fork = nullptr, ev_i2_join = nullptr;
   cudaEvent_t ev_sig_fork = nullptr, ev_sig_join = nullptr;
   int nev = 0;
@@ -2407,6 +2411,11 @@ int etdrk4_step(Ctx& c, cplx* y_orb, cplx* y_cic, double dt, int maxcyc, double 
 // the learned form: split2 with the stage mean fields predicted from the
 // history of exact step-start mean fields (predictor.cu)
 // ---------------------------------------------------------------------------
+void lp_net_bufs(Ctx& c) {  // this context's side of the network's arguments
+  MlpInferArgs& a = c.lp_mi;
+  a.rows = c.lp.nu; a.x = c.lp.feat; a.ldx = 32; a.y = c.lp_out; a.ldy = 8;
+  a.status = c.lp_mi_status;
+}
 int lp_setup(Ctx& c) {
   if (mlp_infer_prepare()) return ST_CUDA;
   if (c.lp_alloc) return 0;
@@ -2427,6 +2436,7 @@ int lp_setup(Ctx& c) {
   c.lp_out = dalloc<float>((size_t)a.nu * 8);
   a.net_out = c.lp_out;
   c.lp_mi_status = dalloc<int>(1);
+  lp_net_bufs(c);
   std::vector<int> kind(c.npair);
   for (int p = 0; p < c.npair; ++p) kind[p] = c.pb[p] < c.nfcore ? 2 : (c.pa[p] == c.pb[p] ? 0 : 1);
   a.pair_kind = dupload(kind);
@@ -2906,8 +2916,35 @@ void hprod_bind_(double* ene_fcore, double* ene_dcore, double* ene_core, double*
   (void)dip_exp; (void)vel_exp; (void)acc_exp; (void)projhigh; (void)cutoff;
 }
 
+static void ens_forget(int id);
+// everything the current context holds on the device beyond its streams: captured steps, events, memory
+static void release(Ctx& c) {
+  ens_forget(g_cur);
+  for (auto& ge : c.graph_exec) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
+  for (auto& ge : c.lp_exec) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
+  for (cudaStream_t q : {c.st, c.st2, c.st3}) if (q) cudaStreamSynchronize(q);
+  rhs_free(c);
+  for (cudaEvent_t e : {c.ev_fork, c.ev_join, c.ev_ob_fork, c.ev_ob_join, c.ev_i2_fork, c.ev_i2_join, c.ev_sig_fork,
+                        c.ev_sig_join})
+    if (e) cudaEventDestroy(e);
+  for (cudaEvent_t& e : c.ev) if (e) { cudaEventDestroy(e); e = nullptr; }
+  for (void* p : c.allocs) cudaFree(p);
+  c.allocs.clear();
+}
+// a second init of a context: every buffer, factor and captured step was sized or built from the tables bound
+// before, so the context starts over with what is bound now (and the restart state, which is the caller's)
+static void renew(Ctx& c) {
+  release(c);
+  Ctx fresh;
+  static_cast<Bound&>(fresh) = std::move(static_cast<Bound&>(c));
+  fresh.rk.reset_orb = c.rk.reset_orb;
+  fresh.rk.reset_cic = c.rk.reset_cic;
+  c = std::move(fresh);
+}
+
 void hprod_init_(void) {
   Ctx& c = ctx();
+  if (c.initialized || !c.allocs.empty()) renew(c);
   if (!c.have_rad || !c.have_sph || !c.have_bas) { c.status |= ST_CONFIG; return; }
   if (c.nfun > 16) { c.status |= ST_CONFIG; return; }
   // the active-active rotations of ORMAS with several subspaces
@@ -2923,15 +2960,10 @@ void hprod_init_(void) {
     if (!lib_stream3) make_stream(&lib_stream3, false);
     c.st = lib_stream; c.st2 = lib_stream2; c.st3 = lib_stream3; c.st4 = lib_stream4;
   } else if (!c.st) {
-    // an ensemble job: its own streams, so that a graph captured over several
-    // jobs (forked from one stream) has no edges between them
+    // an ensemble job: its own streams, so that the jobs' step graphs run side by side
     make_stream(&c.st, true); make_stream(&c.st2, false); make_stream(&c.st3, false); make_stream(&c.st4, true);
     c.own_streams = true;
   }
-  // a second init of a context: what was captured over the old buffers goes
-  if (c.st) cudaStreamSynchronize(c.st);
-  rhs_free(c);
-  c.epoch = ++g_epoch;
   for (cudaEvent_t* e : {&c.ev_fork, &c.ev_join, &c.ev_ob_fork, &c.ev_ob_join, &c.ev_i2_fork, &c.ev_i2_join,
                          &c.ev_sig_fork, &c.ev_sig_join})
     cudaEventCreateWithFlags(e, cudaEventDisableTiming);
@@ -2946,6 +2978,7 @@ void hprod_init_(void) {
   if (rc) { c.status |= ST_CUDA; return; }
   c.rhs = new RhsGraph();
   c.rhs->io = dalloc<RhsIo>(1);
+  if (c.mixed) build_tc_plans(c);
   c.initialized = true;
 }
 
@@ -3038,23 +3071,10 @@ void hprod_htot_(const double* dtime, const double* lfield, const double* wfn, c
   if (c.p_ene_tot) *c.p_ene_tot = c.h_ene[4];
 }
 
-static void ens_forget(int id);
 void hprod_final_(void) {
   if (!g) return;
   Ctx& c = *g;
-  ens_forget(g_cur);
-  for (auto& ge : c.graph_exec) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
-  for (auto& ge : c.lp_exec) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
-  if (c.st) cudaStreamSynchronize(c.st);
-  rhs_free(c);
-  if (c.st2) cudaStreamSynchronize(c.st2);
-  if (c.st3) cudaStreamSynchronize(c.st3);
-  for (cudaEvent_t e : {c.ev_fork, c.ev_join, c.ev_ob_fork, c.ev_ob_join, c.ev_i2_fork, c.ev_i2_join, c.ev_sig_fork,
-                        c.ev_sig_join})
-    if (e) cudaEventDestroy(e);
-  for (cudaEvent_t& e : c.ev) if (e) { cudaEventDestroy(e); e = nullptr; }
-  for (void* p : c.allocs) cudaFree(p);
-  c.allocs.clear();
+  release(c);
   if (c.own_streams)
     for (cudaStream_t q : {c.st, c.st2, c.st3, c.st4}) if (q) cudaStreamDestroy(q);
   delete g;
@@ -3640,8 +3660,8 @@ int td1c_gpu_set_learned(int depth, const int* sizes, const float* const* W, con
   if (depth > MLP_MAXDEPTH || !sizes || !W || !b || !pack || sizes[0] != 32 || sizes[depth] != 8) return ST_CONFIG;
   MlpInferArgs& a = c.lp_mi;
   a = MlpInferArgs{};
-  a.depth = depth; a.rows = c.lp.nu; a.nin = sizes[0]; a.x = c.lp.feat; a.ldx = 32; a.y = c.lp_out; a.ldy = 8;
-  a.status = c.lp_mi_status;
+  lp_net_bufs(c);
+  a.depth = depth; a.nin = sizes[0];
   unsigned short* p = (unsigned short*)pack;
   for (int k = 0; k < depth; ++k) {
     if (sizes[k + 1] < 1 || sizes[k + 1] > 256) return ST_CONFIG;

@@ -143,3 +143,71 @@ def test_learned_steps_after_another_frozen_core(cuda_ok):
         assert np.array_equal(s.run(h, learned), s.run(h, exact))
     finally:
         h.final()
+
+
+SECOND = {
+    "larger": dict(WL, nfe=15, rmax=28.0, rmask=22.0, lmax1=7, lmax2=14),
+    "other_elements": dict(WL, ndvr=10, nfe=6, rmax=11.0, rmask=8.0),
+    "more_orbitals": dict(W.NE_SMALL, split_type=1),
+}
+
+
+def _ensemble(h, wl, x, c):
+    import ctypes
+
+    def one(t, v):
+        return (t * 1)(v)
+    d = ctypes.c_double
+    rc = h.lib._lib.td1c_gpu_ensemble_split2(1, one(ctypes.c_int, h.ctx_id), one(ctypes.c_void_p, x), one(ctypes.c_void_p, c),
+                                             one(d, 30.0), one(d, 0.004), 3, one(d, wl["fint"]), one(d, wl["wlen"]),
+                                             one(d, wl["numcyc"]), one(d, wl["cep"]), 20, 1e-10, ctypes.byref(d(0.0)))
+    assert rc == 0
+
+
+def _everything(h, wl, orb, cic):
+    """One call of each kind that keeps something in the context."""
+    s, out = _State(orb, cic), {}
+    lf = np.zeros(9)
+    lf[2], lf[5], lf[8] = 0.8, 0.1, 0.8
+    out["htot"] = np.concatenate([v.reshape(-1) for v in h.htot(1.0, lf, orb, cic)])
+    for kind, step in _steps(h).items():
+        out[kind] = s.run(h, step)
+        assert np.array_equal(out[kind], s.run(h, step))
+    out["ensemble"] = s.run(h, lambda x, c: _ensemble(h, wl, x, c))
+    out["dipole"] = np.array([h.dipole_dev(s.x.data_ptr(), s.c.data_ptr())])
+    out["dipole3"] = np.concatenate(h.dipole3_dev(s.x.data_ptr(), s.c.data_ptr(), lf))
+    out["learned"] = s.run(h, lambda x, c: h.split2_learned_dev(x, c, 30.0, 0.004, 12))
+    for mode in (1, 3):
+        h.set_mixed(mode)
+        out["mixed%d" % mode] = s.run(h, _steps(h)["split2"])
+    h.set_time_kind(0)
+    out["relax"] = s.run(h, lambda x, c: h.relax_etdrk2_dev(x, c, 0.01, 3))
+    h.set_time_kind(1)
+    h.set_mixed(0)
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", sorted(SECOND))
+def test_second_init_of_a_context(cuda_ok, name):
+    """The default context bound and initialised again without hprod_final_, to other sizes and back: every call
+    does what it does in a fresh context, and the settings made before the second init hold."""
+    refs = {}
+    for key, wl in (("first", WL), ("second", SECOND[name])):
+        h, orb, cic = _context(wl, new_context=True)
+        try:
+            refs[key] = _everything(h, wl, orb, cic)
+        finally:
+            h.final()
+    h = None
+    try:
+        for key, wl in (("first", WL), ("second", SECOND[name]), ("first", WL)):
+            h, orb, cic = _context(wl)
+            got = _everything(h, wl, orb, cic)
+            for k, v in refs[key].items():
+                assert np.array_equal(got[k], v), (key, k)
+        h.set_mixed(1)  # the tensor-core plans are built at once, or by the next init
+        h, orb, cic = _context(WL)
+        assert np.array_equal(_State(orb, cic).run(h, _steps(h)["split2"]), refs["first"]["mixed1"])
+    finally:
+        h.final()
