@@ -131,7 +131,9 @@ int td1c_gpu_ci_tables(unsigned* stra, unsigned* strb, int* detoff, int* afirst,
 /* energies of the last htot: ene_fcore, ene_dcore, ene_core, ene_act, ene_tot */
 int td1c_gpu_energies(double* ene5);
 /* RHS on device-resident buffers (no host copies), on the library stream.
- * lfield is a host array of 9 doubles. */
+ * lfield is a host array of 9 doubles.  d_cic, d_hwfn and d_hcic stand on
+ * 16-byte boundaries (a complex double); d_wfn may stand on any 8-byte one
+ * (from a 16-byte one repeated calls replay a captured right-hand side). */
 int td1c_gpu_htot_dev(double dtime, const double* lfield, const void* d_wfn, const void* d_cic,
                       void* d_hwfn, void* d_hcic);
 /* Copy a named device intermediate of the last htot to host memory

@@ -1732,6 +1732,8 @@ int rhs_call(Ctx& c, RhsGraph& g, const double* lf, const RhsIo& io, double dtim
   cudaStreamIsCapturing(c.st, &cst);
   auto eager = [&]() { return run_htot(c, c.lfield, io.wfn, io.cic, io.hwfn, io.hcic, dtime); };
   if (cst != cudaStreamCaptureStatusNone || c.profile) return eager();
+  // the replayed transform of the caller's buffer reads it in 16 bytes, the eager copy takes any alignment
+  if (reinterpret_cast<uintptr_t>(io.wfn) % sizeof(cplx)) return eager();
   if (g.exec && !(g.key == key)) {
     cudaGraphExecDestroy(g.exec);
     g.exec = nullptr;

@@ -211,3 +211,31 @@ def test_second_init_of_a_context(cuda_ok, name):
         assert np.array_equal(_State(orb, cic).run(h, _steps(h)["split2"]), refs["first"]["mixed1"])
     finally:
         h.final()
+
+
+@pytest.mark.gpu
+def test_repeated_rhs_of_a_state_on_an_8_byte_boundary(cuda_ok):
+    """The orbitals may start on any 8-byte boundary, in the first call and in every repeated one."""
+    import torch
+    h, orb, cic = _context()
+    try:
+        x = torch.from_numpy(orb.reshape(-1).view(np.float64).copy()).cuda()
+        odd = torch.zeros(x.numel() + 1, dtype=torch.float64, device="cuda")
+        odd[1:] = x
+        assert x.data_ptr() % 16 == 0 and odd[1:].data_ptr() % 16 == 8
+        c = torch.from_numpy(cic.copy()).cuda()
+        y, yc = torch.empty(orb.size, dtype=torch.complex128, device="cuda"), torch.empty_like(c)
+        lf = np.zeros(9)
+        lf[2] = lf[8] = 0.8
+
+        def call(t):
+            y.fill_(float("nan"))
+            torch.cuda.synchronize()
+            h.htot_dev(1.0, lf, t.data_ptr(), c.data_ptr(), y.data_ptr(), yc.data_ptr())
+            h.sync()
+            return y.cpu().numpy()
+        want = call(x)
+        for t in (odd[1:], odd[1:], odd[1:], x, x, x, odd[1:], x):
+            assert np.array_equal(call(t), want)
+    finally:
+        h.final()
