@@ -207,7 +207,8 @@ __global__ void __launch_bounds__(128) ci_sigma_kernel(CiArgs a) {
   const double e = *a.ene_act;
   cplx c = a.io ? a.io->cic[J] : a.cic[J];
   sig = csub(sig, cscale(c, e));
-  cplx fac = a.icomp == 1 ? mkc(0.0, -a.dtime) : mkc(-a.dtime, 0.0);
+  const double dt = a.io ? a.io->dtime : a.dtime;
+  cplx fac = a.icomp == 1 ? mkc(0.0, -dt) : mkc(-dt, 0.0);
   const cplx k = cmul(sig, fac);
   if (a.rk.stage == 0) (a.io ? a.io->hcic : a.sigma)[J] = k;
   else rk_put(a.rk, J, k);

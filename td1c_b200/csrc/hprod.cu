@@ -613,6 +613,7 @@ __global__ void invden_kernel(int nact, int need_rr, const cplx* __restrict__ de
 struct SmallArgs {
   int nfun, nfcore, ndcore, nact, ncore, nelact, icomp;
   double dtime, ene_fcore;
+  const RhsIo* io;  // non-null: dtime is its own
   const int* mval;
   const int* ent_index;  // [5][nfun][nfun]
   const cplx* res;       // orbdots results
@@ -682,7 +683,8 @@ __global__ void __launch_bounds__(256) smallmat_kernel(SmallArgs a) {
     a.ene[4] = a.ene_fcore + ed + ene_act;
   }
   // X matrix
-  const cplx tfac = a.icomp == 0 ? mkc(a.dtime, 0) : mkc(0, a.dtime);
+  const double dt = a.io ? a.io->dtime : a.dtime;
+  const cplx tfac = a.icomp == 0 ? mkc(dt, 0) : mkc(0, dt);
   for (int e = tid; e < nf * nf; e += blockDim.x) a.xmat[e] = mkc(0, 0);
   __syncthreads();
   // _fc: X(j,i) = tfac (<(h0+h1) phi_j|phi_i> + <phi_j|(g+v2) phi_i>), j frozen, i dynamic
@@ -767,7 +769,8 @@ __global__ void __launch_bounds__(512) dtorb_kernel(size_t nb, int nfun, int nfc
     if (rk.stage == 0) hwfn[t] = mkc(0, 0);
     return;
   }
-  const cplx tf2 = icomp == 0 ? mkc(-dtime, 0) : mkc(0, -dtime);
+  const double dt = io ? io->dtime : dtime;
+  const cplx tf2 = icomp == 0 ? mkc(-dt, 0) : mkc(0, -dt);
   cplx o = cmul(h, tf2);
   const int mi = sm[i];
   for (int j = 0; j < nfun; ++j)
@@ -776,7 +779,7 @@ __global__ void __launch_bounds__(512) dtorb_kernel(size_t nb, int nfun, int nfc
   else rk_put(rk, t, o);
 }
 
-// lfield[9] (and the caller's buffers) by value into device memory
+// lfield[9] (and the caller's buffers and time step) by value into device memory
 struct Lf9 { double v[9]; };
 __global__ void lfield_kernel(Lf9 f, double* __restrict__ out, RhsIo io, RhsIo* io_out) {
   if (threadIdx.x < 9) out[threadIdx.x] = f.v[threadIdx.x];
@@ -1533,7 +1536,7 @@ int chk(const char* what, int rc) {
 
 // d_lf: device lfield[9]; wfn/cic device inputs (wfn null: the orbitals already stand in c.orb);
 // hwfn/hcic device outputs, or (rk) the RK4 stage that takes the value of the orbitals and of the CI vector,
-// or (io) all four buffers as they stand in the device copy
+// or (io) all four buffers and dtime as they stand in the device copy
 int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cplx* hwfn, cplx* hcic, double dtime,
              const RkStage* rk = nullptr, const RkStage* rk_ci = nullptr, const RhsIo* io = nullptr) {
   cudaStream_t st = c.st;
@@ -1671,7 +1674,7 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
   mark();  // end int2e (its wait for the third stream)
   SmallArgs sa{};
   sa.nfun = c.nfun; sa.nfcore = c.nfcore; sa.ndcore = c.ndcore; sa.nact = c.nact; sa.ncore = c.ncore; sa.nelact = c.nelact;
-  sa.icomp = c.icomp; sa.dtime = dtime; sa.ene_fcore = c.ene_fcore; sa.mval = c.d_mval; sa.ent_index = c.ent_index;
+  sa.icomp = c.icomp; sa.dtime = dtime; sa.io = io; sa.ene_fcore = c.ene_fcore; sa.mval = c.d_mval; sa.ent_index = c.ent_index;
   sa.res = c.od.result; sa.den1 = c.den1; sa.den2 = c.den2; sa.rrden = c.rrden; sa.int1e = c.int1e; sa.int2e = c.int2e;
   sa.xmat = c.xmat; sa.ene = c.ene;
   smallmat_kernel<<<1, 256, 0, st>>>(sa);
@@ -1704,14 +1707,12 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
 // One RHS on the caller's device buffers.  An eager RHS is some twenty launches and events on three
 // streams, more host time than the small workloads' kernels take (us a call among others, eager and replayed: an
 // 8 x 8 box 46.0 and 15.2, He 45.7 and 22.3, Ne's 445 either way); the second call in a row with the same
-// settings captures it once (reading the buffers and the field from device memory, so the capture holds
-// for any buffers), and later calls replay it.  The capture goes with the context, or when a setting changes.
+// settings captures it once (reading the buffers, the field and the time step from device memory, so the capture
+// holds for any of them), and later calls replay it.  The capture goes with the context, or when a setting changes.
 struct RhsKey {
-  double dtime = 0, ene_fcore = 0;
+  double ene_fcore = 0;
   std::array<int, kSettings> set{};
-  bool operator==(const RhsKey& k) const {
-    return memcmp(&dtime, &k.dtime, sizeof(double)) == 0 && memcmp(&ene_fcore, &k.ene_fcore, sizeof(double)) == 0 && set == k.set;
-  }
+  bool operator==(const RhsKey& k) const { return memcmp(&ene_fcore, &k.ene_fcore, sizeof(double)) == 0 && set == k.set; }
 };
 struct RhsGraph {
   cudaGraphExec_t exec = nullptr;
@@ -1720,17 +1721,17 @@ struct RhsGraph {
   bool have_last = false;
   long launches = 0;
 };
-int rhs_call(Ctx& c, RhsGraph& g, const double* lf, const RhsIo& io, double dtime) {
+int rhs_call(Ctx& c, RhsGraph& g, const double* lf, const RhsIo& io) {
   if (!g.io) g.io = dalloc<RhsIo>(1);
   Lf9 f;
   for (int k = 0; k < 9; ++k) f.v[k] = lf[k];
   lfield_kernel<<<1, 32, 0, c.st>>>(f, c.lfield, io, g.io);
   c.launches++;
   RhsKey key;
-  key.dtime = dtime; key.ene_fcore = c.ene_fcore; key.set = settings(c);
+  key.ene_fcore = c.ene_fcore; key.set = settings(c);
   cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(c.st, &cst);
-  auto eager = [&]() { return run_htot(c, c.lfield, io.wfn, io.cic, io.hwfn, io.hcic, dtime); };
+  auto eager = [&]() { return run_htot(c, c.lfield, io.wfn, io.cic, io.hwfn, io.hcic, io.dtime); };
   if (cst != cudaStreamCaptureStatusNone || c.profile) return eager();
   // the replayed transform of the caller's buffer reads it in 16 bytes, the eager copy takes any alignment
   if (reinterpret_cast<uintptr_t>(io.wfn) % sizeof(cplx)) return eager();
@@ -1746,7 +1747,7 @@ int rhs_call(Ctx& c, RhsGraph& g, const double* lf, const RhsIo& io, double dtim
     const long l0 = c.launches;
     cudaGraph_t graph = nullptr;
     if (cudaStreamBeginCapture(c.st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return ST_CUDA;
-    const int rc = run_htot(c, c.lfield, nullptr, nullptr, nullptr, nullptr, dtime, nullptr, nullptr, g.io);
+    const int rc = run_htot(c, c.lfield, nullptr, nullptr, nullptr, nullptr, 0.0, nullptr, nullptr, g.io);
     const cudaError_t e = cudaStreamEndCapture(c.st, &graph);
     g.launches = c.launches - l0;
     c.launches = l0;
@@ -1765,7 +1766,7 @@ int rhs_call(Ctx& c, RhsGraph& g, const double* lf, const RhsIo& io, double dtim
 }
 int rhs_call(Ctx& c, const double* lf, const cplx* wfn, const cplx* cic, cplx* hwfn, cplx* hcic, double dtime) {
   if (!c.rhs) c.rhs = new RhsGraph();
-  return rhs_call(c, *c.rhs, lf, RhsIo{wfn, cic, hwfn, hcic}, dtime);
+  return rhs_call(c, *c.rhs, lf, RhsIo{wfn, cic, hwfn, hcic, dtime});
 }
 void rhs_free(Ctx& c) {
   if (c.rhs && c.rhs->exec) cudaGraphExecDestroy(c.rhs->exec);

@@ -17,11 +17,12 @@
 
 namespace td1c {
 
-// The caller's buffers of one RHS, in device memory: a captured RHS reads them from here, so one capture
-// serves any buffers (the field stands in the context's lfield)
+// The caller's buffers and time step of one RHS, in device memory: a captured RHS reads them from here, so one
+// capture serves any (the field stands in the context's lfield)
 struct RhsIo {
   const cplx *wfn, *cic;
   cplx *hwfn, *hcic;
+  double dtime;
 };
 
 // What an RHS does with its value k: writes it out (stage 0), or makes it stage 1 .. 4 of an RK4 step
@@ -331,7 +332,7 @@ struct CiArgs {
   const double* ene_act;  // device scalar
   double dtime; int icomp;
   RkStage rk;             // stage > 0: sigma goes into an RK4 stage of the CI vector instead of out
-  const RhsIo* io = nullptr;  // non-null: the CI vector and sigma are its buffers
+  const RhsIo* io = nullptr;  // non-null: the CI vector, sigma and dtime are its own
 };
 int launch_ci_dvec(const CiArgs& a, int maxsec, cudaStream_t st);
 int launch_ci_rdm(const CiArgs& a, cudaStream_t st);

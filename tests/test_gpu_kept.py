@@ -239,3 +239,45 @@ def test_repeated_rhs_of_a_state_on_an_8_byte_boundary(cuda_ok):
             assert np.array_equal(call(t), want)
     finally:
         h.final()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("wl", [W.HE_SMALL, W.MIXED_SMALL], ids=lambda w: w["name"])
+def test_rhs_of_changing_time_steps_is_replayed(cuda_ok, wl):
+    """A time step that changes every two calls costs no capture: the calls take as long as with one time step
+    (a capture and an instantiation take ten times as long as a call; the best of several rounds on both sides)."""
+    import time
+    import torch
+    h, orb, cic = _context(wl)
+    try:
+        x, c = torch.from_numpy(orb.reshape(-1).copy()).cuda(), torch.from_numpy(cic.copy()).cuda()
+        y, yc = torch.empty_like(x), torch.empty_like(c)
+        lf = np.zeros(9)
+        lf[2] = lf[8] = 0.8
+
+        def call(dt):
+            h.htot_dev(dt, lf, x.data_ptr(), c.data_ptr(), y.data_ptr(), yc.data_ptr())
+
+        def best(dts):
+            out = []
+            for _ in range(7):
+                h.sync()
+                t = time.perf_counter()
+                for dt in dts:
+                    call(dt)
+                h.sync()
+                out.append(time.perf_counter() - t)
+            return min(out)
+        torch.cuda.synchronize()
+        one = best([1.0] * 24)
+        two = best([0.25, 0.25, 0.5, 0.5] * 6)
+        assert two < 3.0 * one, (one, two)
+        want = {}
+        for dt in (0.25, 1.0, 0.5):
+            call(dt)
+            h.sync()
+            want[dt] = (y.cpu().numpy(), yc.cpu().numpy())
+        for dt in (0.25, 0.5):  # powers of two: exact multiples
+            assert np.array_equal(want[dt][0], dt * want[1.0][0]) and np.array_equal(want[dt][1], dt * want[1.0][1])
+    finally:
+        h.final()
