@@ -12,14 +12,17 @@
 // context).  Ne's right-hand side from host buffers: 2700 -> 1480 us (the RHS itself 450).
 // From 512 KB on: a host call of 5 orbitals, us through the ring and on the plain path,
 // by the state's size: 75 KB 149 and 137, 249 KB 161 and 156, 412 KB 177 and 182, 749 KB
-// 200 and 233, 1.5 MB 280 to 320 and 335 to 355.  A copy that finds the ring in use by another thread, a forked
-// child, a second device, or a failed allocation takes the plain path.
+// 200 and 233, 1.5 MB 280 to 320 and 335 to 355.  Page-locked (or managed) buffers cross the bus as they are, and a
+// copy that finds the ring in use by another thread, a forked child, a second device, or a failed allocation takes
+// the plain path too.
 #include <pthread.h>
+#include <sched.h>
 #include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <thread>
@@ -33,6 +36,16 @@ namespace {
 
 constexpr size_t HC_SLOT = 2u << 20, HC_MIN = 512u << 10, HC_PIECE = 128u << 10;
 constexpr int HC_SLOTS = 4, HC_WORKERS = 7;
+
+// threads that copy, the caller's included: at most one per core the process may run on, or TD1C_HOST_THREADS
+int copy_threads() {
+  int n = HC_WORKERS + 1;
+  cpu_set_t set;
+  if (sched_getaffinity(0, sizeof(set), &set) == 0) n = std::min(n, CPU_COUNT(&set));
+  const char* v = getenv("TD1C_HOST_THREADS");
+  if (v && atoi(v) > 0) n = std::min(HC_WORKERS + 1, atoi(v));
+  return n;
+}
 
 // memcpy by several threads: the caller and the workers take pieces in turn
 class CopyTeam {
@@ -56,7 +69,7 @@ class CopyTeam {
     if (started_) return pid_ == getpid();
     started_ = true;
     pid_ = getpid();
-    const int n = std::min<int>(HC_WORKERS, (int)std::thread::hardware_concurrency() - 1);
+    const int n = copy_threads() - 1;
     try {
       for (int k = 0; k < n; ++k) std::thread([this] { loop(); }).detach();
     } catch (...) {  // fewer workers: the caller takes their pieces
@@ -135,11 +148,23 @@ Ring& ring() {
   return *r;
 }
 
+// whether a copy of n bytes goes through the ring: large, and of pageable memory
+bool staged(const void* host, size_t n) {
+  if (n < HC_MIN) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return at.type == cudaMemoryTypeUnregistered;
+}
+
 }  // namespace
 
-// queue the copy of n host bytes to the device on st; the host buffer is free on return
+// queue the copy of n host bytes to the device on st; a pageable host buffer is free on return, a page-locked one
+// when st is synchronised
 cudaError_t host_to_device(void* dst, const void* src, size_t n, cudaStream_t st) {
-  if (n >= HC_MIN) {
+  if (staged(src, n)) {
     Ring& r = ring();
     std::unique_lock<std::mutex> l(r.m, std::try_to_lock);
     if (l.owns_lock() && r.ready()) {
@@ -160,9 +185,9 @@ cudaError_t host_to_device(void* dst, const void* src, size_t n, cudaStream_t st
 }
 
 // copy n device bytes to the host after the work queued on st; complete on return where the ring was used,
-// else (small copies) when st is synchronised
+// else when st is synchronised
 cudaError_t device_to_host(void* dst, const void* src, size_t n, cudaStream_t st) {
-  if (n >= HC_MIN) {
+  if (staged(dst, n)) {
     Ring& r = ring();
     std::unique_lock<std::mutex> l(r.m, std::try_to_lock);
     if (l.owns_lock() && r.ready()) {
