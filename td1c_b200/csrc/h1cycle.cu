@@ -7,9 +7,9 @@
 // bridge points (a serial chain of 2 nfe complex steps per orbital).  M is a
 // short time step, so the inverse of that tridiagonal matrix falls off fast
 // away from its diagonal: by a factor of 1e-4 to 1e-9 per element.  Here the
-// inverse itself is formed once per factor and its band of half-width w kept,
-// where every entry outside the band is below 2^-64 of the row's diagonal
-// (far below the rounding of the products it would enter); an element's CTA
+// columns of the inverse are formed once per factor and a band of half-width w
+// of it kept, where every entry outside the band is below 2^-64 of the row's
+// diagonal (far below the rounding of the products it would enter); an element's CTA
 // then gets its two bridge values as short dot products with the shares of the
 // 2 w + 2 elements around it, and a whole cycle is one launch, which also
 // decides whether the graph's loop goes on.  A factor whose inverse falls off
@@ -77,9 +77,11 @@ size_t h1c_band_size(int nd) { return (size_t)h1c_mtp(nd) * h1c_ksp(nd) * 32; } 
 // set-up
 // ---------------------------------------------------------------------------
 // per element: P (derivative; the diagonal only at the points the element owns, i.e. not at its right
-// bridge) and T (kinetic off-diagonal, l >= 1) over the element's points, in fragment order
-__global__ void h1c_band_kernel(int nfe, int nd, int Nr, const double* __restrict__ radp, const double* __restrict__ radk0,
-                                double* __restrict__ pf, double* __restrict__ tf) {
+// bridge) and T (kinetic off-diagonal, l >= 1) over the element's points, in fragment order; 1 / r
+__global__ void h1c_band_kernel(int nfe, int nd, int Nr, const double* __restrict__ xrad, const double* __restrict__ radp,
+                                const double* __restrict__ radk0, double* __restrict__ rinv, double* __restrict__ pf,
+                                double* __restrict__ tf) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k <= Nr + 1; k += gridDim.x * blockDim.x) rinv[k] = k ? 1.0 / xrad[k] : 0.0;
   const int e = blockIdx.x, mt = h1c_mtp(nd), ks = h1c_ksp(nd), bw = 2 * nd + 1;
   for (int i = threadIdx.x; i < mt * ks * 32; i += blockDim.x) {
     const int lane = i & 31, k = (i >> 5) % ks, t = (i >> 5) / ks;
@@ -116,61 +118,69 @@ __global__ void h1c_af_kernel(H1Fac f) {
   }
 }
 
-// per (l, column): a column of the inverse of the bridge matrix from its pivoted LU
-// (ZGTTRS algorithm), stored as sinv[l][row][column]
-__global__ void h1c_sinv_kernel(H1Fac f) {
-  const int l = blockIdx.x, nb = f.nb, c = blockIdx.y * blockDim.x + threadIdx.x;
-  if (c >= nb) return;
-  const cplx *dl = f.tdl + (size_t)l * nb, *di = f.tdi + (size_t)l * nb, *du = f.tdu + (size_t)l * nb, *du2 = f.tdu2 + (size_t)l * nb;
-  const int* ip = f.tpiv + (size_t)l * nb;
-  cplx* x = f.sinv + (size_t)l * nb * nb + c;  // x[i * nb]
-  cplx cur = mkc(c == 0 ? 1.0 : 0.0, 0.0);
-  for (int i = 0; i + 1 < nb; ++i) {
-    const cplx nxt = mkc(c == i + 1 ? 1.0 : 0.0, 0.0);
-    if (ip[i] == i) {
-      x[(size_t)i * nb] = cur;
-      cur = csub(nxt, cmul(dl[i], cur));
-    } else {
-      x[(size_t)i * nb] = nxt;
-      cur = csub(cur, cmul(dl[i], nxt));
+// The inverse of the bridge matrix, a CTA per l and a thread per column (every ncol-th one), from its pivoted LU
+// (ZGTTRS algorithm), with the thread's column in the scratch x[l][row][thread].  The band goes to
+// sinv[l][row][H1C_BW]; then *w = the largest |row - column| of an entry above 2^-64 of its row's diagonal.  The
+// whole inverse is not kept: its size goes with the square of the number of elements.
+__global__ void h1c_sinv_kernel(H1Fac f, cplx* __restrict__ scratch, int ncol, int* w) {
+  const int l = blockIdx.x, nb = f.nb, j = threadIdx.x;
+  const cplx *__restrict__ dl = f.tdl + (size_t)l * nb, *__restrict__ di = f.tdi + (size_t)l * nb;
+  const cplx *__restrict__ du = f.tdu + (size_t)l * nb, *__restrict__ du2 = f.tdu2 + (size_t)l * nb;
+  const int* __restrict__ ip = f.tpiv + (size_t)l * nb;
+  cplx* x = scratch + (size_t)l * nb * ncol + j;  // x[i * ncol]
+  cplx* S = f.sinv + (size_t)l * nb * H1C_BW + H1C_WMAX;  // S(r, c) at [r * H1C_BW + c - r]
+  auto column = [&](int c) {
+    cplx cur = mkc(c == 0 ? 1.0 : 0.0, 0.0);
+#pragma unroll 8
+    for (int i = 0; i + 1 < nb; ++i) {
+      const cplx nxt = mkc(c == i + 1 ? 1.0 : 0.0, 0.0), m = __ldg(dl + i);
+      const bool sw = __ldg(ip + i) != i;
+      const cplx a = sw ? nxt : cur, b = sw ? cur : nxt;
+      x[(size_t)i * ncol] = a;
+      cur = csub(b, cmul(m, a));
     }
+    cplx x1 = cmul(cur, di[nb - 1]), x2 = mkc(0, 0);
+    x[(size_t)(nb - 1) * ncol] = x1;
+#pragma unroll 8
+    for (int i = nb - 2; i >= 0; --i) {
+      cplx v = csub(x[(size_t)i * ncol], cmul(__ldg(du + i), x1));
+      if (i + 2 < nb) v = csub(v, cmul(__ldg(du2 + i), x2));
+      v = cmul(v, __ldg(di + i));
+      x[(size_t)i * ncol] = v;
+      x2 = x1;
+      x1 = v;
+    }
+  };
+  for (int c = j; c < nb && j < ncol; c += ncol) {
+    column(c);
+    for (int i = max(0, c - H1C_WMAX); i <= min(nb - 1, c + H1C_WMAX); ++i) S[(size_t)i * H1C_BW + c - i] = x[(size_t)i * ncol];
   }
-  cplx x1 = cmul(cur, di[nb - 1]), x2 = mkc(0, 0);
-  x[(size_t)(nb - 1) * nb] = x1;
-  for (int i = nb - 2; i >= 0; --i) {
-    cplx v = csub(x[(size_t)i * nb], cmul(du[i], x1));
-    if (i + 2 < nb) v = csub(v, cmul(du2[i], x2));
-    v = cmul(v, di[i]);
-    x[(size_t)i * nb] = v;
-    x2 = x1;
-    x1 = v;
-  }
-}
-
-// *w = the largest |row - column| of an entry above 2^-64 of its row's diagonal
-__global__ void h1c_width_kernel(H1Fac f, int* w) {
-  const int nb = f.nb, l = blockIdx.x;
-  const cplx* S = f.sinv + (size_t)l * nb * nb;
+  __syncthreads();
   int far = 0;
-  for (int i = threadIdx.x; i < nb * nb; i += blockDim.x) {
-    const int r = i / nb, c = i % nb, d = r < c ? c - r : r - c;
-    if (d <= far) continue;
-    const cplx v = S[i], g = S[(size_t)r * nb + r];
-    if (!(fabs(v.x) + fabs(v.y) <= 0x1p-64 * (fabs(g.x) + fabs(g.y)))) far = d;
+  for (int c = j; c < nb && j < ncol; c += ncol) {
+    if (nb > ncol) column(c);  // else the column still stands in x
+#pragma unroll 4
+    for (int i = 0; i < nb; ++i) {
+      const int d = i < c ? c - i : i - c;
+      const cplx v = x[(size_t)i * ncol], g = S[(size_t)i * H1C_BW];
+      if (d > far && !(fabs(v.x) + fabs(v.y) <= 0x1p-64 * (fabs(g.x) + fabs(g.y)))) far = d;
+    }
   }
   if (far) atomicMax(w, far);
 }
 
-int launch_h1c_bands(int nfe, int nd, int Nr, const double* radp, const double* radk0, double* pf, double* tf, cudaStream_t st) {
-  h1c_band_kernel<<<nfe, 128, 0, st>>>(nfe, nd, Nr, radp, radk0, pf, tf);
+int launch_h1c_bands(int nfe, int nd, int Nr, const double* xrad, const double* radp, const double* radk0, double* rinv,
+                     double* pf, double* tf, cudaStream_t st) {
+  h1c_band_kernel<<<nfe, 128, 0, st>>>(nfe, nd, Nr, xrad, radp, radk0, rinv, pf, tf);
   return (int)cudaGetLastError();
 }
 int launch_h1c_setup(const H1Fac& f, int* w, cudaStream_t st) {
-  h1c_af_kernel<<<dim3(f.nfe, f.L1), 128, 0, st>>>(f);
   if (f.nb > 0) {
-    h1c_sinv_kernel<<<dim3(f.L1, (f.nb + 63) / 64), 64, 0, st>>>(f);
-    h1c_width_kernel<<<f.L1, 256, 0, st>>>(f, w);
+    // A' is formed last: its place, h1c_af_size >= 32 columns of it, is the scratch
+    const int ncol = std::min({f.nb, (int)h1c_af_size(f.nd), 512});
+    h1c_sinv_kernel<<<f.L1, (ncol + 31) / 32 * 32, 0, st>>>(f, f.af, ncol, w);
   }
+  h1c_af_kernel<<<dim3(f.nfe, f.L1), 128, 0, st>>>(f);
   return (int)cudaGetLastError();
 }
 
@@ -301,7 +311,7 @@ __global__ void __launch_bounds__(H1C_NT, 3) h1c_kernel(H1CycArgs a) {
       for (int q = tid; q < 2 * bwd; q += H1C_NT) {
         const int side = q >= bwd, d = q - side * bwd - w, b = e - 1 + side;
         const bool ok = lok && b >= 0 && b < nb && b + d >= 0 && b + d < nb;
-        h1c_cp16(SI + lq * 2 * bwd + q, F.sinv + (ok ? ((size_t)l * nb + b) * nb + b + d : 0), ok);
+        h1c_cp16(SI + lq * 2 * bwd + q, F.sinv + (ok ? ((size_t)l * nb + b) * H1C_BW + H1C_WMAX + d : 0), ok);
       }
     }
 #pragma unroll
@@ -569,7 +579,8 @@ bool h1c_fits(int nd, int nfun, int w, int igauge) {
   if (w < 0 || w > H1C_WMAX || nd < 2 || nd > 20 || nfun > 16) return false;
   for (int mode = 0; mode < 3; ++mode)
     if (H1CSmem{nd, nfun, w, mode, igauge == 1}.bytes() > 220 * 1024) return false;
-  return nfun * nd <= H1C_TPR * H1C_NT;
+  static_assert(16 * 20 <= H1C_TPR * H1C_NT, "a thread holds H1C_TPR values of torb");
+  return true;
 }
 
 int launch_h1c(const H1CycArgs& a, int mode, cudaStream_t st) {

@@ -1888,20 +1888,29 @@ void pulse_lfield(const Pulse& p, double t, double* lf) {
 // one-body propagators (h1prop.cu): factor cache and the application of
 // h1itr_prop / dpade_prod to the orbitals of a device state
 // ---------------------------------------------------------------------------
+// several arrays in one allocation, each on a 256-byte boundary
+struct Pool {
+  std::vector<std::pair<void**, size_t>> part;  // pointer, offset
+  size_t bytes = 0;
+  template <class T>
+  void add(T** p, size_t n) {
+    part.push_back({reinterpret_cast<void**>(p), bytes});
+    bytes += (n * sizeof(T) + 255) / 256 * 256;
+  }
+  bool allocate() {
+    char* base = dalloc<char>(bytes);
+    for (auto& q : part) *q.first = base ? base + q.second : nullptr;
+    return base != nullptr;
+  }
+};
+
 // the tables of the folded passes (h1cycle.cu) beside a new factor; sizes or bands they do not
 // take leave w < 0 (the band's width is read back, so not inside a graph capture)
 int h1c_build(Ctx& c, H1Fac& f) {
   f.w = -1;
   cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(c.st, &cst);
-  if (cst != cudaStreamCaptureStatusNone || !h1c_fits(c.nd, c.nfun, 0, c.igauge)) return 0;
-  const size_t ne = (size_t)c.L1 * f.nfe;
-  if (!f.af) {
-    f.af = dalloc<cplx>(ne * h1c_af_size(c.nd));
-    f.glr = dalloc<cplx>(ne * 2 * f.ni);
-    f.sinv = dalloc<cplx>((size_t)c.L1 * std::max(1, f.nb) * std::max(1, f.nb));
-  }
-  if (!f.af || !f.glr || !f.sinv) return 0;
+  if (cst != cudaStreamCaptureStatusNone || !f.af) return 0;
   int w = 0;
   int* d_w = c.h1_flags + 3;
   cudaMemsetAsync(d_w, 0, sizeof(int), c.st);
@@ -1910,6 +1919,29 @@ int h1c_build(Ctx& c, H1Fac& f) {
   if (rc || cudaStreamSynchronize(c.st) != cudaSuccess) return ST_CUDA;
   f.w = h1c_fits(c.nd, c.nfun, w, c.igauge) ? w : -1;
   return 0;
+}
+
+// the arrays of a factor: with those of the folded passes where the sizes fit and the memory is there,
+// else without (the two-launch passes run)
+bool h1_factor_alloc(Ctx& c, H1Fac& f) {
+  f = H1Fac{};
+  f.nfe = c.nfe; f.nd = c.nd; f.ni = c.nd - 1; f.nb = c.nfe - 1; f.L1 = c.L1;
+  const size_t le = (size_t)c.L1 * f.nfe, ne = le * f.ni, nbt = (size_t)c.L1 * std::max(1, f.nb);
+  for (int folded = h1c_fits(c.nd, c.nfun, 0, c.igauge); folded >= 0; --folded) {
+    Pool p;
+    p.add(&f.ainv, ne * f.ni);
+    for (cplx** q : {&f.gl, &f.gr, &f.vl, &f.vr}) p.add(q, ne);
+    for (cplx** q : {&f.tdl, &f.tdi, &f.tdu, &f.tdu2}) p.add(q, nbt);
+    p.add(&f.tpiv, nbt);
+    if (folded) {
+      p.add(&f.af, le * h1c_af_size(c.nd));
+      p.add(&f.glr, 2 * ne);
+      p.add(&f.sinv, nbt * H1C_BW);
+    }
+    if (p.allocate()) return true;
+    cudaGetLastError();
+  }
+  return false;
 }
 
 int h1_factor(Ctx& c, cplx fac, H1Fac* out) {
@@ -1921,14 +1953,9 @@ int h1_factor(Ctx& c, cplx fac, H1Fac* out) {
     if (std::isnan(c.h1slot[i].cre)) sl = &c.h1slot[i];  // invalidated by a change of T
   if (sl) {
   } else if (c.n_h1 < Ctx::kH1Slots) {
-    sl = &c.h1slot[c.n_h1++];
-    H1Fac& f = sl->f;
-    f.nfe = c.nfe; f.nd = c.nd; f.ni = c.nd - 1; f.nb = c.nfe - 1; f.L1 = c.L1;
-    const size_t ne = (size_t)c.L1 * f.nfe * f.ni, nbt = (size_t)c.L1 * std::max(1, f.nb);
-    f.ainv = dalloc<cplx>(ne * f.ni);
-    f.gl = dalloc<cplx>(ne); f.gr = dalloc<cplx>(ne); f.vl = dalloc<cplx>(ne); f.vr = dalloc<cplx>(ne);
-    f.tdl = dalloc<cplx>(nbt); f.tdi = dalloc<cplx>(nbt); f.tdu = dalloc<cplx>(nbt); f.tdu2 = dalloc<cplx>(nbt);
-    f.tpiv = dalloc<int>(nbt);
+    sl = &c.h1slot[c.n_h1];
+    if (!h1_factor_alloc(c, sl->f)) return ST_CUDA;
+    c.n_h1++;
   } else {
     // all slots taken: rebuild the oldest in place; captured steps may hold its factors
     c.epoch = ++g_epoch;
@@ -1949,20 +1976,20 @@ int h1_bufs(Ctx& c) {
   if (c.h1_z[0]) return 0;
   const size_t nrow = (size_t)c.nfun * c.L1;
   if (c.nfun - c.nfcore > 64 || h1elem_smem(c.nd, c.nfun) > 220 * 1024) return ST_CONFIG;
-  c.h1_z[0] = dalloc<cplx>(nrow * c.nfe * (c.nd - 1));
-  c.h1_z[1] = dalloc<cplx>(nrow * c.nfe * (c.nd - 1));
-  c.h1_cb[0] = dalloc<cplx>(nrow * c.nfe * 2);
-  c.h1_cb[1] = dalloc<cplx>(nrow * c.nfe * 2);
-  c.h1_xb = dalloc<cplx>(nrow * std::max(1, c.nfe - 1));
-  c.h1_partial = dalloc<double>(h1elem_partials(c.nfe, c.L1));
-  c.h1_ticket = dalloc<unsigned>(1);  // zero (dalloc clears)
-  c.h1_flags = dalloc<int>(4);
-  c.h1_pf = dalloc<double>((size_t)c.nfe * h1c_band_size(c.nd));
-  c.h1_tf = dalloc<double>((size_t)c.nfe * h1c_band_size(c.nd));
-  std::vector<double> rinv(c.h_xrad.size(), 0.0);
-  for (size_t k = 1; k < rinv.size(); ++k) rinv[k] = 1.0 / c.h_xrad[k];
-  c.h1_rinv = dupload(rinv);
-  if (launch_h1c_bands(c.nfe, c.nd, c.Nr, c.radp, c.radk0, c.h1_pf, c.h1_tf, c.st)) return ST_CUDA;
+  Pool p;
+  p.add(&c.h1_z[0], nrow * c.nfe * (c.nd - 1));
+  p.add(&c.h1_z[1], nrow * c.nfe * (c.nd - 1));
+  p.add(&c.h1_cb[0], nrow * c.nfe * 2);
+  p.add(&c.h1_cb[1], nrow * c.nfe * 2);
+  p.add(&c.h1_xb, nrow * std::max(1, c.nfe - 1));
+  p.add(&c.h1_partial, h1elem_partials(c.nfe, c.L1));
+  p.add(&c.h1_ticket, 1);  // zero (dalloc clears)
+  p.add(&c.h1_flags, 4);
+  p.add(&c.h1_pf, (size_t)c.nfe * h1c_band_size(c.nd));
+  p.add(&c.h1_tf, (size_t)c.nfe * h1c_band_size(c.nd));
+  p.add(&c.h1_rinv, c.h_xrad.size());
+  if (!p.allocate()) { cudaGetLastError(); return ST_CUDA; }
+  if (launch_h1c_bands(c.nfe, c.nd, c.Nr, c.xrad, c.radp, c.radk0, c.h1_rinv, c.h1_pf, c.h1_tf, c.st)) return ST_CUDA;
   return 0;
 }
 

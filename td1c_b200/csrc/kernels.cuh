@@ -350,6 +350,12 @@ __device__ __forceinline__ void fedvr_row_span(int ir, int nd, int Nr, int& jlo,
   jhi = jhi > Nr ? Nr : jhi;
 }
 
+// widest band of the bridge inverse the folded passes take.  Up to 4 the shares they stage (10 (2 w + 3) values per
+// orbital) fit where the coupled sums stand later; 8 adds 10 KB and costs the third CTA of an SM.  A time step's band
+// is 1 to 5 on elements of 9 to 21 points (a Ne cycle 42 us, the two-launch pass 64); long steps on fine grids, whose
+// inverse is no band, go there.
+constexpr int H1C_WMAX = 8;
+constexpr int H1C_BW = 2 * H1C_WMAX + 1;
 // ---- one-body propagators of the split schemes (h1prop.cu) ----------------
 // Condensed inverse of M_l = 1 + c T_l, l = 0..L1-1: per finite element the
 // inverse of the interior block and its couplings to the two bridge points,
@@ -369,8 +375,8 @@ struct H1Fac {
   // the folded passes (h1cycle.cu); w < 0: not built, the two-launch passes run
   cplx* af = nullptr;    // [L1][nfe][h1c_af_size] interior inverse and bridge-share rows, fragment order
   cplx* glr = nullptr;   // [L1][nfe][2][ni]: GL, GR
-  cplx* sinv = nullptr;  // [L1][nb][nb] inverse of the bridge matrix
-  int w = -1;            // half-width of the band of sinv that is used
+  cplx* sinv = nullptr;  // [L1][nb][H1C_BW] band of the inverse of the bridge matrix
+  int w = -1;            // half-width of the band that is used
 };
 struct H1FacSrc {
   int Nr, L1, nd, nfe;
@@ -429,11 +435,6 @@ int launch_h1loop_ctl(int* iter, const int* done, int maxcyc, cudaGraphCondition
 int launch_h1bridge(const H1ElemArgs& a, cudaStream_t st);
 // The folded passes of h1cycle.cu: one launch per pass, z in [l][element][orbital][point] and the bridge
 // shares in [l][element][side][orbital], two buffers of each by the cycle's parity
-// widest band of the bridge inverse the folded passes take.  Up to 4 the shares they stage (10 (2 w + 3) values per
-// orbital) fit where the coupled sums stand later; 8 adds 10 KB and costs the third CTA of an SM.  A time step's band
-// is 1 to 5 on elements of 9 to 21 points (a Ne cycle 42 us, the two-launch pass 64); long steps on fine grids, whose
-// inverse is no band, go there.
-constexpr int H1C_WMAX = 8;
 struct H1CycArgs {
   H1Fac fac;
   int Nr, L1, nfun, nfcore, mmax1, igauge;
@@ -461,7 +462,8 @@ struct H1CycArgs {
 };
 size_t h1c_af_size(int nd);
 size_t h1c_band_size(int nd);
-int launch_h1c_bands(int nfe, int nd, int Nr, const double* radp, const double* radk0, double* pf, double* tf, cudaStream_t st);
+int launch_h1c_bands(int nfe, int nd, int Nr, const double* xrad, const double* radp, const double* radk0, double* rinv,
+                     double* pf, double* tf, cudaStream_t st);
 int launch_h1c_setup(const H1Fac& f, int* w, cudaStream_t st);
 bool h1c_fits(int nd, int nfun, int w, int igauge);
 int launch_h1c(const H1CycArgs& a, int mode, cudaStream_t st);  // mode 0 first pass, 1 cycle, 2 the only solve
