@@ -22,6 +22,7 @@
 namespace td1c {
 
 constexpr int PSW_NT = PS_FEW / 4;  // n-tiles of four pairs
+constexpr int PSF_MAXND = 25;       // the condensed factors' largest element
 
 // tiles of the element pass's operand (rows: ni interior points and the left bridge; depth: ni points,
 // the two bridge values and t) and of the share pass's (3 rows, nd points), values per (l, element)
@@ -92,15 +93,14 @@ __global__ void ps_few_binv_kernel(PsCond f) {
 // per-RHS passes
 // ---------------------------------------------------------------------------
 // 1. the element's shares of t and of the bridge right-hand sides
-template <int NDT>
+template <int ND>
 __global__ void __launch_bounds__(32) ps_few_share_kernel(PsCondArgs a) {
   const PsCond& F = a.f;
-  const int nd = NDT > 0 ? NDT : F.nd, ks_n = ps_sf_ks(nd);
+  constexpr int KS = ps_sf_ks(ND);
   const int nfe = F.nfe, Nr = a.Nr, L2 = a.L2, npair = a.npair;
   const int lane = threadIdx.x, gid = lane >> 2, tig = lane & 3, nt = (npair + 3) / 4;
-  const int e = blockIdx.x, l = blockIdx.y, i0 = nd * e - 1;
+  const int e = blockIdx.x, l = blockIdx.y, i0 = ND * e - 1;
   const size_t le = (size_t)l * nfe + e;
-  constexpr int KS = NDT > 0 ? ps_sf_ks(NDT) : 7;
   const double* rho = reinterpret_cast<const double*>(a.rho2) + (gid & 1);
   double b[PSW_NT][KS], A[KS];
 #pragma unroll
@@ -111,18 +111,17 @@ __global__ void __launch_bounds__(32) ps_few_share_kernel(PsCondArgs a) {
 #pragma unroll
     for (int k = 0; k < KS; ++k) {
       const int i = i0 + 4 * k + tig;  // owned points: the left bridge and the interior
-      b[t][k] = (p < npair && k < ks_n && 4 * k + tig < nd && i >= 0) ? __ldg(src + 2 * i) : 0.0;
+      b[t][k] = (p < npair && 4 * k + tig < ND && i >= 0) ? __ldg(src + 2 * i) : 0.0;
     }
   }
 #pragma unroll
-  for (int k = 0; k < KS; ++k) A[k] = (k < ks_n && gid < 3) ? __ldg(F.sfrag + le * ps_sf_size(nd) + k * 32 + lane) : 0.0;
+  for (int k = 0; k < KS; ++k) A[k] = gid < 3 ? __ldg(F.sfrag + le * ps_sf_size(ND) + k * 32 + lane) : 0.0;
 #pragma unroll
   for (int t = 0; t < PSW_NT; ++t) {
     if (t >= nt) break;
     double c0 = 0.0, c1 = 0.0;
 #pragma unroll
-    for (int k = 0; k < KS; ++k)
-      if (NDT > 0 || k < ks_n) psf_dmma(c0, c1, A[k], b[t][k]);
+    for (int k = 0; k < KS; ++k) psf_dmma(c0, c1, A[k], b[t][k]);
     const int p = 4 * t + tig;  // C(row gid, pair tig): re, im
     if (p >= npair || gid > 2) continue;
     if (gid == 0) a.tpart[le * npair + p] = mkc(c0, c1);
@@ -205,14 +204,13 @@ __global__ void __launch_bounds__(PSB_T) ps_few_bridge_kernel(PsCondArgs a) {
 // 3. v on the element's owned points: the interior products with the bridge
 // values and t as three more depths, the left bridge as one more row; zeros
 // for l < |m|
-template <int NDT>
+template <int ND>
 __global__ void __launch_bounds__(32) ps_few_elem_kernel(PsCondArgs a) {
   const PsCond& F = a.f;
-  const int nd = NDT > 0 ? NDT : F.nd, ni = nd - 1, ks_n = ps_wf_ks(nd), mt_n = ps_wf_mt(nd);
+  constexpr int ni = ND - 1, KS = ps_wf_ks(ND), MT = ps_wf_mt(ND);
   const int nfe = F.nfe, nb = F.nb, Nr = a.Nr, L2 = a.L2, npair = a.npair;
   const int lane = threadIdx.x, gid = lane >> 2, tig = lane & 3, nt = (npair + 3) / 4;
-  const int e = blockIdx.x, l = blockIdx.y, i0 = nd * e;
-  constexpr int KS = NDT > 0 ? ps_wf_ks(NDT) : 7, MT = NDT > 0 ? ps_wf_mt(NDT) : 4;
+  const int e = blockIdx.x, l = blockIdx.y, i0 = ND * e;
   const int part = gid & 1;
   double b[PSW_NT][KS];
 #pragma unroll
@@ -228,7 +226,7 @@ __global__ void __launch_bounds__(32) ps_few_elem_kernel(PsCondArgs a) {
       else if (j == ni) { if (e >= 1) s = reinterpret_cast<const double*>(a.xb + ((size_t)l * nb + e - 1) * npair + pp) + part; }
       else if (j == ni + 1) { if (e < nb) s = reinterpret_cast<const double*>(a.xb + ((size_t)l * nb + e) * npair + pp) + part; }
       else if (j == ni + 2) s = reinterpret_cast<const double*>(a.t + (size_t)l * npair + pp) + part;
-      b[t][k] = (p < npair && k < ks_n && s) ? *s : 0.0;
+      b[t][k] = (p < npair && s) ? *s : 0.0;
     }
   }
   int zero = 0;  // bit t: l < |m| of the lane's output pair in n-tile t
@@ -237,20 +235,19 @@ __global__ void __launch_bounds__(32) ps_few_elem_kernel(PsCondArgs a) {
     const int p = 4 * t + tig, m = p < npair ? a.pair_m[p] : 0;
     if (l < (m < 0 ? -m : m)) zero |= 1 << t;
   }
-  const double* wf = F.wfrag + ((size_t)l * nfe + e) * ps_wf_size(nd) + lane;
+  const double* wf = F.wfrag + ((size_t)l * nfe + e) * ps_wf_size(ND) + lane;
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt) {
-    if (NDT == 0 && mt >= mt_n) break;
     double c[PSW_NT][2], A[KS];
 #pragma unroll
-    for (int k = 0; k < KS; ++k) A[k] = (NDT > 0 || k < ks_n) ? __ldg(wf + (mt * ks_n + k) * 32) : 0.0;
+    for (int k = 0; k < KS; ++k) A[k] = __ldg(wf + (mt * KS + k) * 32);
 #pragma unroll
     for (int t = 0; t < PSW_NT; ++t) c[t][0] = c[t][1] = 0.0;
 #pragma unroll
     for (int k = 0; k < KS; ++k)
 #pragma unroll
       for (int t = 0; t < PSW_NT; ++t)
-        if (t < nt && (NDT > 0 || k < ks_n)) psf_dmma(c[t][0], c[t][1], A[k], b[t][k]);
+        if (t < nt) psf_dmma(c[t][0], c[t][1], A[k], b[t][k]);
     const int r = 8 * mt + gid;  // row: interior point, then the left bridge
     if (r > ni || (r == ni && e == 0)) continue;
     const int i = r < ni ? i0 + r : i0 - 1;
@@ -275,28 +272,29 @@ int launch_ps_few_setup(const PsCond& f, cudaStream_t st) {
   return (int)cudaGetLastError();
 }
 
-template <int NDT>
+// Every element size has its own instance: the rows, depths and their guards are then constants.  One instance with
+// loops to the largest size and guards, and this, us a right-hand side of 30 elements, lmax1 20, by points per
+// element less one: 9 pairs 5: 67.1, 64.4; 7: 69.7, 65.7; 8: 69.3, 66.3; 10: 71.4, 67.3; 12: 72.7, 68.8; 16: 72.8, 68.9;
+// 18: 78.9, 75.4; one pair 8: 44.2, 42.2; 12: 46.2, 45.0; 18: 45.9, 44.2 (7 and 20 within 0.6).
+template <int ND>
 static int psf_launch(const PsCondArgs& a, cudaStream_t st) {
+  if (a.f.nd != ND) {
+    if constexpr (ND > 2) return psf_launch<ND - 1>(a, st);
+    return ST_CONFIG;
+  }
   const dim3 grid(a.f.nfe, a.L2);
   const size_t smem = sizeof(double) * 4 * (size_t)((a.f.nb + 3) / 4) * PSB_LD;
-  ps_few_share_kernel<NDT><<<grid, 32, 0, st>>>(a);
+  ps_few_share_kernel<ND><<<grid, 32, 0, st>>>(a);
   ps_few_bridge_kernel<<<a.L2, PSB_T, smem, st>>>(a);
-  ps_few_elem_kernel<NDT><<<grid, 32, 0, st>>>(a);
+  ps_few_elem_kernel<ND><<<grid, 32, 0, st>>>(a);
   return (int)cudaGetLastError();
 }
 
-int launch_ps_few(const PsCondArgs& a, cudaStream_t st) {
-  switch (a.f.nd) {  // 21-, 9- and 8-point Lobatto elements get the unrolled rows
-    case 20: return psf_launch<20>(a, st);
-    case 8: return psf_launch<8>(a, st);
-    case 7: return psf_launch<7>(a, st);
-    default: return psf_launch<0>(a, st);
-  }
-}
+int launch_ps_few(const PsCondArgs& a, cudaStream_t st) { return psf_launch<PSF_MAXND>(a, st); }
 
 // whether the few-pair passes take these sizes (48 KB of shared memory for the bridge pass)
 bool ps_few_fits(const PsCond& f, int npair) {
-  return npair <= PS_FEW && f.ni <= 24 && sizeof(double) * 4 * (size_t)((f.nb + 3) / 4) * PSB_LD <= 48 * 1024;
+  return npair <= PS_FEW && f.nd >= 2 && f.nd <= PSF_MAXND && sizeof(double) * 4 * (size_t)((f.nb + 3) / 4) * PSB_LD <= 48 * 1024;
 }
 
 }  // namespace td1c
