@@ -138,6 +138,24 @@ def test_memory_of_a_factor_goes_with_the_elements(cuda_ok):
         h.final()
 
 
+def _take(n):
+    """n bytes of device memory from the driver, or None."""
+    import ctypes
+    p = ctypes.c_uint64()
+    f = ctypes.CDLL("libcuda.so.1").cuMemAlloc_v2
+    f.argtypes = [ctypes.POINTER(ctypes.c_uint64), ctypes.c_size_t]
+    return p.value if f(ctypes.byref(p), n) == 0 else None
+
+
+def _give(ps):
+    import ctypes
+    f = ctypes.CDLL("libcuda.so.1").cuMemFree_v2
+    f.argtypes = [ctypes.c_uint64]
+    while ps:
+        p = ps.pop()
+        assert not p or f(p) == 0
+
+
 @pytest.mark.gpu
 def test_factor_without_memory_for_the_folded_passes(cuda_ok):
     """With room for the two-launch arrays of a factor (20 MB) but not for the folded ones beside them (45 MB), the
@@ -168,21 +186,24 @@ def test_factor_without_memory_for_the_folded_passes(cuda_ok):
         torch.cuda.synchronize()
         d = torch.from_numpy(orb.reshape(-1).copy()).cuda()
         torch.cuda.empty_cache()
-        for left, piece in ((512 << 20, 64 << 20), (32 << 20, 8 << 20)):
-            while torch.cuda.mem_get_info()[0] > left + piece:
-                hog.append(torch.empty(max(piece, (torch.cuda.mem_get_info()[0] - left) // piece * piece), dtype=torch.uint8, device="cuda"))
+        hog.append(_take(torch.cuda.mem_get_info()[0] - (1 << 30)))
+        for size in (36 << 20, 2 << 20):  # then nothing of either size is left
+            while True:
+                p = _take(size)
+                if not p:
+                    break
+                hog.append(p)
+        _give([hog.pop(1)])  # 36 MB
         before = h.launch_count()
         h.h1itr_dev(d.data_ptr(), lf, dtime, CYC, 0.0)
         assert h.launch_count() - before == TWO
         h.sync()
-        hog.clear()
-        torch.cuda.empty_cache()
+        _give(hog)
         assert rel_err(d.cpu().numpy(), want) < TOL
         h.split2_dev(x.data_ptr(), c.data_ptr(), 30.0, 0.004, 2)
         h.sync()
         _, n = _step(h, orb, lf, 2 * dtime)
         assert n == FOLDED
     finally:
-        hog.clear()
-        torch.cuda.empty_cache()
+        _give(hog)
         h.final()
