@@ -635,6 +635,7 @@ __global__ void __launch_bounds__(256) smallmat_kernel(SmallArgs a) {
   __shared__ cplx F[16 * 16];
   const int n = a.nact, nf = a.nfun, nc = a.ncore, nfc = a.nfcore;
   const int tid = threadIdx.x;
+  const double dt = a.io ? a.io->dtime : a.dtime;
   // int1e(ja, ia) = A(j, i) for ja <= ia, conj fill
   for (int e = tid; e < n * n; e += blockDim.x) {
     int ja = e % n, ia = e / n;
@@ -683,7 +684,6 @@ __global__ void __launch_bounds__(256) smallmat_kernel(SmallArgs a) {
     a.ene[4] = a.ene_fcore + ed + ene_act;
   }
   // X matrix
-  const double dt = a.io ? a.io->dtime : a.dtime;
   const cplx tfac = a.icomp == 0 ? mkc(dt, 0) : mkc(0, dt);
   for (int e = tid; e < nf * nf; e += blockDim.x) a.xmat[e] = mkc(0, 0);
   __syncthreads();
@@ -762,6 +762,7 @@ __global__ void __launch_bounds__(512) dtorb_kernel(size_t nb, int nfun, int nfc
   for (int e = threadIdx.x; e < nfun * nfun; e += blockDim.x) sx[e] = xmat[e];
   if (threadIdx.x < nfun) sm[threadIdx.x] = mval[threadIdx.x];
   cplx* hwfn = io ? io->hwfn : hwfn_arg;
+  const double dt = io ? io->dtime : dtime;
   if (io && no_ci && blockIdx.x == 0 && threadIdx.x == 0) io->hcic[0] = mkc(0, 0);  // no active space: hcic = 0
   __syncthreads();
   if (!in) return;
@@ -769,7 +770,6 @@ __global__ void __launch_bounds__(512) dtorb_kernel(size_t nb, int nfun, int nfc
     if (rk.stage == 0) hwfn[t] = mkc(0, 0);
     return;
   }
-  const double dt = io ? io->dtime : dtime;
   const cplx tf2 = icomp == 0 ? mkc(-dt, 0) : mkc(0, -dt);
   cplx o = cmul(h, tf2);
   const int mi = sm[i];
