@@ -33,9 +33,9 @@
 //
 // What bounds it: the latency of the chain stage, bridge dots, sum, products,
 // store within a CTA (three CTAs of 70 KB share an SM).  Measured (Ne, 60
-// elements of 21 points, lmax1 50, 6 orbitals): a cycle 52 + 12.3 us (element
-// pass + bridge solve) -> 42, a first pass 45 + 12 -> 34; He (lmax1 19) a cycle
-// 15 + 9.5 -> 14.  Taking the derivative of every neighbour instead of their
+// elements of 21 points, lmax1 47, 10 orbitals): a cycle 52 + 12.3 us (element
+// pass + bridge solve) -> 42, a first pass 45 + 12 -> 34; He (40 elements, lmax1 23,
+// 1 orbital) a cycle 15 + 9.5 -> 14.  Taking the derivative of every neighbour instead of their
 // sum (step 3) took 51 us: more operands in shared memory, two CTAs per SM.
 #include <algorithm>
 

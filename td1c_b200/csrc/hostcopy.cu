@@ -9,7 +9,7 @@
 //
 // The ring and its threads belong to the process: four slots of 2 MB, made by
 // the first large copy and given back by host_copy_release (with the last
-// context).  Ne's right-hand side from host buffers: 2700 -> 1480 us (the RHS itself 450).
+// context).  Ne's right-hand side from host buffers: 2825 -> 1493 us (the RHS itself 490).
 // From 512 KB on: a host call of 5 orbitals, us through the ring and on the plain path,
 // by the state's size: 75 KB 149 and 137, 249 KB 161 and 156, 412 KB 177 and 182, 749 KB
 // 200 and 233, 1.5 MB 280 to 320 and 335 to 355.  Page-locked (or managed) buffers cross the bus as they are, and a

@@ -1705,8 +1705,9 @@ int run_htot(Ctx& c, const double* d_lf, const cplx* wfn, const cplx* cic_in, cp
 }
 
 // One RHS on the caller's device buffers.  An eager RHS is some twenty launches and events on three
-// streams, more host time than the small workloads' kernels take (us a call among others, eager and replayed: an
-// 8 x 8 box 46.0 and 15.2, He 45.7 and 22.3, Ne's 445 either way); the second call in a row with the same
+// streams, more host time than the small workloads' kernels take (us a call, eager and replayed, one context in a
+// row: an 8 x 8 box 61 and 36, He 72 and 46, Ne 507 and 490; three contexts in turn, whose kernels overlap: 46 and
+// 13, 47 and 20, 441 and 451).  A context's first call is eager; the second call in a row with the same
 // settings captures it once (reading the buffers, the field and the time step from device memory, so the capture
 // holds for any of them), and later calls replay it.  The capture goes with the context, or when a setting changes.
 struct RhsKey {

@@ -21,10 +21,11 @@
 // partial sums; dot_sum_kernel adds them in a fixed order and
 // int2e_form_kernel forms the integrals.
 //
-// What bounds it: staging (60 rows of 16 points a stage, 8 warps waiting for
-// it together) and the tensor pipe in turn.  Ne, CAS(8e,9o), K = 127260:
-// 93 + 8 us (complex tiles) -> 42 + 3; 66 before the item shapes were unrolled
-// one by one (dp_item).
+// What bounds it: staging (90 rows of 16 points a stage for the 45 pairs of
+// 9 orbitals, 8 warps waiting for it together) and the tensor pipe in turn.
+// Ne, CAS(8e,9o), K = 113905: 93 + 8 us (complex tiles, their sum) -> 42 + 8 + 3
+// (products, sum, form); 66 for the products before the item shapes were
+// unrolled one by one (dp_item).
 #include <algorithm>
 
 #include "common.cuh"

@@ -350,10 +350,14 @@ __device__ __forceinline__ void fedvr_row_span(int ir, int nd, int Nr, int& jlo,
   jhi = jhi > Nr ? Nr : jhi;
 }
 
-// widest band of the bridge inverse the folded passes take.  Up to 4 the shares they stage (10 (2 w + 3) values per
-// orbital) fit where the coupled sums stand later; 8 adds 10 KB and costs the third CTA of an SM.  A time step's band
-// is 1 to 5 on elements of 9 to 21 points (a Ne cycle 42 us, the two-launch pass 64); long steps on fine grids, whose
-// inverse is no band, go there.
+// Widest band of the bridge inverse the folded passes take.  The shares they stage, 10 (2 w + 3) values per orbital,
+// stand where the 6 (nd + 1) of the coupled sums do later, so they cost no shared memory up to w = 3 (nd + 1) / 10 - 1.5
+// (4 for nd = 20, 0 for nd = 7); w = 8 adds 10 KB and the third CTA of an SM for Ne.  A time step's band is 1 to 5 on
+// elements of 9 to 21 points, up to 8 on shorter ones.  The folded passes are the faster ones at every width (a split
+// step of twice 6 cycles, us, by w = 5, 6, 7, 8, and on the two-launch passes): He, 100 elements of 4 points 574, 574,
+// 586, 580 and 740; Ne's orbitals there 1450, 1445, 1464, 1438 and 1570 to 1605; He, 80 elements of 8 points 582, 581,
+// 591, 587 and 677; Ne, 60 elements of 21 points (long steps) 7520, 7541, 7653, 7658 and 7788.  Long steps on fine
+// grids, whose inverse is no band, go to the two-launch passes.
 constexpr int H1C_WMAX = 8;
 constexpr int H1C_BW = 2 * H1C_WMAX + 1;
 // ---- one-body propagators of the split schemes (h1prop.cu) ----------------

@@ -26,10 +26,10 @@
 // writes both mirrors of its half of the rows.
 //
 // What bounds it: the FP64 tensor pipe (55% busy) and, between chunks, the
-// barrier that frees a buffer.  Measured against the dense kernel (Ne, nrad
-// 1260, nlat 108, 42 pairs, lmax2 100): pair densities to l 107.6 -> 62 us,
-// potentials to theta 96 -> 59, orbitals to theta 17 -> 11.3, g and v2 to l
-// 21.6 -> 17; a right-hand side 633 -> 538.  Three m-tiles per warp made the
+// barrier that frees a buffer.  Measured against the dense kernel (Ne, 1199
+// radial points, nlat 95, lmax2 94, 54 pairs): pair densities to l 107.6 -> 64.5
+// us, potentials to theta 96 -> 61.4, orbitals to theta 17 -> 11.0, g and v2 to l
+// 21.6 -> 16.8; a right-hand side 633 -> 538.  Three m-tiles per warp made the
 // right-hand side 11% slower (fewer warps in flight), and 512-thread
 // persistent CTAs over the same tiles took 75 and 74 us where this takes 62
 // and 59.

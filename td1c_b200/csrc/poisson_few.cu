@@ -10,7 +10,7 @@
 //
 // What bounds it: latency, of the loads within a pass and of the three launches.  He (1 pair, 40 elements of 21
 // points, lmax2 46): a right-hand side
-// 25.5 -> 19.4 us among others, 8 split steps 2700 -> 2385 us.  From about 20 pairs on the staged passes are as fast
+// 25.5 -> 19.4 us (calls of several contexts in turn), 8 split steps 2700 -> 2385 us.  From about 20 pairs on the staged passes are as fast
 // (21 pairs, 33 elements, lmax2 52: equal) or faster (6 orbitals, 37 elements of 13 points: 57 us a right-hand
 // side against 59 here; 55 pairs, 80 elements, lmax2 126: 1.8% less of a split step), since they read each
 // operand table once per 32 pairs and leave more of the SM to the kernels beside them.
